@@ -44,7 +44,7 @@ HOST_SOURCES = ["xml.cpp", "mesh.cpp", "task.cpp", "solver.cpp", "solver_adjoint
 DEVICE_SOURCES = {"kern_fp64.cu": "false", "kern_common.cu": "false", "kern_mixed.cu": "true",
                   "noalloc.cu": "false", "adjoint.cu": "false", "adjoint_mixed.cu": "true",
                   "implicit.cu": "false", "gmres.cu": "fma", "rkdg.cu": "false"}
-HEADERS = ["xml.hpp", "mesh.hpp", "task.hpp", "solver.hpp", "kernels.hpp", "kernels.cuh", "kern_inst.cuh",
+HEADERS = ["intpipe.cuh", "xml.hpp", "mesh.hpp", "task.hpp", "solver.hpp", "kernels.hpp", "kernels.cuh", "kern_inst.cuh",
            "adjoint.cuh", "adj_inst.cuh", "implicit.hpp", "rkdg.hpp"]
 
 

@@ -133,11 +133,15 @@ __device__ __forceinline__ void adj_flux_edge(const DevCase& c, const AdjCase& a
 // the forward kernels' flags and the same code, so F is the forward's bit for bit.
 template <typename T, int RECON>
 __global__ void __launch_bounds__(128) k_flux_rec(const DevCase c, const FluxRec r) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= c.ne) return;
-    T out[4];
-    flux_edge<T, FLUX_HLLC, RECON, true>(c, e, out, r);
-    st4(F_of<T>(c), e, out[0], out[1], out[2], out[3]);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if constexpr (FluxLanes<T, RECON>::n == 2) {
+        const bool live = t < 2 * c.ne;
+        if ((t & ~31) < 2 * c.ne) flux_lane<FLUX_HLLC, RECON, true>(c, live ? t >> 1 : c.ne - 1, t & 1, live, r);
+    } else if (t < c.ne) {
+        T out[4];
+        flux_edge<T, FLUX_HLLC, RECON, true>(c, t, out, r);
+        st4(F_of<T>(c), t, out[0], out[1], out[2], out[3]);
+    }
 }
 
 // k_adj_flux (HLLC) reading the forward's record of each Gauss point instead of
@@ -367,9 +371,8 @@ void KFN(adj_flux)(const DevCase& c, const AdjCase& a, int flux, int recon, cuda
     else adj_flux_by_recon<FLUX_LAX>(c, a, recon, s);
 }
 void KFN(flux_rec)(const DevCase& c, int recon, const FluxRec& r, cudaStream_t s) {
-    // 128-thread blocks: at ~164 registers a thread, 256-thread blocks leave one block (8
-    // warps) per SM, 128-thread blocks three (12 warps)
-    const int g = adj_nblk(c.ne, 128);
+    // 128-thread blocks: finer than 256 in registers, so more warps fit an SM
+    const int g = adj_nblk(c.ne * (sizeof(KT) == 8 && recon != RECON_NONE ? 2 : 1), 128);
     if (recon == RECON_NONE) k_flux_rec<KT, RECON_NONE><<<g, 128, 0, s>>>(c, r);
     else if (recon == RECON_LINEAR) k_flux_rec<KT, RECON_LINEAR><<<g, 128, 0, s>>>(c, r);
     else k_flux_rec<KT, RECON_MINMOD><<<g, 128, 0, s>>>(c, r);

@@ -443,7 +443,7 @@ void ImplicitSolver::profile_steps(int n, double ms[4], int launches[4]) {
             CUDA_CHECK(cudaEventElapsedTime(&t, ev[k], ev[k + 1]));
             ms[k] += t;
         }
-        launches[0] += 2; launches[1] += 1; launches[2] += 1; launches[3] += gm_launches;
+        launches[0] += 2; launches[1] += 2; launches[2] += 1; launches[3] += gm_launches;
         for (int guard = 0; ctl_host_->restart && guard <= task_.gmres_maxit; guard++) {
             CUDA_CHECK(cudaGraphLaunch(g_restart_, stream_));
             CUDA_CHECK(cudaStreamSynchronize(stream_));

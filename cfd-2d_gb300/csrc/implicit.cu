@@ -14,15 +14,14 @@ __device__ __forceinline__ const DevMat& imat(const ImpCase& c, int i) { return 
 // FVM_TVD_IMPLICIT::boundaryCond, :963-1008. INLET: (T, P, Vx, Vy) then URS(2)
 // rho = p M / (T gR); OUTLET: the cell state; WALL: the cell state with the normal
 // velocity mirrored, u - 2 (u.n) n. Only r, u, v, p are consumed downstream.
-__device__ __forceinline__ Prim<double> imp_ghost(const DevBnd& b, const Prim<double>& q, double nx, double ny,
-                                                  double M) {
-    Prim<double> g = q;
+__device__ __forceinline__ Prim<xd> imp_ghost(const DevBnd& b, const Prim<xd>& q, xd nx, xd ny, double M) {
+    Prim<xd> g = q;
     if (b.kind == IBND_INLET) {
-        g.u = b.u; g.v = b.v; g.p = b.p;
-        g.r = g.p * M / (b.T * GAS_R);
+        g.u = xd(b.u); g.v = xd(b.v); g.p = xd(b.p);
+        g.r = g.p * xd(M) / (xd(b.T) * xd(GAS_R));
     } else if (b.kind == IBND_WALL) {
-        const double Un = q.u * nx + q.v * ny;
-        const double Vx = nx * Un * 2.0, Vy = ny * Un * 2.0;
+        const xd Un = q.u * nx + q.v * ny;
+        const xd Vx = nx * Un * xd(2.0), Vy = ny * Un * xd(2.0);
         g.u = q.u - Vx;
         g.v = q.v - Vy;
     }
@@ -45,92 +44,104 @@ __global__ void __launch_bounds__(256) k_imp_grad(const ImpCase c) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.nc) return;
     const int nc = c.nc;
-    const Prim<double> q = load_prim(c.W, i);
-    double g[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    const Prim<xd> q = prim_as<xd>(load_prim(c.W, i));
+    xd g[8];
+#pragma unroll
+    for (int m = 0; m < 8; m++) g[m] = xd(0.0);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         const int f = c.face[k * nc + i], e = f >> 1;
         const bool side2 = f & 1;
-        const double nx = c.nx[e], ny = c.ny[e], l = c.l[e];
-        Prim<double> o;
-        if (e < c.n_int) o = load_prim(c.W, side2 ? c.ec1[e] : c.ec2[e]);
+        const xd nx(c.nx[e]), ny(c.ny[e]), l(c.l[e]);
+        Prim<xd> o;
+        if (e < c.n_int) o = prim_as<xd>(load_prim(c.W, side2 ? c.ec1[e] : c.ec2[e]));
         else o = imp_ghost(c.bnds[c.ebnd[e]], q, nx, ny, imat(c, i).M);
         grad_face(g, q, o, nx, ny, l, side2);
     }
-    const double s = c.S[i], y = c.invS[i];
+    const xd s(c.S[i]);
+    const ip::Recip y = recip_of(s);
 #pragma unroll
-    for (int m = 0; m < 8; m++) g[m] = div_rn(g[m], s, y);
-    st8(c.G, i, g);
+    for (int m = 0; m < 8; m++) g[m] = div_y(g[m], s, y);
+    st8x(c.G, i, g);
 }
 
 // calcRoeAverage (:408-429) over roe_orig (src/global.cpp:407-441) with W = 0:
 // the W terms add +0 to sums of squares and change no bit, so they are left out.
-struct Roe { double r, u, v, p, E, cz; };
-__device__ __forceinline__ Roe roe_average(const Prim<double>& L, const Prim<double>& R, double GAM) {
-    const double AGAM = (GAM - 1.0);
-    const double fSB = sqrt(L.r), fSE = sqrt(R.r);
-    const double fS_ = 1.0 / (fSB + fSE);
+struct Roe { xd r, u, v, p, E, cz; };
+__device__ __forceinline__ Roe roe_average(const Prim<xd>& L, const Prim<xd>& R, xd GAM) {
+    const xd AGAM = GAM - xd(1.0);
+    const xd fSB = t_sqrt(L.r), fSE = t_sqrt(R.r);
+    const xd fS_ = xd(ip::rcp((fSB + fSE).v));
     Roe a;
     a.r = fSB * fSE;
     a.u = (fSB * L.u + fSE * R.u) * fS_;
     a.v = (fSB * L.v + fSE * R.v) * fS_;
-    const double EB = L.p / (L.r * AGAM), EE = R.p / (R.r * AGAM);
-    const double HB = EB + (L.u * L.u + L.v * L.v) * 0.5 + L.p / L.r;
-    const double HE = EE + (R.u * R.u + R.v * R.v) * 0.5 + R.p / R.r;
-    const double HI = (fSB * HB + fSE * HE) * fS_;
-    a.p = (HI - (a.u * a.u + a.v * a.v) * 0.5) * a.r * (GAM - 1.0) / GAM;
-    const double e = a.p / (a.r * AGAM);
-    a.cz = sqrt(GAM * a.p / a.r);
-    a.E = e + 0.5 * (a.u * a.u + a.v * a.v);
+    const xd EB = L.p / (L.r * AGAM), EE = R.p / (R.r * AGAM);
+    const xd HB = EB + half(L.u * L.u + L.v * L.v) + L.p / L.r;
+    const xd HE = EE + half(R.u * R.u + R.v * R.v) + R.p / R.r;
+    const xd HI = (fSB * HB + fSE * HE) * fS_;
+    a.p = (HI - half(a.u * a.u + a.v * a.v)) * a.r * (GAM - xd(1.0)) / GAM;
+    const xd e = a.p / (a.r * AGAM);
+    a.cz = t_sqrt(GAM * a.p / a.r);
+    a.E = e + half(a.u * a.u + a.v * a.v);
     return a;
 }
 
 // The two Gauss-point fluxes of an edge times l/2 (run's loop, :612-633): interior
 // faces reconstruct linearly from both centres (reconstruct(iFace, pL, pR, p),
-// :444-476), boundary faces take the centre state and its ghost.
+// :444-476), boundary faces take the centre state and its ghost. Two lanes per edge, one
+// Gauss point each (k_flux of the explicit method says why).
 template <int FLUX>
-__global__ void __launch_bounds__(256) k_imp_flux(const ImpCase c) {
+__global__ void __launch_bounds__(128, 6) k_imp_flux(const ImpCase c) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if ((t & ~31) >= 2 * c.ne) return;
+    const bool live = t < 2 * c.ne;
+    const int e = live ? t >> 1 : c.ne - 1, gp = t & 1;
+    const size_t ne = c.ne;
+    const int c1 = c.ec1[e];
+    const bool inner = e < c.n_int;
+    const xd nx(c.nx[e]), ny(c.ny[e]), GAM(c.gam_flux);
+    Prim<xd> pL = prim_as<xd>(load_prim(c.W, c1)), pR;
+    if (inner) {
+        const int c2 = c.ec2[e];
+        const double* __restrict__ dl = c.dl + (size_t)(4 * gp) * ne + e;
+        pR = prim_as<xd>(load_prim(c.W, c2));
+        double g[8];
+        ld8(c.G, c1, g);
+        reconstruct<xd, RECON_LINEAR>(pL, g, xd(dl[0]), xd(dl[ne]), pL);
+        ld8(c.G, c2, g);
+        reconstruct<xd, RECON_LINEAR>(pR, g, xd(dl[2 * ne]), xd(dl[3 * ne]), pR);
+    } else {  // both Gauss points see the same centre state and ghost
+        pR = imp_ghost(c.bnds[c.ebnd[e]], pL, nx, ny, imat(c, c1).M);
+    }
+    xd f[4];
+    bool hit = false;
+    if constexpr (FLUX == FLUX_LAX) flux_lax(f, pL, pR, nx, ny, GAM, xd(c.ig1_flux), recip_of(pL.r), recip_of(pR.r));
+    else hit = flux_godunov(f, pL, pR, nx, ny, c.rg_flux, c.newton_cap, recip_of(pL.r), recip_of(pR.r));
+    if (hit && live) atomicOr(c.err, ERRBIT_NEWTON_CAP);
+    const xd lh = half(xd(c.l[e]));  // right4 -= 0.5*l*fr, :623-633
+    double out[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {  // the points' sum from +0, two components per lane
+        double mine = gp ? f[2 + k].v : f[k].v;
+        double other = __shfl_xor_sync(0xffffffffu, gp ? f[k].v : f[2 + k].v, 1);
+        (gp ? other : mine) = ip::plus_zero(gp ? other : mine);
+        out[k] = ((xd(mine) + xd(other)) * lh).v;
+    }
+    if (live) reinterpret_cast<double2*>(c.F)[2 * (size_t)e + gp] = make_double2(out[0], out[1]);
+}
+
+// calcRoeAverage of the edge's centre states (cellL = c1, cellR = c2 or the ghost,
+// :553-554), for both cells' block rows
+__global__ void __launch_bounds__(128) k_imp_roe(const ImpCase c) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= c.ne) return;
-    const int ne = c.ne;
     const int c1 = c.ec1[e];
-    const double nx = c.nx[e], ny = c.ny[e], l = c.l[e];
-    const double GAM = c.gam_flux;
-    const Prim<double> qL = load_prim(c.W, c1);
-    double fs[4] = {0.0, 0.0, 0.0, 0.0};
-    bool hit = false;
-    if (e < c.n_int) {
-        const int c2 = c.ec2[e];
-        const Prim<double> qR = load_prim(c.W, c2);
-        double gL[8], gR[8];
-        ld8(c.G, c1, gL);
-        ld8(c.G, c2, gR);
-#pragma unroll
-        for (int gp = 0; gp < 2; gp++) {
-            Prim<double> pL = qL, pR = qR;
-            reconstruct<double, RECON_LINEAR>(pL, gL, c.dl[(4 * gp) * ne + e], c.dl[(4 * gp + 1) * ne + e], qL);
-            reconstruct<double, RECON_LINEAR>(pR, gR, c.dl[(4 * gp + 2) * ne + e], c.dl[(4 * gp + 3) * ne + e], qR);
-            double f[4];
-            if constexpr (FLUX == FLUX_LAX) flux_lax(f, pL, pR, nx, ny, GAM, c.ig1_flux);
-            else hit |= flux_godunov<double, false>(f, pL, pR, nx, ny, c.rg_flux, c.newton_cap);
-            fs[0] = fs[0] + f[0]; fs[1] = fs[1] + f[1]; fs[2] = fs[2] + f[2]; fs[3] = fs[3] + f[3];
-        }
-    } else {  // both Gauss points see the same centre state and ghost
-        const Prim<double> pR = imp_ghost(c.bnds[c.ebnd[e]], qL, nx, ny, imat(c, c1).M);
-        double f[4];
-        if constexpr (FLUX == FLUX_LAX) flux_lax(f, qL, pR, nx, ny, GAM, c.ig1_flux);
-        else hit |= flux_godunov<double, false>(f, qL, pR, nx, ny, c.rg_flux, c.newton_cap);
-        fs[0] = fs[0] + f[0]; fs[1] = fs[1] + f[1]; fs[2] = fs[2] + f[2]; fs[3] = fs[3] + f[3];
-        fs[0] = fs[0] + f[0]; fs[1] = fs[1] + f[1]; fs[2] = fs[2] + f[2]; fs[3] = fs[3] + f[3];
-    }
-    if (hit) atomicOr(c.err, ERRBIT_NEWTON_CAP);
-    const double lh = 0.5 * l;  // right4 -= 0.5*l*fr, :623-633
-    st4(c.F, e, fs[0] * lh, fs[1] * lh, fs[2] * lh, fs[3] * lh);
-    // calcRoeAverage of the edge's centre states (cellL = c1, cellR = c2 or the ghost,
-    // :553-554), for both cells' block rows
-    const Prim<double> cR = e < c.n_int ? load_prim(c.W, c.ec2[e]) : imp_ghost(c.bnds[c.ebnd[e]], qL, nx, ny, imat(c, c1).M);
-    const Roe a = roe_average(qL, cR, GAM);
-    st4(c.R, e, a.u, a.v, a.cz, a.E + a.p / a.r);  // H of eigenValues' callers, :565
+    const Prim<xd> qL = prim_as<xd>(load_prim(c.W, c1));
+    const Prim<xd> qR = e < c.n_int ? prim_as<xd>(load_prim(c.W, c.ec2[e]))
+                                    : imp_ghost(c.bnds[c.ebnd[e]], qL, xd(c.nx[e]), xd(c.ny[e]), imat(c, c1).M);
+    const Roe a = roe_average(qL, qR, xd(c.gam_flux));
+    st4(c.R, e, a.u.v, a.v.v, a.cz.v, (a.E + a.p / a.r).v);  // H of eigenValues' callers, :565
 }
 
 // (s * 0.5) * l as s * (0.5 l): halving is exact for |s| >= 2^-1021 (exponent field >= 2,
@@ -138,15 +149,12 @@ __global__ void __launch_bounds__(256) k_imp_flux(const ImpCase c) {
 // a zero gives the same signed zero; smaller nonzero s take the two products (out of line,
 // so that the common path is not evaluated beside them).
 static __device__ __noinline__ double mul_half_l_tiny(double s, double l) { return (s * 0.5) * l; }
-__device__ __forceinline__ double mul_half_l(double s, double hl, double l) {
-    const long long b = __double_as_longlong(s);
+__device__ __forceinline__ xd mul_half_l(xd s, xd hl, xd l) {
+    const long long b = __double_as_longlong(s.v);
     if (__builtin_expect(((b >> 52) & 0x7ff) >= 2 || (b << 1) == 0, 1)) return s * hl;  // (zeros: +-0 either way)
-    return mul_half_l_tiny(s, l);
+    return xd(mul_half_l_tiny(s.v, l.v));
 }
-// 0.0 + x: x, with -0 turned into +0 (on the integer pipe)
-__device__ __forceinline__ double plus_zero(double x) {
-    return __double_as_longlong(x) == (long long)0x8000000000000000ull ? 0.0 : x;
-}
+__device__ __forceinline__ xd plus_zero(xd x) { return xd(ip::plus_zero(x.v)); }
 
 // One face's 0.5 l R diag(lam+-) L (eigenValues / rightEigenVector / leftEigenVector /
 // calcAP / calcAM, :335-406, scaled by l in run, :572-600) from the Roe state (u, v, c,
@@ -156,55 +164,52 @@ __device__ __forceinline__ double plus_zero(double x) {
 // a zero term never changes such a sum (started from +0 it cannot become -0), so column k
 // contributes to A+ only where lam_k > 0 and to A- only where lam_k < 0, in the
 // reference's order of k: the same bits with half the products.
-// Adds A+ into dg (the cell's diagonal block; first: dg holds nothing yet, the sums start
-// from 0); returns A- in am.
-template <bool FIRST>
-__device__ __forceinline__ void face_jacobians(double u, double v, double c, double H, double GAM, double nx,
-                                               double ny, double l, double* dg, double* am) {
-    const double hl = 0.5 * l;
-    const double qn = u * nx + v * ny;
-    const double q2 = u * u + v * v;
-    const double lx = -ny, ly = nx;
-    const double ql = u * lx + v * ly;
-    const double g1 = GAM - 1.0, c2 = c * c;
-    // the quotients of leftEigenVector, each correctly rounded (div_rn equals '/')
-    const double yc2 = 1.0 / c2, yc = 1.0 / c;
-    const double A0 = div_rn(0.5 * q2 * g1, c2, yc2);
-    const double B0 = div_rn(qn, c, yc);
-    const double Cu = div_rn(g1 * u, c2, yc2);
-    const double Dn = div_rn(nx, c, yc);
-    const double Ev = div_rn(g1 * v, c2, yc2);
-    const double Fn = div_rn(ny, c, yc);
-    const double G0 = div_rn(0.5 * g1, c2, yc2);
-    const double Hg = div_rn(g1, c2, yc2);
-    const double L[16] = {0.5 * (A0 + B0), -0.5 * (Cu + Dn), -0.5 * (Ev + Fn), G0,
-                          1 - A0,          Cu,               Ev,               neg_if(Hg, true),
-                          0.5 * (A0 - B0), -0.5 * (Cu - Dn), -0.5 * (Ev - Fn), G0,
-                          neg_if(ql, true), lx,              ly,               0.0};
-    const double lam[4] = {qn - c, qn, qn + c, qn};
+// Adds A+ into dg (the cell's diagonal block); returns A- in am.
+__device__ __forceinline__ void face_jacobians(xd u, xd v, xd c, xd H, xd GAM, xd nx, xd ny, xd l, xd* dg, xd* am) {
+    const xd hl = half(l);
+    const xd qn = u * nx + v * ny;
+    const xd q2 = u * u + v * v;
+    const xd lx = -ny, ly = nx;
+    const xd ql = u * lx + v * ly;
+    const xd g1 = GAM - xd(1.0), c2 = c * c;
+    // the quotients of leftEigenVector
+    const ip::Recip yc2 = recip_of(c2), yc = recip_of(c);
+    const xd A0 = div_y(half(q2) * g1, c2, yc2);
+    const xd B0 = div_y(qn, c, yc);
+    const xd Cu = div_y(g1 * u, c2, yc2);
+    const xd Dn = div_y(nx, c, yc);
+    const xd Ev = div_y(g1 * v, c2, yc2);
+    const xd Fn = div_y(ny, c, yc);
+    const xd G0 = div_y(half(g1), c2, yc2);
+    const xd Hg = div_y(g1, c2, yc2);
+    const xd L[16] = {half(A0 + B0), -half(Cu + Dn), -half(Ev + Fn), G0,
+                          xd(1.0) - A0,    Cu,               Ev,               neg_if(Hg, true),
+                          half(A0 - B0),  -half(Cu - Dn), -half(Ev - Fn), G0,
+                          neg_if(ql, true), lx,              ly,               xd(0.0)};
+    const xd lam[4] = {qn - c, qn, qn + c, qn};
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        double Rr[4];
-        if (i == 0) { Rr[0] = 1.0; Rr[1] = 1.0; Rr[2] = 1.0; Rr[3] = 0.0; }
+        xd Rr[4];
+        if (i == 0) { Rr[0] = xd(1.0); Rr[1] = xd(1.0); Rr[2] = xd(1.0); Rr[3] = xd(0.0); }
         if (i == 1) { Rr[0] = u - c * nx; Rr[1] = u; Rr[2] = u + c * nx; Rr[3] = lx; }
         if (i == 2) { Rr[0] = v - c * ny; Rr[1] = v; Rr[2] = v + c * ny; Rr[3] = ly; }
-        if (i == 3) { Rr[0] = H - qn * c; Rr[1] = q2 / 2; Rr[2] = H + qn * c; Rr[3] = ql; }
-        double sp[4] = {0.0, 0.0, 0.0, 0.0}, sm[4] = {0.0, 0.0, 0.0, 0.0};
+        if (i == 3) { Rr[0] = H - qn * c; Rr[1] = half(q2); Rr[2] = H + qn * c; Rr[3] = ql; }
+        xd sp[4] = {xd(0.0), xd(0.0), xd(0.0), xd(0.0)}, sm[4] = {xd(0.0), xd(0.0), xd(0.0), xd(0.0)};
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            const double t = Rr[k] * lam[k];
-            if (lam[k] > 0) {
+            const xd t = i == 0 && k < 3 ? lam[k] : Rr[k] * lam[k];  // 1.0 * lam
+            if (lam[k].v > 0) {
 #pragma unroll
                 for (int j = 0; j < 4; j++) sp[j] = sp[j] + t * L[4 * k + j];
-            } else if (lam[k] < 0) {
+            } else if (lam[k].v < 0) {
 #pragma unroll
                 for (int j = 0; j < 4; j++) sm[j] = sm[j] + t * L[4 * k + j];
             }
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const double ap = mul_half_l(sp[j], hl, l);
-            dg[4 * i + j] = FIRST ? plus_zero(ap) : dg[4 * i + j] + ap;
+            const xd ap = mul_half_l(sp[j], hl, l);
+            dg[4 * i + j] = dg[4 * i + j] + ap;
             am[4 * i + j] = plus_zero(mul_half_l(sm[j], hl, l));
         }
     }
@@ -214,16 +219,16 @@ __device__ __forceinline__ void face_jacobians(double u, double v, double c, dou
 // cell in ascending edge order, and the diagonal S/cTau of :640-664): the Roe
 // average of the face's two centre states, the spectral radius (steady), A+ into
 // the diagonal block, A- as the face's block, and the right-hand side -sum F l/2.
-__global__ void __launch_bounds__(128) k_imp_assemble(const ImpCase c) {
+__global__ void __launch_bounds__(128, 4) k_imp_assemble(const ImpCase c) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.nc) return;
     const int nc = c.nc;
-    const double GAM = c.gam_flux;
-    double dg[16];
+    const xd GAM(c.gam_flux);
+    xd dg[16];
 #pragma unroll
-    for (int m = 0; m < 16; m++) dg[m] = 0.0;
-    double rhs[4] = {0.0, 0.0, 0.0, 0.0};
-    double lam = 0.0;
+    for (int m = 0; m < 16; m++) dg[m] = xd(0.0);
+    xd rhs[4] = {xd(0.0), xd(0.0), xd(0.0), xd(0.0)};
+    xd lam(0.0);
 #pragma unroll 1
     for (int k = 0; k < 3; k++) {
         const int f = c.face[k * nc + i], e = f >> 1;
@@ -231,40 +236,40 @@ __global__ void __launch_bounds__(128) k_imp_assemble(const ImpCase c) {
         double fe[4];
         ld4(c.F, e, fe);
 #pragma unroll
-        for (int m = 0; m < 4; m++) rhs[m] = rhs[m] + neg_if(fe[m], !side2);
-        const double nx = c.nx[e], ny = c.ny[e], l = c.l[e];
-        double a[4];  // the edge's Roe state (u, v, c, H), formed once by k_imp_flux
-        ld4(c.R, e, a);
-        if (c.steady) lam = lam + (sqrt(a[0] * a[0] + a[1] * a[1]) + a[2]) * l;
-        double am[16];
-        if (k == 0) face_jacobians<true>(a[0], a[1], a[2], a[3], GAM, neg_if(nx, side2), neg_if(ny, side2), l, dg, am);
-        else face_jacobians<false>(a[0], a[1], a[2], a[3], GAM, neg_if(nx, side2), neg_if(ny, side2), l, dg, am);
+        for (int m = 0; m < 4; m++) rhs[m] = rhs[m] + xd(neg_if(fe[m], !side2));
+        const xd nx(c.nx[e]), ny(c.ny[e]), l(c.l[e]);
+        double ra[4];  // the edge's Roe state (u, v, c, H), formed once by k_imp_roe
+        ld4(c.R, e, ra);
+        const xd a[4] = {xd(ra[0]), xd(ra[1]), xd(ra[2]), xd(ra[3])};
+        if (c.steady) lam = lam + (t_sqrt(a[0] * a[0] + a[1] * a[1]) + a[2]) * l;
+        xd am[16];
+        face_jacobians(a[0], a[1], a[2], a[3], GAM, neg_if(nx, side2), neg_if(ny, side2), l, dg, am);
         const bool inner = e < c.n_int;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             double2* o = reinterpret_cast<double2*>(c.O + oblk(nc, i, k, 0, q));
-            o[0] = inner ? make_double2(am[q], am[4 + q]) : make_double2(0.0, 0.0);
-            o[1] = inner ? make_double2(am[8 + q], am[12 + q]) : make_double2(0.0, 0.0);
+            o[0] = inner ? make_double2(am[q].v, am[4 + q].v) : make_double2(0.0, 0.0);
+            o[1] = inner ? make_double2(am[8 + q].v, am[12 + q].v) : make_double2(0.0, 0.0);
         }
     }
-    const double S = c.S[i];
-    double tau;
+    const xd S(c.S[i]);
+    xd tau;
     if (c.steady) {
-        tau = 2.0 * (*c.cfl) * S / (lam + 1.0e-100);
-        c.ctau[i] = tau;
+        tau = xd(2.0) * xd(*c.cfl) * S / (lam + xd(1.0e-100));
+        c.ctau[i] = tau.v;
     } else {
-        tau = c.ctau[i];
+        tau = xd(c.ctau[i]);
     }
-    const double sd = S / tau;
+    const xd sd = S / tau;
 #pragma unroll
     for (int m = 0; m < 16; m++) dg[m] = (m % 5) == 0 ? dg[m] + sd : plus_zero(dg[m]);  // + 0.0 off the diagonal
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         double2* d = reinterpret_cast<double2*>(c.D + dblk(nc, i, 0, q));
-        d[0] = make_double2(dg[q], dg[4 + q]);
-        d[1] = make_double2(dg[8 + q], dg[12 + q]);
+        d[0] = make_double2(dg[q].v, dg[4 + q].v);
+        d[1] = make_double2(dg[8 + q].v, dg[12 + q].v);
     }
-    st4(c.b, i, rhs[0], rhs[1], rhs[2], rhs[3]);
+    st4(c.b, i, rhs[0].v, rhs[1].v, rhs[2].v, rhs[3].v);
 }
 
 __device__ __forceinline__ bool solve_ok(const GmresCtl* g) { return g->final_ && !g->restart && g->status == 0; }
@@ -415,8 +420,9 @@ inline int blocks(int n, int t) { return (n + t - 1) / t; }
 void imp_launch_prims(const ImpCase& c, cudaStream_t s) { k_imp_prims<<<blocks(c.nc, 256), 256, 0, s>>>(c); }
 void imp_launch_grad(const ImpCase& c, cudaStream_t s) { k_imp_grad<<<blocks(c.nc, 256), 256, 0, s>>>(c); }
 void imp_launch_flux(const ImpCase& c, cudaStream_t s) {
-    if (c.flux == FLUX_LAX) k_imp_flux<FLUX_LAX><<<blocks(c.ne, 256), 256, 0, s>>>(c);
-    else k_imp_flux<FLUX_GODUNOV><<<blocks(c.ne, 256), 256, 0, s>>>(c);
+    if (c.flux == FLUX_LAX) k_imp_flux<FLUX_LAX><<<blocks(2 * c.ne, 128), 128, 0, s>>>(c);
+    else k_imp_flux<FLUX_GODUNOV><<<blocks(2 * c.ne, 128), 128, 0, s>>>(c);
+    k_imp_roe<<<blocks(c.ne, 128), 128, 0, s>>>(c);
 }
 void imp_launch_assemble(const ImpCase& c, cudaStream_t s) {
     k_imp_assemble<<<blocks(c.nc, 128), 128, 0, s>>>(c);

@@ -1,0 +1,377 @@
+// IEEE binary64 arithmetic on the integer pipes.
+//
+// GB300's FP64 unit takes two lanes per clock and SM: a warp's FP64 instruction holds it for
+// 16 clocks, in which the SM can issue 64 instructions to its other pipes. The FP64 kernels
+// keep that unit 83-88% busy and the integer pipes under 5%, so an operation formed from about
+// thirty integer instructions is cheaper than the FP64 instruction itself, and the two run side
+// by side. Every function here returns the correctly rounded (to nearest, ties to even) result,
+// the very bits of the FP64 instruction or of the IEEE quotient and square root, so a kernel may
+// form any of its operations on either side.
+//
+// Measured on one SM with all warps resident (clocks per warp operation): product 16.9 native,
+// 13.8 here; with both kinds in flight 8.9 per product.
+//
+// The common path takes operands with 2^-510 <= |x| < 2^510, whose products and quotients
+// stay normal; zeros, and anything else, leave it by a branch.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+namespace cfd2d {
+namespace ip {
+
+typedef unsigned int u32;
+typedef unsigned long long u64;
+
+#if defined(__CUDA_ARCH__)
+#define IP_FN __device__ __forceinline__
+__device__ __forceinline__ u32 hi(double x) { return (u32)__double2hiint(x); }
+__device__ __forceinline__ u32 lo(double x) { return (u32)__double2loint(x); }
+__device__ __forceinline__ double make(u32 h, u32 l) { return __hiloint2double((int)h, (int)l); }
+// low word of (h:l) >> s, 0 <= s < 32
+__device__ __forceinline__ u32 shr2(u32 l, u32 h, u32 s) { return __funnelshift_r(l, h, s); }
+__device__ __forceinline__ u32 shl2(u32 l, u32 h, u32 s) { return __funnelshift_l(l, h, s); }
+__device__ __forceinline__ int clz32(u32 x) { return __clz((int)x); }
+// approximations of 1/x and 1/sqrt(x), within a few units of the 23rd fraction bit
+__device__ __forceinline__ float rcp_seed(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float rsqrt_seed(float x) { float y; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ u32 f2u(float x) { return __float2uint_rz(x); }
+__device__ __forceinline__ float u2f_bits(u32 b) { return __uint_as_float(b); }
+// (qh:ql) + (E << 32), plus one when z > 0x80000000 (z: the bits below the last place with the
+// parity and sticky bit merged into bit 0)
+__device__ __forceinline__ double round_pack(u32 qh, u32 ql, u32 z, u32 E) {
+    u32 h, l;
+    asm("{\n\t.reg .u32 d;\n\tadd.cc.u32 d, %4, 0x7fffffff;\n\taddc.cc.u32 %1, %2, 0;\n\taddc.u32 %0, %3, %5;\n\t}"
+        : "=r"(h), "=r"(l) : "r"(ql), "r"(qh), "r"(z), "r"(E));
+    return make(h, l);
+}
+// the same with the bits below z in `low`: plus one when z:low > 0x80000000:0 (z's bit 0: the parity)
+__device__ __forceinline__ double round_pack2(u32 qh, u32 ql, u32 z, u32 low, u32 E) {
+    u32 h, l;
+    asm("{\n\t.reg .u32 d;\n\tadd.cc.u32 d, %6, 0xffffffff;\n\taddc.cc.u32 d, %4, 0x7fffffff;\n\t"
+        "addc.cc.u32 %1, %2, 0;\n\taddc.u32 %0, %3, %5;\n\t}"
+        : "=r"(h), "=r"(l) : "r"(ql), "r"(qh), "r"(z), "r"(E), "r"(low));
+    return make(h, l);
+}
+#else
+#define IP_FN inline
+inline u64 bits(double x) { u64 b; std::memcpy(&b, &x, 8); return b; }
+inline u32 hi(double x) { return (u32)(bits(x) >> 32); }
+inline u32 lo(double x) { return (u32)bits(x); }
+inline double make(u32 h, u32 l) { const u64 b = ((u64)h << 32) | l; double x; std::memcpy(&x, &b, 8); return x; }
+inline u32 shr2(u32 l, u32 h, u32 s) { return (u32)((((u64)h << 32) | l) >> (s & 31)); }
+inline u32 shl2(u32 l, u32 h, u32 s) { return (u32)(((((u64)h << 32) | l) << (s & 31)) >> 32); }
+inline int clz32(u32 x) { return x ? __builtin_clz(x) : 32; }
+inline u32 f2u(float x) { return (u32)x; }
+inline float u2f_bits(u32 b) { float x; std::memcpy(&x, &b, 4); return x; }
+// off by seed_ulps units in the last place: the results must not depend on the seed
+inline int& seed_ulps() { static int d = 0; return d; }
+inline float nudge(float x) { u32 b; std::memcpy(&b, &x, 4); return u2f_bits(b + (u32)seed_ulps()); }
+inline float rcp_seed(float x) { return nudge(1.0f / x); }
+inline float rsqrt_seed(float x) { return nudge((float)(1.0 / __builtin_sqrt((double)x))); }
+inline double round_pack(u32 qh, u32 ql, u32 z, u32 E) {
+    const u64 q = (((u64)qh << 32) | ql) + (z > 0x80000000u ? 1 : 0) + ((u64)E << 32);
+    return make((u32)(q >> 32), (u32)q);
+}
+inline double round_pack2(u32 qh, u32 ql, u32 z, u32 low, u32 E) { return round_pack(qh, ql, z + (low != 0 ? 1 : 0), E); }
+#endif
+
+IP_FN u64 wide(u32 a, u32 b) { return (u64)a * b; }
+// 2^-510 <= |x| < 2^510
+IP_FN bool in_range(double x) { return (hi(x) << 1) - 0x40200000u < 0x7f800000u; }
+IP_FN u32 mant_hi(double x) { return (hi(x) & 0xfffffu) | 0x100000u; }
+
+// a b for operands in range: the 106-bit product of the significands in four wide
+// multiplications, shifted to 53 bits and rounded.
+IP_FN double mul_core(double a, double b) {
+    const u32 ma = mant_hi(a), mb = mant_hi(b), al = lo(a), bl = lo(b);
+    const u64 p0 = wide(al, bl);
+    u64 t = wide(ma, bl) + (u32)(p0 >> 32);
+    t += wide(al, mb);
+    const u64 p1 = wide(ma, mb) + (u32)(t >> 32);  // 41 or 42 bits
+    const u32 mid = (u32)t, p1l = (u32)p1, p1h = (u32)(p1 >> 32), low = (u32)p0;
+    const u32 s = p1h >> 9, sh = s + 20;
+    const u32 ql = shr2(mid, p1l, sh), qh = shr2(p1l, p1h, sh), rm = shr2(0u, mid, sh);
+    // the sign bits add to their exclusive or, the exponents to the product's
+    const u32 E = (hi(a) & 0xfff00000u) + (hi(b) & 0xfff00000u) + (s << 20) - (1024u << 20);
+    return round_pack2(qh, ql, rm | (ql & 1u), low, E);
+}
+
+// a + b for operands in range whose exponents differ by less than 32; ok: the sum was formed
+// (it was not when 32 or more leading bits cancelled)
+IP_FN double add_core(double a, double b, bool& ok) {
+    const u32 xa = hi(a) & 0x7fffffffu, xb = hi(b) & 0x7fffffffu, al = lo(a), bl = lo(b);
+    const bool sw = xa < xb || (xa == xb && al < bl);
+    const u32 ph = sw ? xb : xa, pl = sw ? bl : al, qh0 = sw ? xa : xb, ql0 = sw ? al : bl;
+    const u32 sgn = (sw ? hi(b) : hi(a)) & 0x80000000u;
+    const u32 e = ph >> 20, d = e - (qh0 >> 20);
+    const u32 mh = (ph & 0xfffffu) | 0x100000u, sh0 = (qh0 & 0xfffffu) | 0x100000u;
+    const u32 Mh = shl2(pl, mh, 10), Ml = pl << 10, sh1 = shl2(ql0, sh0, 10), sl1 = ql0 << 10;
+    const u32 rh = sh1 >> (d & 31u), ext = shr2(0u, sl1, d);
+    const u32 rl = shr2(sl1, sh1, d) | (ext < 1u ? ext : 1u);
+    const u32 neg = (u32)((int)(hi(a) ^ hi(b)) >> 31);
+    const u64 S = (((u64)Mh << 32) | Ml) + (((u64)(rh ^ neg) << 32) | (rl ^ neg)) + (neg & 1u);
+    const u32 Sh = (u32)(S >> 32), Sl = (u32)S;
+    ok = d < 32u && Sh != 0;
+    const u32 z = (u32)clz32(Sh) & 31u;
+    const u32 Nh = shl2(Sl, Sh, z), Nl = Sl << z;
+    const u32 ql = shr2(Nl, Nh, 11), qh = Nh >> 11;
+    return round_pack(qh, ql, (Nl << 21) | (ql & 1u), ((e - z) << 20) + sgn);
+}
+
+// ---- any operands: what the branches above leave to
+
+#if defined(__CUDA_ARCH__)
+#define IP_RARE static __device__ __noinline__
+#else
+#define IP_RARE static inline
+#endif
+
+IP_RARE double mul_rare(double a, double b) {
+    if (in_range(a) && in_range(b)) return mul_core(a, b);
+    return a * b;
+}
+// a zero times a finite number is the signed zero
+IP_FN bool zero_product(double a, double b) {
+    const u32 xa = hi(a) << 1, xb = hi(b) << 1;
+    return ((xa | lo(a)) == 0 && xb < 0xffe00000u) || ((xb | lo(b)) == 0 && xa < 0xffe00000u);
+}
+IP_FN double mul_any(double a, double b) {
+    if (zero_product(a, b)) return make((hi(a) ^ hi(b)) & 0x80000000u, 0u);
+    return mul_rare(a, b);
+}
+IP_RARE double add_rare(double a, double b) {
+    const u32 xa = hi(a) & 0x7fffffffu, xb = hi(b) & 0x7fffffffu;
+    if ((xb | lo(b)) == 0 && xa - 1u < 0x7fefffffu) return a;  // a finite and not zero: a + 0
+    if ((xa | lo(a)) == 0 && xb - 1u < 0x7fefffffu) return b;
+    if (in_range(a) && in_range(b)) {
+        if (xa == xb && lo(a) == lo(b) && ((hi(a) ^ hi(b)) >> 31)) return make(0u, 0u);
+        const u32 ea = xa >> 20, eb = xb >> 20;
+        if (ea >= eb + 55u) return a;  // below a quarter of the last place
+        if (eb >= ea + 55u) return b;
+    }
+    return a + b;
+}
+
+// a b and a + b for any operands
+IP_FN double mul(double a, double b) {
+    if (__builtin_expect(in_range(a) && in_range(b), 1)) return mul_core(a, b);
+    return mul_any(a, b);
+}
+IP_FN double add(double a, double b) {
+    bool ok;
+    const double s = add_core(a, b, ok);
+    if (__builtin_expect(ok && in_range(a) && in_range(b), 1)) return s;
+    return add_rare(a, b);
+}
+IP_FN double neg(double x) { return make(hi(x) ^ 0x80000000u, lo(x)); }
+IP_FN double sub(double a, double b) { return add(a, neg(b)); }
+
+// N products behind one branch: the compiler interleaves them
+template <int N>
+IP_FN void muln(double* r, const double* a, const double* b) {
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < N; k++) ok = ok && in_range(a[k]) && in_range(b[k]);
+    if (__builtin_expect(ok, 1)) {
+#pragma unroll
+        for (int k = 0; k < N; k++) r[k] = mul_core(a[k], b[k]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; k++) r[k] = mul_any(a[k], b[k]);
+    }
+}
+
+// ---- reciprocal, quotient, square root
+
+// 1/m for the significand m of b (1 <= m < 2), Q63, within 4 units: a binary32 seed and two
+// Newton steps in fixed point, the first with a 64-bit significand and a 32-bit reciprocal
+// (error 2^-22 -> 2^-43), the second with both in 64 bits (-> 2^-62).
+// The last bit of a quotient is decided by the guard bits below it unless these lie within the
+// approximation's error of one half; then the exact remainder decides (a quotient of two
+// 53-bit significands is never a tie).
+struct Recip { u32 yh, yl; };
+IP_FN Recip recip_of(double b) {
+    const u32 Bh = shl2(lo(b), mant_hi(b), 11), Bl = lo(b) << 11;  // Q63
+    // seed: 1/(m 2^-31) in [2^30, 2^31)
+    u32 y0 = f2u(rcp_seed(u2f_bits(((Bh >> 8) & 0x7fffffu) | (96u << 23))));
+    y0 = y0 < 0x7fffffffu ? y0 : 0x7fffffffu;
+    const u64 p = wide(Bh, y0) + (u32)(wide(Bl, y0) >> 32);                   // Q62, about 2^62
+    const int e0 = (int)((long long)((1ull << 62) - p) >> 10);                // Q52
+    const u64 y1 = ((u64)y0 << 32) + (u64)(((long long)(int)y0 * e0) >> 20);  // Q63
+    const u32 yh = (u32)(y1 >> 32), yl = (u32)y1;
+    // 1 - m y1 in Q94, modulo 2^64 (the product's lowest 32 bits left out)
+    const u64 q = wide(Bh, yl) + wide(Bl, yh) + ((u64)(Bh * yh) << 32);
+    const int e1 = (int)((long long)(0ull - q) >> 22);                        // Q72
+    const u64 y2 = y1 + (u64)(((long long)(int)yh * e1) >> 40);
+    return Recip{(u32)(y2 >> 32), (u32)y2};
+}
+
+// whether twice the remainder n 2^k - q mb exceeds mb (modulo 2^64; nl: the low 64 bits of n 2^k)
+IP_RARE u32 round_by_remainder(u64 nl, u32 qh, u32 ql, u32 mbh, u32 mbl) {
+    const u64 pr = wide(ql, mbl) + ((u64)(ql * mbh + qh * mbl) << 32);
+    return 2 * (nl - pr) > (((u64)mbh << 32) | mbl) ? 0xffffffffu : 0u;
+}
+
+// 1/b, b in range, y = recip_of(b)
+IP_FN double rcp_core(double b, const Recip& y) {
+    const u32 ql = shr2(y.yl, y.yh, 10), qh = y.yh >> 10;
+    u32 z = y.yl << 22;  // ten guard bits; y is at most 1 unit too small, 2 too large
+    if (__builtin_expect(z - (0x80000000u - (2u << 22)) <= (5u << 22), 0))
+        z = round_by_remainder(0ull, qh, ql, mant_hi(b), lo(b));
+    return round_pack(qh, ql, z, ((2044u << 20) - (hi(b) & 0x7ff00000u)) + (hi(b) & 0x80000000u));
+}
+
+// a/b, both in range, y = recip_of(b)
+IP_FN double quot_core(double a, double b, const Recip& y) {
+    const u32 Ah = shl2(lo(a), mant_hi(a), 11), Al = lo(a) << 11;  // Q63
+    const u64 T = wide(Ah, y.yh) + (u32)(wide(Ah, y.yl) >> 32) + (u32)(wide(Al, y.yh) >> 32);  // Q62, in (2^61, 2^63)
+    const u32 Th = (u32)(T >> 32), Tl = (u32)T;
+    const u32 s = Th >> 30, sh = 9 + s;
+    const u32 ql = shr2(Tl, Th, sh), qh = Th >> sh;
+    u32 z = shr2(0u, Tl, sh);  // nine or ten guard bits; T is within 5 units
+    if (__builtin_expect(z - (0x80000000u - (5u << 23)) <= (10u << 23), 0))
+        z = round_by_remainder((((u64)mant_hi(a) << 32) | lo(a)) << (53 - s), qh, ql, mant_hi(b), lo(b));
+    const u32 E = (hi(a) & 0x7ff00000u) - (hi(b) & 0x7ff00000u) + ((1021u + s) << 20);
+    return round_pack(qh, ql, z, E + ((hi(a) ^ hi(b)) & 0x80000000u));
+}
+
+IP_RARE double quot_rare(double a, double b) {
+    const u32 xa = hi(a) & 0x7fffffffu, xb = hi(b) & 0x7fffffffu;
+    if ((xa | lo(a)) == 0 && xb < 0x7ff00000u && (xb | lo(b)) != 0)  // 0 / b
+        return make((hi(a) ^ hi(b)) & 0x80000000u, 0u);
+    return a / b;
+}
+IP_RARE double rcp_rare(double b) { return 1.0 / b; }
+
+IP_FN double rcp(double b) {
+    if (__builtin_expect(in_range(b), 1)) return rcp_core(b, recip_of(b));
+    return rcp_rare(b);
+}
+IP_FN double quot(double a, double b) {
+    if (__builtin_expect(in_range(a) && in_range(b), 1)) return quot_core(a, b, recip_of(b));
+    return quot_rare(a, b);
+}
+// N quotients by one divisor
+template <int N>
+IP_FN void quotn(double* r, const double* a, double b) {
+    bool ok = in_range(b);
+#pragma unroll
+    for (int k = 0; k < N; k++) ok = ok && in_range(a[k]);
+    if (__builtin_expect(ok, 1)) {
+        const Recip y = recip_of(b);
+#pragma unroll
+        for (int k = 0; k < N; k++) r[k] = quot_core(a[k], b, y);
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; k++) r[k] = quot(a[k], b);
+    }
+}
+
+// square root of a positive x in range: m = x / 2^(2k) in [1, 4), a binary32 seed y of
+// 1/sqrt(m), one Newton step (2^-44), s = m y, and s + (m - s^2) y / 2 from the exact
+// remainder (2^-60); the last bit as for the quotient.
+IP_RARE u32 round_by_square(u64 xl, u32 qh, u32 ql) {
+    const u64 R = xl - (wide(ql, ql) + ((u64)(2 * ql * qh) << 32));  // x 2^j - q^2, below 2 q + 1
+    return R > (((u64)qh << 32) | ql) ? 0xffffffffu : 0u;
+}
+IP_FN double sqrt_core(double x) {
+    const u32 odd = (~hi(x) >> 20) & 1u;  // the exponent without its bias is odd
+    const u32 mh = mant_hi(x), ml = lo(x);
+    const u32 Mh = shl2(ml, mh, 10 + odd), Ml = ml << (10 + odd);  // Q62
+    const u32 y0r = f2u(rsqrt_seed(u2f_bits(((mh << 3) & 0x7fffffu) | (ml >> 29) | ((65u + odd) << 23))));
+    const u32 y0 = y0r < 0x7fffffffu ? y0r : 0x7fffffffu;          // Q31, in (2^30, 2^31)
+    const u64 yy = wide(y0, y0);                                    // Q62
+    const u32 yyh = (u32)(yy >> 32), yyl = (u32)yy;
+    const u64 p = wide(Mh, yyh) + (u32)(wide(Mh, yyl) >> 32) + (u32)(wide(Ml, yyh) >> 32);  // Q60
+    const int e0 = (int)((long long)((1ull << 60) - p) >> 9);      // Q51
+    const u64 y1 = ((u64)y0 << 32) + (u64)(((long long)(int)y0 * e0) >> 20);  // Q63: y0 (1 + e0/2)
+    const u32 yh = (u32)(y1 >> 32), yl = (u32)y1;
+    const u64 s1 = wide(Mh, yh) + (u32)(wide(Mh, yl) >> 32) + (u32)(wide(Ml, yh) >> 32);    // Q61
+    const u32 sh = (u32)(s1 >> 32), sl = (u32)s1;
+    const u64 sq = ((u64)(sh * sh) << 32) + 2 * wide(sh, sl) + (u32)(wide(sl, sl) >> 32);   // Q90, modulo 2^64
+    const u64 M28 = ((u64)shl2(Ml, Mh, 28) << 32) | (Ml << 28);
+    const int r = (int)((long long)(M28 - sq) >> 20);              // Q70
+    const u64 s2 = s1 + (u64)(((long long)(int)yh * r) >> 41);     // r y / 2
+    const u32 Sh = (u32)(s2 >> 32), Sl = (u32)s2;
+    const u32 ql = shr2(Sl, Sh, 9), qh = Sh >> 9;
+    u32 z = Sl << 23;  // nine guard bits
+    if (__builtin_expect(z - (0x80000000u - (4u << 23)) <= (8u << 23), 0))
+        z = round_by_square((((u64)mh << 32) | ml) << (52 + odd), qh, ql);
+    return round_pack(qh, ql, z, ((((hi(x) >> 20) + 1021u) >> 1) << 20));
+}
+IP_RARE double sqrt_rare(double x) { return ::sqrt(x); }
+IP_FN double sqrt(double x) {
+    // positive and in range: the sign bit would put hi(x) above the range
+    if (__builtin_expect(hi(x) - 0x20100000u < 0x3fc00000u, 1)) return sqrt_core(x);
+    return sqrt_rare(x);
+}
+
+// x / 2: exact for normal results and zeros, by the exponent
+IP_FN double half(double x) {
+    const u32 xa = hi(x) & 0x7fffffffu;
+    if (__builtin_expect(xa - 0x00200000u < 0x7fd00000u, 1)) return make(hi(x) - 0x00100000u, lo(x));
+    return (xa | lo(x)) == 0 ? x : mul_rare(x, 0.5);
+}
+// 0 + x: x, with -0 turned into +0
+IP_FN double plus_zero(double x) { return make((hi(x) == 0x80000000u && lo(x) == 0) ? 0u : hi(x), lo(x)); }
+// a/b with y = recip_of(b)
+IP_FN double quot_by(double a, double b, const Recip& y) {
+    if (__builtin_expect(in_range(a) && in_range(b), 1)) return quot_core(a, b, y);
+    return quot_rare(a, b);
+}
+
+#if defined(__CUDACC__)
+// 1.0 in a register the compiler cannot see through. A fused multiply-add of three registers
+// takes 17 clocks of the FP64 unit per warp, an addition, a product, or a multiply-add with an
+// operand from the constant bank, a uniform register or an immediate 20 (measured, one SM, all
+// warps resident). a + b is therefore formed as a * one + b: the same rounding of the same sum.
+__device__ __forceinline__ double one() {
+#if defined(__CUDA_ARCH__)
+    u32 h;
+    asm("{\n\t.reg .u32 m;\n\tmov.u32 m, %%lanemask_eq;\n\tpopc.b32 m, m;\n\tadd.u32 %0, m, 0x3fefffff;\n\t}" : "=r"(h));
+    return make(h, 0u);
+#else
+    return 1.0;
+#endif
+}
+// a constant in a register of its own, for the same reason
+__device__ __forceinline__ double reg(double x) {
+#if defined(__CUDA_ARCH__)
+    u32 z;
+    asm("{\n\t.reg .u32 m;\n\tmov.u32 m, %%lanemask_eq;\n\tpopc.b32 m, m;\n\tsub.u32 %0, m, 1;\n\t}" : "=r"(z));
+    return make(hi(x) + z, lo(x) + z);
+#else
+    return x;
+#endif
+}
+__device__ __forceinline__ double fadd(double a, double b) { return __fma_rn(a, one(), b); }
+__device__ __forceinline__ double fsub(double a, double b) { return __fma_rn(a, one(), neg(b)); }
+
+// A binary64 number whose products, quotients and square roots are formed on the integer
+// pipes and whose sums run on the FP64 unit as multiply-adds: the two sides of a kernel then
+// overlap. Bit for bit the arithmetic of double.
+struct xd {
+    double v;
+    xd() = default;
+    __device__ __forceinline__ explicit xd(double x) : v(x) {}
+    __device__ __forceinline__ explicit operator double() const { return v; }
+};
+__device__ __forceinline__ xd operator+(xd a, xd b) { return xd(fadd(a.v, b.v)); }
+__device__ __forceinline__ xd operator-(xd a, xd b) { return xd(fsub(a.v, b.v)); }
+__device__ __forceinline__ xd operator-(xd a) { return xd(neg(a.v)); }
+__device__ __forceinline__ xd operator*(xd a, xd b) { return xd(mul(a.v, b.v)); }
+__device__ __forceinline__ xd operator/(xd a, xd b) { return xd(quot(a.v, b.v)); }
+__device__ __forceinline__ xd& operator+=(xd& a, xd b) { a = a + b; return a; }
+__device__ __forceinline__ xd& operator-=(xd& a, xd b) { a = a - b; return a; }
+__device__ __forceinline__ bool operator>(xd a, xd b) { return a.v > b.v; }
+__device__ __forceinline__ bool operator<(xd a, xd b) { return a.v < b.v; }
+__device__ __forceinline__ bool operator>=(xd a, xd b) { return a.v >= b.v; }
+__device__ __forceinline__ bool operator<=(xd a, xd b) { return a.v <= b.v; }
+#endif
+
+}  // namespace ip
+}  // namespace cfd2d

@@ -151,6 +151,10 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {  // 
     return x ^ (x >> 31);
 }
 
+__device__ __forceinline__ bool differ(double a, double b) {  // in bits, NaNs being alike
+    return __double_as_longlong(a) != __double_as_longlong(b) && !(a != a && b != b);
+}
+
 __global__ void k_selftest(int which, long long n, unsigned long long seed, unsigned long long* bad) {
     unsigned long long local = 0;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
@@ -166,6 +170,19 @@ __global__ void k_selftest(int which, long long n, unsigned long long seed, unsi
             const double y = 1.0 / b2;
             const double q1 = div_rn(a2, b2, y), q2 = a2 / b2;
             local += __double_as_longlong(q1) != __double_as_longlong(q2);
+            // the integer-pipe operations; c: near a in magnitude, for sums that cancel
+            const unsigned long long r3 = mix64(r2);
+            const unsigned ea = (unsigned)(((unsigned long long)__double_as_longlong(a2) >> 52) & 0x7ff);
+            double c = __longlong_as_double((long long)(((r3 & 1) << 63) | (unsigned long long)((ea + (r3 >> 1) % 70 - 35) & 0x7ff) << 52 |
+                                                        (r1 & 0xfffffffffffffull)));
+            if ((r3 & 0x300) == 0) c = __longlong_as_double(__double_as_longlong(-a2) + (long long)((r3 >> 12) % 5) - 2);
+            const double s = fabs(b2);
+            local += differ(ip::mul(a2, b2), __dmul_rn(a2, b2)) + differ(ip::mul(a2, c), __dmul_rn(a2, c)) +
+                     differ(ip::add(a2, c), __dadd_rn(a2, c)) + differ(ip::sub(a2, b2), __dsub_rn(a2, b2)) +
+                     differ(ip::fadd(a2, c), __dadd_rn(a2, c)) + differ(ip::fsub(a2, c), __dsub_rn(a2, c)) +
+                     differ(ip::rcp(b2), __drcp_rn(b2)) + differ(ip::quot(a2, b2), __ddiv_rn(a2, b2)) +
+                     differ(ip::quot(a2, c), __ddiv_rn(a2, c)) + differ(ip::sqrt(s), __dsqrt_rn(s)) +
+                     differ(ip::half(c), __dmul_rn(c, 0.5)) + differ(ip::plus_zero(c), __dadd_rn(0.0, c));
         } else if (which == 1) {  // widening of random normal floats
             const float f = __uint_as_float((unsigned)(((r1 % 254) + 1) << 23) | (unsigned)(r2 & 0x807fffffu));
             local += __double_as_longlong(widen(f)) != __double_as_longlong((double)f);

@@ -13,7 +13,7 @@ inline int grid_of(const LaunchShape& l, int n) { return l.grid > 0 ? l.grid : n
 template <int FLUX, bool ST>
 void flux_by_recon(const DevCase& c, int recon, cudaStream_t s) {
     const LaunchShape& l = c.shape[KIND_FLUX];
-    const int g = grid_of(l, c.ne), b = l.block;
+    const int b = l.block, g = grid_of(l, c.ne * (sizeof(KT) == 8 && recon != RECON_NONE ? 2 : 1));
     switch (recon) {
     case RECON_NONE: k_flux<KT, FLUX, RECON_NONE, ST><<<g, b, 0, s>>>(c); break;
     case RECON_LINEAR: k_flux<KT, FLUX, RECON_LINEAR, ST><<<g, b, 0, s>>>(c); break;

@@ -14,22 +14,41 @@
 
 #include <cmath>
 
+#include "intpipe.cuh"
 #include "kernels.hpp"
 
 namespace cfd2d {
 
 template <typename T>
 struct Prim { T r, u, v, p; };
+template <typename A, typename T>
+__device__ __forceinline__ Prim<A> prim_as(const Prim<T>& q) { return Prim<A>{A(q.r), A(q.u), A(q.v), A(q.p)}; }
 
 __device__ __forceinline__ double t_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float t_sqrt(float x) { return sqrtf(x); }
-__device__ __forceinline__ double t_exp(double x) { return exp(x); }
-__device__ __forceinline__ float t_exp(float x) { return expf(x); }
-__device__ __forceinline__ double t_log(double x) { return log(x); }
-__device__ __forceinline__ float t_log(float x) { return logf(x); }
 __device__ __forceinline__ double t_abs(double x) { return fabs(x); }
 __device__ __forceinline__ float t_abs(float x) { return fabsf(x); }
 __device__ __forceinline__ double t_fma(double a, double b, double c) { return fma(a, b, c); }
+// FP64 face arithmetic: sums on the FP64 unit, products, quotients and square roots on the
+// integer pipes (intpipe.cuh; the same bits as double's)
+using ip::xd;
+__device__ __forceinline__ xd t_sqrt(xd x) { return xd(ip::sqrt(x.v)); }
+// x^a for positive x (the reference's exp(log(x) a))
+__device__ __forceinline__ xd t_pow(xd x, xd a) { return xd(exp(log(x.v) * a.v)); }
+__device__ __forceinline__ float t_pow(float x, float a) { return expf(logf(x) * a); }
+__device__ __forceinline__ xd t_abs(xd x) { return xd(ip::make(ip::hi(x.v) & 0x7fffffffu, ip::lo(x.v))); }
+__device__ __forceinline__ xd t_fma(xd a, xd b, xd c) { return xd(__fma_rn(a.v, b.v, c.v)); }
+// x / 2 (exact)
+__device__ __forceinline__ float half(float x) { return 0.5f * x; }
+__device__ __forceinline__ double half(double x) { return 0.5 * x; }
+__device__ __forceinline__ xd half(xd x) { return xd(ip::half(x.v)); }
+// the type a face precision computes in
+template <typename T> struct ArithOf { typedef T type; };
+template <> struct ArithOf<double> { typedef xd type; };
+template <typename T> using Arith = typename ArithOf<T>::type;
+// the FP64 type of a form's state update
+template <typename T> struct WideArith { typedef double type; };
+template <> struct WideArith<double> { typedef xd type; };
 __device__ __forceinline__ float t_fma(float a, float b, float c) { return fmaf(a, b, c); }
 template <typename T> __device__ __forceinline__ T t_max(T a, T b) { return a > b ? a : b; }  // _max_, src/mesh/grid.h:102
 template <typename T> __device__ __forceinline__ T t_min(T a, T b) { return a < b ? a : b; }
@@ -99,6 +118,11 @@ __device__ __forceinline__ void st8(T* __restrict__ p, int i, const T* v) {
     st4(p, 2 * i + 1, v[4], v[5], v[6], v[7]);
 }
 
+__device__ __forceinline__ void st8x(double* __restrict__ p, int i, const xd* v) {
+    st4(p, 2 * i, v[0].v, v[1].v, v[2].v, v[3].v);
+    st4(p, 2 * i + 1, v[4].v, v[5].v, v[6].v, v[7].v);
+}
+
 // Per-item data a kernel reads once and no later kernel of the stage reads again (edge
 // geometry, face lists) is loaded with the evict-first hint, so the L2 keeps the cell
 // records the neighbour gathers hit.
@@ -126,6 +150,10 @@ template <> __device__ __forceinline__ MatT<double> matT_of<double>(const DevCas
     const DevMat m = c.cmat ? c.mats[c.cmat[cell]] : c.mat0;
     return MatT<double>{m.M, m.Cv, m.gm1};
 }
+template <> __device__ __forceinline__ MatT<xd> matT_of<xd>(const DevCase& c, int cell) {
+    const MatT<double> m = matT_of<double>(c, cell);
+    return MatT<xd>{xd(m.M), xd(m.Cv), xd(m.gm1)};
+}
 template <> __device__ __forceinline__ MatT<float> matT_of<float>(const DevCase& c, int cell) {
     if (!c.cmat) return MatT<float>{c.mat0_f[0], c.mat0_f[1], c.mat0_f[2]};
     const DevMat m = c.mats[c.cmat[cell]];
@@ -133,9 +161,11 @@ template <> __device__ __forceinline__ MatT<float> matT_of<float>(const DevCase&
 }
 template <typename T> __device__ __forceinline__ T gam_of(const DevCase& c);
 template <> __device__ __forceinline__ double gam_of<double>(const DevCase& c) { return c.gam_flux; }
+template <> __device__ __forceinline__ xd gam_of<xd>(const DevCase& c) { return xd(c.gam_flux); }
 template <> __device__ __forceinline__ float gam_of<float>(const DevCase& c) { return c.gam_flux_f; }
 template <typename T> __device__ __forceinline__ T ig1_of(const DevCase& c);
 template <> __device__ __forceinline__ double ig1_of<double>(const DevCase& c) { return c.ig1_flux; }
+template <> __device__ __forceinline__ xd ig1_of<xd>(const DevCase& c) { return xd(ip::reg(c.ig1_flux)); }
 template <> __device__ __forceinline__ float ig1_of<float>(const DevCase& c) { return c.ig1_flux_f; }
 
 // a / b correctly rounded from y = RN(1/b): q = RN(a y), r = a - b q exactly
@@ -167,10 +197,17 @@ __device__ __forceinline__ double div_rn(double a, double b, double y) {
 __device__ __forceinline__ double neg_if(double x, bool s) {
     return __hiloint2double(__double2hiint(x) ^ (s ? (int)0x80000000 : 0), __double2loint(x));
 }
+__device__ __forceinline__ xd neg_if(xd x, bool s) { return xd(neg_if(x.v, s)); }
 __device__ __forceinline__ float neg_if(float x, bool s) { return __int_as_float(__float_as_int(x) ^ (s ? (int)0x80000000 : 0)); }
 // a / b given y = RN(1/b): the correctly rounded quotient in FP64, a * y in the FP32 faces.
 __device__ __forceinline__ double div_by(double a, double b, double y) { return div_rn(a, b, y); }
 __device__ __forceinline__ float div_by(float a, float, float y) { return a * y; }
+// Quotients by a shared divisor: recip_of the divisor once, div_y per dividend (FP32 divides).
+struct NoRecip {};
+__device__ __forceinline__ NoRecip recip_of(float) { return NoRecip{}; }
+__device__ __forceinline__ float div_y(float a, float b, NoRecip) { return a / b; }
+__device__ __forceinline__ ip::Recip recip_of(xd b) { return ip::recip_of(b.v); }
+__device__ __forceinline__ xd div_y(xd a, xd b, const ip::Recip& y) { return xd(ip::quot_by(a.v, b.v, y)); }
 
 // FP32 <-> FP64 conversions on the integer pipe. GB300's FP64 unit issues ~2
 // instructions per clock and SM, and the hardware conversions run there; these
@@ -205,19 +242,22 @@ template <typename T>
 __device__ __forceinline__ Prim<T> cons2prim(T ro, T ru, T rv, T re, T gm1) {
     Prim<T> q;
     q.r = ro;
-    T E;
     if constexpr (sizeof(T) == 8) {  // the three quotients by ro share one reciprocal
-        const double y = 1.0 / ro;
-        q.u = div_rn(ru, ro, y);
-        q.v = div_rn(rv, ro, y);
-        E = div_rn(re, ro, y);
+        const double n[3] = {ru, rv, re};
+        double d[3];
+        ip::quotn<3>(d, n, ro);
+        const xd u(d[0]), v(d[1]);
+        const xd e = xd(d[2]) - half(u * u + v * v);
+        q.u = d[0];
+        q.v = d[1];
+        q.p = (xd(ro) * e * xd(gm1)).v;
     } else {
         q.u = ru / ro;
         q.v = rv / ro;
-        E = re / ro;
+        const T E = re / ro;
+        T e = E - T(0.5) * (q.u * q.u + q.v * q.v);
+        q.p = q.r * e * gm1;
     }
-    T e = E - T(0.5) * (q.u * q.u + q.v * q.v);
-    q.p = q.r * e * gm1;
     return q;
 }
 
@@ -272,6 +312,8 @@ __device__ __forceinline__ bool mm_pos(double a, double b) {
 __device__ __forceinline__ bool mm_first(double a, double b) {
     return (__double_as_longlong(a) & 0x7fffffffffffffffll) < (__double_as_longlong(b) & 0x7fffffffffffffffll);
 }
+__device__ __forceinline__ bool mm_pos(xd a, xd b) { return mm_pos(a.v, b.v); }
+__device__ __forceinline__ bool mm_first(xd a, xd b) { return mm_first(a.v, b.v); }
 __device__ __forceinline__ bool mm_pos(float a, float b) {
     const int pb = __float_as_int(a * b);
     return pb > 0 && pb <= 0x7f800000;
@@ -286,51 +328,45 @@ __device__ __forceinline__ T minmod(T a, T b) {
 
 // ------------------------------------------------------------------ fluxes
 
-// a / b: from y = RN(1/b) when RECIP (correctly rounded, the same bits as '/', div_rn),
-// else '/' itself; the FP32 faces always divide outright
-template <bool RECIP>
-__device__ __forceinline__ double div_x(double a, double b, double y) { return RECIP ? div_rn(a, b, y) : a / b; }
-template <bool RECIP>
-__device__ __forceinline__ float div_x(float a, float b, float) { return a / b; }
-
 // Exact Riemann solver rim_orig (src/global.cpp:232-405), structured, with a cap
-// on its Newton loop (the reference has none and can spin forever). With RECIP the
-// quotients by the side densities (yRB, yRE = their reciprocals), by the side pressures
-// and by the gas constants go through div_rn: the same bits, a third of the FP64 work of
-// a division each.
-template <typename T, bool RECIP = false>
+// on its Newton loop (the reference has none and can spin forever). yRB, yRE are the side
+// densities' reciprocals (recip_of); the side pressures' and the gas constants' are formed
+// here once for all the quotients by them.
+template <typename T, typename G, typename Y>
 __device__ __forceinline__ bool riemann_exact(T& RI, T& EI, T& PI, T& UI, T& VI, T RB, T PB, T UB, T VB, T RE,
-                                              T PE, T UE, T VE, const RimGas<T>& g, int cap, T yRB = T(0),
-                                              T yRE = T(0)) {
-    const T GAM = g.GAM, AGAM = g.AGAM, DGAM = g.DGAM, GGAM = g.GGAM, HGAM = g.HGAM, FGAM = g.FGAM;
-    const T OGAM = g.OGAM, QGAM = g.QGAM, PGAM = g.PGAM, RGAM = g.RGAM, SGAM = g.SGAM, TGAM = g.TGAM;
+                                              T PE, T UE, T VE, const RimGas<G>& g, int cap, const Y& yRB,
+                                              const Y& yRE) {
+    const T GAM(g.GAM), AGAM(g.AGAM), DGAM(g.DGAM), GGAM(g.GGAM), HGAM(g.HGAM), FGAM(g.FGAM);
+    const T OGAM(g.OGAM), QGAM(g.QGAM), PGAM(g.PGAM), RGAM(g.RGAM), SGAM(g.SGAM), TGAM(g.TGAM);
+    const T E1(g.eAGAM), D1 = T(1.0) + DGAM;
+    const Y yAGAM = recip_of(AGAM), ySGAM = recip_of(SGAM), yD1 = recip_of(D1);
     T US = T(0.0), UF = T(0.0);
     T RF, RS, EF, ES, SBL, SFL, SSL, SEL, D, P;
     const T eps = T(1.0e-5);
-    T CB = t_sqrt(div_x<RECIP>(GAM * PB, RB, yRB));
-    T CE = t_sqrt(div_x<RECIP>(GAM * PE, RE, yRE));
-    T EB = div_x<RECIP>(CB * CB, SGAM, g.iSGAM);
-    T EE = div_x<RECIP>(CE * CE, SGAM, g.iSGAM);
+    T CB = t_sqrt(div_y(GAM * PB, RB, yRB));
+    T CE = t_sqrt(div_y(GAM * PE, RE, yRE));
+    T EB = div_y(CB * CB, SGAM, ySGAM);
+    T EE = div_y(CE * CE, SGAM, ySGAM);
+    const Y yPB = recip_of(PB), yPE = recip_of(PE);
     T RCB = RB * CB;
     T RCE = RE * CE;
     T DU = UB - UE;
     bool hit = false;
-    if (DU < div_x<RECIP>(T(-2.0) * (CB + CE), AGAM, g.iAGAM)) {  // vacuum
+    if (DU < div_y(T(-2.0) * (CB + CE), AGAM, yAGAM)) {  // vacuum
         RF = T(0.0); RS = T(0.0); EF = T(0.0); ES = T(0.0);
         SBL = UB - CB;
-        SFL = UB + div_x<RECIP>(T(2.0) * CB, AGAM, g.iAGAM);
-        SSL = UE - div_x<RECIP>(T(2.0) * CE, AGAM, g.iAGAM);
+        SFL = UB + div_y(T(2.0) * CB, AGAM, yAGAM);
+        SSL = UE - div_y(T(2.0) * CE, AGAM, yAGAM);
         SEL = UE + CE;
     } else {
         P = (PB * RCE + PE * RCB + DU * RCB * RCE) / (RCB + RCE);
-        const T yPB = RECIP ? T(1) / PB : T(0), yPE = RECIP ? T(1) / PE : T(0);
         int it = 0;
         for (;;) {
             T F1, FS1, F2, FS2;
             if (P < eps) P = eps;
-            T PPB = div_x<RECIP>(P, PB, yPB);
+            T PPB = div_y(P, PB, yPB);
             if (PB > P) {
-                T ZFB = CB * t_exp(t_log(PPB) * OGAM);
+                T ZFB = CB * t_pow(PPB, OGAM);
                 F1 = DGAM * (ZFB - CB);
                 FS1 = ZFB / (GAM * P);
             } else {
@@ -339,9 +375,9 @@ __device__ __forceinline__ bool riemann_exact(T& RI, T& EI, T& PI, T& UI, T& VI,
                 F1 = (P - PB) / ZNB;
                 FS1 = (QGAM * PPB + FGAM) / (RGAM * ZNB * PKB);
             }
-            T PPE = div_x<RECIP>(P, PE, yPE);
+            T PPE = div_y(P, PE, yPE);
             if (PE > P) {
-                T ZFE = CE * t_exp(t_log(PPE) * OGAM);
+                T ZFE = CE * t_pow(PPE, OGAM);
                 F2 = DGAM * (ZFE - CE);
                 FS2 = ZFE / (GAM * P);
             } else {
@@ -358,30 +394,30 @@ __device__ __forceinline__ bool riemann_exact(T& RI, T& EI, T& PI, T& UI, T& VI,
         // the reference forms ZFB and ZFE here for both sides; each is read only on its
         // rarefaction branch, so it is formed there (same value, no exp/log for a shock)
         if (!(PB > P)) {
-            D = UB - t_sqrt(div_x<RECIP>(TGAM * P + HGAM * PB, RB, yRB));
+            D = UB - t_sqrt(div_y(TGAM * P + HGAM * PB, RB, yRB));
             T UBD = UB - D, RUBD = RB * UBD;
             RF = RUBD * RUBD / (PB - P + RUBD * UBD);
             UF = D + RUBD / RF;
             EF = P / (AGAM * RF);
             SBL = D; SFL = D;
         } else {
-            const T ZFB = CB * t_exp(t_log(div_x<RECIP>(P, PB, yPB)) * OGAM);
-            EF = div_x<RECIP>(ZFB * ZFB, SGAM, g.iSGAM);
+            const T ZFB = CB * t_pow(div_y(P, PB, yPB), OGAM);
+            EF = div_y(ZFB * ZFB, SGAM, ySGAM);
             UF = UB + DGAM * (CB - ZFB);
             RF = P / (AGAM * EF);
             SBL = UB - CB;
             SFL = UF - ZFB;
         }
         if (!(PE > P)) {
-            D = UE + t_sqrt(div_x<RECIP>(TGAM * P + HGAM * PE, RE, yRE));
+            D = UE + t_sqrt(div_y(TGAM * P + HGAM * PE, RE, yRE));
             T UED = UE - D, RUED = RE * UED;
             RS = RUED * RUED / (PE - P + RUED * UED);
             US = D + RUED / RS;
             ES = P / (AGAM * RS);
             SEL = D; SSL = D;
         } else {
-            const T ZFE = CE * t_exp(t_log(div_x<RECIP>(P, PE, yPE)) * OGAM);
-            ES = div_x<RECIP>(ZFE * ZFE, SGAM, g.iSGAM);
+            const T ZFE = CE * t_pow(div_y(P, PE, yPE), OGAM);
+            ES = div_y(ZFE * ZFE, SGAM, ySGAM);
             US = UE - DGAM * (CE - ZFE);
             RS = P / (AGAM * ES);
             SSL = US + ZFE;
@@ -394,64 +430,66 @@ __device__ __forceinline__ bool riemann_exact(T& RI, T& EI, T& PI, T& UI, T& VI,
         if (US >= T(0.0)) { RI = RF; EI = EF; UI = UF; VI = VB; }
         else { RI = RS; EI = ES; UI = US; VI = VE; }
     } else if (SFL > T(0.0)) {
-        UI = div_x<RECIP>(UB + DGAM * GGAM * t_sqrt(EB), T(1) + DGAM, g.i1DGAM);
+        UI = div_y(UB + DGAM * GGAM * t_sqrt(EB), D1, yD1);
         VI = VB;
-        EI = div_x<RECIP>(UI * UI, SGAM, g.iSGAM);
-        RI = RB * t_exp(t_log(EI / EB) * g.eAGAM);
+        EI = div_y(UI * UI, SGAM, ySGAM);
+        RI = RB * t_pow(EI / EB, E1);
     } else {
-        UI = div_x<RECIP>(UE - DGAM * GGAM * t_sqrt(EE), T(1) + DGAM, g.i1DGAM);
+        UI = div_y(UE - DGAM * GGAM * t_sqrt(EE), D1, yD1);
         VI = VE;
-        EI = div_x<RECIP>(UI * UI, SGAM, g.iSGAM);
-        RI = RE * t_exp(t_log(EI / EE) * g.eAGAM);
+        EI = div_y(UI * UI, SGAM, ySGAM);
+        RI = RE * t_pow(EI / EE, E1);
     }
     PI = AGAM * EI * RI;
     return hit;
 }
 
 // Godunov flux, FVM_TVD::calcFlux, src/methods/fvm_tvd.cpp:602-622 (FEM_RKDG's, :918-937, is
-// the same). With RECIP: a fixed gas and the side densities' reciprocals yL, yR.
-template <typename T, bool RECIP = false>
+// the same). yL, yR: the side densities' reciprocals.
+template <typename T, typename G, typename Y>
 __device__ __forceinline__ bool flux_godunov(T* f, const Prim<T>& L, const Prim<T>& R, T nx, T ny,
-                                             const RimGas<T>& g, int cap, T yL = T(0), T yR = T(0)) {
+                                             const RimGas<G>& g, int cap, const Y& yL, const Y& yR) {
     T RI, EI, PI, UN, UT;
     T unl = L.u * nx + L.v * ny;
     T unr = R.u * nx + R.v * ny;
     T utl = L.u * ny - L.v * nx;
     T utr = R.u * ny - R.v * nx;
-    bool hit = riemann_exact<T, RECIP>(RI, EI, PI, UN, UT, L.r, L.p, unl, utl, R.r, R.p, unr, utr, g, cap, yL, yR);
+    bool hit = riemann_exact<T>(RI, EI, PI, UN, UT, L.r, L.p, unl, utl, R.r, R.p, unr, utr, g, cap, yL, yR);
     T UI = UN * nx + UT * ny;
     T VI = UN * ny - UT * nx;
     f[0] = RI * UN;
     f[1] = f[0] * UI + PI * nx;
     f[2] = f[0] * VI + PI * ny;
-    f[3] = (RI * (EI + T(0.5) * (UI * UI + VI * VI)) + PI) * UN;
+    f[3] = (RI * (EI + half(UI * UI + VI * VI)) + PI) * UN;
     return hit;
 }
 
-template <typename T>
-__device__ __forceinline__ bool flux_godunov(T* f, const Prim<T>& L, const Prim<T>& R, T nx, T ny, T GAM, int cap) {
-    return flux_godunov<T, false>(f, L, R, nx, ny, rim_gas<T>(GAM), cap);
-}
-
 // Lax-Friedrichs (Rusanov), the reference's template src/methods/fvm_tvd_implicit.cpp:939-960
-// (FEM_RKDG's, :938-958, is the same). With RECIP the quotients by the densities use their
-// reciprocals yL, yR (div_rn: the same bits).
-template <typename T, bool RECIP = false>
+// (FEM_RKDG's, :938-958, is the same). yL, yR: the densities' reciprocals (recip_of).
+template <typename T, typename Y>
 __device__ __forceinline__ void flux_lax(T* f, const Prim<T>& L, const Prim<T>& R, T nx, T ny, T GAM, T IG1,
-                                         T yL = T(0), T yR = T(0)) {
+                                         const Y& yL, const Y& yR) {
     T unl = L.u * nx + L.v * ny;
     T unr = R.u * nx + R.v * ny;
-    T alpha = t_max(t_abs(unl) + t_sqrt(div_x<RECIP>(GAM * L.p, L.r, yL)),
-                    t_abs(unr) + t_sqrt(div_x<RECIP>(GAM * R.p, R.r, yR)));
+    T alpha = t_max(t_abs(unl) + t_sqrt(div_y(GAM * L.p, L.r, yL)),
+                    t_abs(unr) + t_sqrt(div_y(GAM * R.p, R.r, yR)));
     T rol = L.r, rul = L.r * L.u, rvl = L.r * L.v;
-    T rel = div_by(L.p, GAM - T(1.0), IG1) + T(0.5) * L.r * (L.u * L.u + L.v * L.v);
     T ror = R.r, rur = R.r * R.u, rvr = R.r * R.v;
-    T rer = div_by(R.p, GAM - T(1.0), IG1) + T(0.5) * R.r * (R.u * R.u + R.v * R.v);
+    T rel, rer;
+    if constexpr (sizeof(T) == 8) {
+        const T G1 = GAM - T(1.0);
+        const Y y1 = recip_of(G1);
+        rel = div_y(L.p, G1, y1) + half(L.r) * (L.u * L.u + L.v * L.v);
+        rer = div_y(R.p, G1, y1) + half(R.r) * (R.u * R.u + R.v * R.v);
+    } else {
+        rel = L.p * IG1 + half(L.r) * (L.u * L.u + L.v * L.v);
+        rer = R.p * IG1 + half(R.r) * (R.u * R.u + R.v * R.v);
+    }
     T frl = rol * unl, frr = ror * unr;
-    f[0] = T(0.5) * (frr + frl - alpha * (ror - rol));
-    f[1] = T(0.5) * (frr * R.u + frl * L.u + (R.p + L.p) * nx - alpha * (rur - rul));
-    f[2] = T(0.5) * (frr * R.v + frl * L.v + (R.p + L.p) * ny - alpha * (rvr - rvl));
-    f[3] = T(0.5) * ((rer + R.p) * unr + (rel + L.p) * unl - alpha * (rer - rel));
+    f[0] = half(frr + frl - alpha * (ror - rol));
+    f[1] = half(frr * R.u + frl * L.u + (R.p + L.p) * nx - alpha * (rur - rul));
+    f[2] = half(frr * R.v + frl * L.v + (R.p + L.p) * ny - alpha * (rvr - rvl));
+    f[3] = half((rer + R.p) * unr + (rel + L.p) * unl - alpha * (rer - rel));
 }
 
 // The fluxes below (HLLC, Roe, the minmod increment) have no counterpart in the
@@ -466,7 +504,7 @@ __device__ __forceinline__ void phys_flux(T* f, T r, T u, T v, T p, T E, T un, T
 }
 template <typename T> __device__ __forceinline__ T dot2(T a, T x, T b, T y) { return t_fma(a, x, b * y); }
 template <typename T> __device__ __forceinline__ T energy(T r, T u, T v, T p, T IG1) {
-    return t_fma(p, IG1, (T(0.5) * r) * t_fma(u, u, v * v));
+    return t_fma(p, IG1, half(r) * t_fma(u, u, v * v));
 }
 
 // Newton-refined quotient, reciprocal and sound speed of the FP64 HLLC flux. HLLC has no
@@ -492,7 +530,7 @@ __device__ __forceinline__ float hllc_seed(double x) {
 // 1/b to ~2^-46 (one Newton step from the binary32 reciprocal of the seed)
 __device__ __forceinline__ double hllc_rcp1(double b) {
     const double y0 = widen(__frcp_rn(hllc_seed(b)));
-    return fma(y0, fma(-b, y0, 1.0), y0);
+    return fma(y0, fma(-b, y0, ip::one()), y0);
 }
 // a / b: one Newton step for 1/b, then q = a y corrected once (|a|, |b| in range; a = 0
 // gives the IEEE signed zero)
@@ -504,7 +542,7 @@ __device__ __forceinline__ double hllc_quot(double a, double b) {
     if (hllc_in_range(b)) {
         if (__builtin_expect(hllc_in_range(a), 1)) {
             const double y = hllc_rcp1(b);
-            const double q = a * y;
+            const double q = ip::mul(a, y);
             return fma(fma(-q, b, a), y, q);
         }
         const long long ia = __double_as_longlong(a);
@@ -513,13 +551,15 @@ __device__ __forceinline__ double hllc_quot(double a, double b) {
     }
     return div_outright(a, b);
 }
+__device__ __forceinline__ xd hllc_quot(xd a, xd b) { return xd(hllc_quot(a.v, b.v)); }
 __device__ __forceinline__ float hllc_quot(float a, float b) { return a / b; }
 // 1/b: two Newton steps
 __device__ __forceinline__ double hllc_recip(double b) {
     if (__builtin_expect(!hllc_in_range(b), 0)) return recip_outright(b);
     const double y = hllc_rcp1(b);
-    return fma(y, fma(-b, y, 1.0), y);
+    return fma(y, fma(-b, y, ip::one()), y);
 }
+__device__ __forceinline__ xd hllc_recip(xd b) { return xd(hllc_recip(b.v)); }
 __device__ __forceinline__ float hllc_recip(float b) { return 1.0f / b; }
 // sqrt(a / r) for a = GAMMA p, r the density (both positive and in range): s0 and
 // h = 1/(2 r s0) from binary32, then two steps s <- s + (a - (r s) s) h
@@ -530,10 +570,11 @@ __device__ __forceinline__ double hllc_sound(double a, double r) {
     const float sf = __fsqrt_rn(__fdiv_rn(af, rf));
     const double h = widen(__fdiv_rn(0.5f, __fmul_rn(rf, sf)));
     double s = widen(sf);
-    s = fma(fma(-(r * s), s, a), h, s);
-    s = fma(fma(-(r * s), s, a), h, s);
+    s = fma(fma(ip::neg(ip::mul(r, s)), s, a), h, s);
+    s = fma(fma(ip::neg(ip::mul(r, s)), s, a), h, s);
     return s;
 }
+__device__ __forceinline__ xd hllc_sound(xd a, xd r) { return xd(hllc_sound(a.v, r.v)); }
 __device__ __forceinline__ float hllc_sound(float a, float r) { return t_sqrt(a / r); }
 
 // HLLC (Toro, Riemann Solvers and Numerical Methods for Fluid Dynamics, sec. 10.4-10.6),
@@ -655,80 +696,77 @@ static __device__ __noinline__ double rsqrt_outright(double x) { return 1.0 / sq
 __device__ __forceinline__ double roe_rsqrt(double x) {
     if (__builtin_expect(__double_as_longlong(x) <= 0 || !hllc_in_range(x), 0)) return rsqrt_outright(x);
     double t = widen(__fdiv_rn(1.0f, __fsqrt_rn(hllc_seed(x))));
-    t = fma(0.5 * t, fma(-(x * t), t, 1.0), t);
-    t = fma(0.5 * t, fma(-(x * t), t, 1.0), t);
+    t = fma(ip::half(t), fma(ip::neg(ip::mul(x, t)), t, ip::one()), t);
+    t = fma(ip::half(t), fma(ip::neg(ip::mul(x, t)), t, ip::one()), t);
     return t;
 }
+__device__ __forceinline__ xd roe_rsqrt(xd x) { return xd(roe_rsqrt(x.v)); }
 static __device__ __noinline__ double sqrt_outright(double x) { return sqrt(x); }
 
 // The Roe flux with FP64 faces, this project's arithmetic (the oracle's flux_roe does the
 // same): the Roe averages from t = 1/sqrt(rho) (sqrt(rho) = rho t, sqrt(rho) H = (E + p) t),
 // c~ = c~^2 t~ and 1/c~^2 = t~^2 with t~ = 1/sqrt(c~^2), the side sound speeds as HLLC's,
 // 1/(sqrt(rho_L) + sqrt(rho_R)) Newton-refined, and the wave sums fused.
-__device__ __forceinline__ void flux_roe(double* f, const Prim<double>& L, const Prim<double>& R, double nx,
-                                         double ny, double GAM, double IG1) {
-    const double G1 = GAM - 1.0;
-    const double unL = dot2(L.u, nx, L.v, ny), unR = dot2(R.u, nx, R.v, ny);
-    const double EL = energy(L.r, L.u, L.v, L.p, IG1), ER = energy(R.r, R.u, R.v, R.p, IG1);
-    const double tL = roe_rsqrt(L.r), tR = roe_rsqrt(R.r);
-    const double sL = L.r * tL, sR = R.r * tR;
-    const double w = hllc_recip(sL + sR);
-    const double ut = fma(sL, L.u, sR * R.u) * w, vt = fma(sL, L.v, sR * R.v) * w;
-    const double Ht = fma(EL + L.p, tL, (ER + R.p) * tR) * w;
-    const double q2 = fma(ut, ut, vt * vt);
-    const double c2 = G1 * fma(-0.5, q2, Ht);
-    double c, ic2;
-    if (__builtin_expect(c2 > 0.0 && hllc_in_range(c2), 1)) {
-        const double t = roe_rsqrt(c2);
+__device__ __forceinline__ void flux_roe(xd* f, const Prim<xd>& L, const Prim<xd>& R, xd nx, xd ny, xd GAM,
+                                         xd IG1) {
+    const xd G1 = GAM - xd(1.0);
+    const xd unL = dot2(L.u, nx, L.v, ny), unR = dot2(R.u, nx, R.v, ny);
+    const xd EL = energy(L.r, L.u, L.v, L.p, IG1), ER = energy(R.r, R.u, R.v, R.p, IG1);
+    const xd tL = roe_rsqrt(L.r), tR = roe_rsqrt(R.r);
+    const xd sL = L.r * tL, sR = R.r * tR;
+    const xd w = hllc_recip(sL + sR);
+    const xd ut = t_fma(sL, L.u, sR * R.u) * w, vt = t_fma(sL, L.v, sR * R.v) * w;
+    const xd Ht = t_fma(EL + L.p, tL, (ER + R.p) * tR) * w;
+    const xd q2 = t_fma(ut, ut, vt * vt);
+    const xd c2 = G1 * t_fma(xd(ip::reg(-0.5)), q2, Ht);
+    xd c, ic2;
+    if (__builtin_expect(c2.v > 0.0 && hllc_in_range(c2.v), 1)) {
+        const xd t = roe_rsqrt(c2);
         c = c2 * t;
         ic2 = t * t;
     } else {
-        c = sqrt_outright(c2);
-        ic2 = recip_outright(c2);
+        c = xd(sqrt_outright(c2.v));
+        ic2 = xd(recip_outright(c2.v));
     }
-    const double unt = dot2(ut, nx, vt, ny);
-    const double rt = sL * sR;
-    const double dr = R.r - L.r, dp = R.p - L.p, dun = unR - unL;
-    const double dtx = fma(-dun, nx, R.u - L.u), dty = fma(-dun, ny, R.v - L.v);
-    const double h = 0.5 * ic2, x = (rt * c) * dun;
-    const double a1 = (dp - x) * h, a2 = fma(-dp, ic2, dr), a4 = (dp + x) * h;
-    const double l1 = unt - c, l4 = unt + c;
-    const double cL = hllc_sound(GAM * L.p, L.r), cR = hllc_sound(GAM * R.p, R.r);
-    const double d1 = t_max(0.0, t_max(l1 - (unL - cL), (unR - cR) - l1));
-    const double d4 = t_max(0.0, t_max(l4 - (unL + cL), (unR + cR) - l4));
-    double al1 = t_abs(l1); if (al1 < d1) al1 = d1;
-    double al4 = t_abs(l4); if (al4 < d4) al4 = d4;
-    const double al2 = t_abs(unt);
-    const double w1 = al1 * a1, w2 = al2 * a2, w4 = al4 * a4, ws = al2 * rt;
-    const double cx = c * nx, cy = c * ny, cu = unt * c;
-    const double D0 = (w1 + w2) + w4;
-    const double D1 = fma(w4, ut + cx, fma(w1, ut - cx, fma(w2, ut, ws * dtx)));
-    const double D2 = fma(w4, vt + cy, fma(w1, vt - cy, fma(w2, vt, ws * dty)));
-    const double D3 = fma(w4, Ht + cu, fma(w1, Ht - cu, fma(0.5 * w2, q2, ws * dot2(ut, dtx, vt, dty))));
-    double FL[4], FR[4];
+    const xd unt = dot2(ut, nx, vt, ny);
+    const xd rt = sL * sR;
+    const xd dr = R.r - L.r, dp = R.p - L.p, dun = unR - unL;
+    const xd dtx = t_fma(-dun, nx, R.u - L.u), dty = t_fma(-dun, ny, R.v - L.v);
+    const xd h = half(ic2), x = (rt * c) * dun;
+    const xd a1 = (dp - x) * h, a2 = t_fma(-dp, ic2, dr), a4 = (dp + x) * h;
+    const xd l1 = unt - c, l4 = unt + c;
+    const xd cL = hllc_sound(GAM * L.p, L.r), cR = hllc_sound(GAM * R.p, R.r);
+    const xd d1 = t_max(xd(0.0), t_max(l1 - (unL - cL), (unR - cR) - l1));
+    const xd d4 = t_max(xd(0.0), t_max(l4 - (unL + cL), (unR + cR) - l4));
+    xd al1 = t_abs(l1); if (al1 < d1) al1 = d1;
+    xd al4 = t_abs(l4); if (al4 < d4) al4 = d4;
+    const xd al2 = t_abs(unt);
+    const xd w1 = al1 * a1, w2 = al2 * a2, w4 = al4 * a4, ws = al2 * rt;
+    const xd cx = c * nx, cy = c * ny, cu = unt * c;
+    const xd D0 = (w1 + w2) + w4;
+    const xd D1 = t_fma(w4, ut + cx, t_fma(w1, ut - cx, t_fma(w2, ut, ws * dtx)));
+    const xd D2 = t_fma(w4, vt + cy, t_fma(w1, vt - cy, t_fma(w2, vt, ws * dty)));
+    const xd D3 = t_fma(w4, Ht + cu, t_fma(w1, Ht - cu, t_fma(half(w2), q2, ws * dot2(ut, dtx, vt, dty))));
+    xd FL[4], FR[4];
     phys_flux(FL, L.r, L.u, L.v, L.p, EL, unL, nx, ny);
     phys_flux(FR, R.r, R.u, R.v, R.p, ER, unR, nx, ny);
-    f[0] = 0.5 * ((FL[0] + FR[0]) - D0);
-    f[1] = 0.5 * ((FL[1] + FR[1]) - D1);
-    f[2] = 0.5 * ((FL[2] + FR[2]) - D2);
-    f[3] = 0.5 * ((FL[3] + FR[3]) - D3);
+    f[0] = half((FL[0] + FR[0]) - D0);
+    f[1] = half((FL[1] + FR[1]) - D1);
+    f[2] = half((FL[2] + FR[2]) - D2);
+    f[3] = half((FL[3] + FR[3]) - D3);
 }
 
-template <typename T, int FLUX>
-__device__ __forceinline__ bool num_flux(T* f, const Prim<T>& L, const Prim<T>& R, T nx, T ny, T GAM, T IG1,
-                                         int cap) {
-    if (FLUX == FLUX_LAX) { flux_lax(f, L, R, nx, ny, GAM, IG1); return false; }
-    if (FLUX == FLUX_ROE) { flux_roe(f, L, R, nx, ny, GAM, IG1); return false; }
-    if (FLUX == FLUX_HLLC) { flux_hllc(f, L, R, nx, ny, GAM, IG1); return false; }
-    return flux_godunov(f, L, R, nx, ny, GAM, cap);
-}
-// The same with the FP64 Riemann solver's gas constants formed once (on the host, in the
-// same operations): FP64 faces use them, FP32 faces form their own per call as before.
+// rg: the exact Riemann solver's gas constants, formed once on the host; FP32 faces form
+// their own per call.
 template <typename T, int FLUX>
 __device__ __forceinline__ bool num_flux(T* f, const Prim<T>& L, const Prim<T>& R, T nx, T ny, T GAM, T IG1,
                                          int cap, const RimGas<double>& rg) {
-    if constexpr (FLUX == FLUX_GODUNOV && sizeof(T) == 8) return flux_godunov<double, false>(f, L, R, nx, ny, rg, cap);
-    return num_flux<T, FLUX>(f, L, R, nx, ny, GAM, IG1, cap);
+    if constexpr (FLUX == FLUX_LAX) flux_lax(f, L, R, nx, ny, GAM, IG1, recip_of(L.r), recip_of(R.r));
+    else if constexpr (FLUX == FLUX_ROE) flux_roe(f, L, R, nx, ny, GAM, IG1);
+    else if constexpr (FLUX == FLUX_HLLC) flux_hllc(f, L, R, nx, ny, GAM, IG1);
+    else if constexpr (sizeof(T) == 8) return flux_godunov(f, L, R, nx, ny, rg, cap, recip_of(L.r), recip_of(R.r));
+    else return flux_godunov(f, L, R, nx, ny, rim_gas<T>(GAM), cap, recip_of(L.r), recip_of(R.r));
+    return false;
 }
 
 // ------------------------------------------------------------------ kernels
@@ -740,8 +778,8 @@ __device__ __forceinline__ bool num_flux(T* f, const Prim<T>& L, const Prim<T>& 
 template <typename T>
 __device__ __forceinline__ void grad_face(T* g, const Prim<T>& q, const Prim<T>& o, T nx, T ny, T l, bool side2) {
     // x * 0.5 is the correctly rounded x / 2 (exact halving), without a division
-    const T hr = (q.r + o.r) * T(0.5), hp = (q.p + o.p) * T(0.5);
-    const T hu = (q.u + o.u) * T(0.5), hv = (q.v + o.v) * T(0.5);
+    const T hr = half(q.r + o.r), hp = half(q.p + o.p);
+    const T hu = half(q.u + o.u), hv = half(q.v + o.v);
     const T v[8] = {hr * nx * l, hr * ny * l, hp * nx * l, hp * ny * l,
                     hu * nx * l, hu * ny * l, hv * nx * l, hv * ny * l};
 #pragma unroll
@@ -754,33 +792,34 @@ __device__ __forceinline__ Prim<T> grad_ghost(const DevCase& c, int i, int e, co
     const T Tc = temperature(q, mt.gm1, mt.Cv);
     return ghost_state(c.bnds[c.ebnd[e]], q, Tc, nx, ny, mt.M);
 }
-// The sum divided by the area through the host-rounded reciprocal (correctly rounded, the
-// reference's division); FP64 faces only (the mixed form's gradients are grad_one_w's).
+// The sum divided by the area (correctly rounded, the reference's division); FP64 faces only
+// (the mixed form's gradients are grad_one_w's).
 template <typename T>
 __device__ __forceinline__ void grad_finish(const DevCase& c, int i, T* g) {
     static_assert(sizeof(T) == 8, "the reference's Green-Gauss rounding is kept in FP64");
-    const double s = c.S[i], y = c.invS[i];  // y = RN(1/S), computed on the host
+    const xd s(c.S[i]);
+    const ip::Recip y = recip_of(s);
 #pragma unroll
-    for (int m = 0; m < 8; m++) g[m] = div_rn(g[m], s, y);
+    for (int m = 0; m < 8; m++) g[m] = div_y(g[m], s, y);
 }
 
-template <typename T>
 __device__ __forceinline__ void grad_one(const DevCase& c, int i) {
     const int nc = c.nc;
-    const T* __restrict__ W = W_of<T>(c);
-    const Prim<T> q = load_prim(W, i);
-    T g[8] = {T(0.0), T(0.0), T(0.0), T(0.0), T(0.0), T(0.0), T(0.0), T(0.0)};
-    const CellFaces<T> cf = cf_of<T>(c);
+    const double* __restrict__ W = c.W64;
+    const Prim<xd> q = prim_as<xd>(load_prim(W, i));
+    xd g[8];
+#pragma unroll
+    for (int m = 0; m < 8; m++) g[m] = xd(0.0);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         const int nb = ldcs(c.cf_nb + k * nc + i);
-        const T nx = ldcs(cf.nx + k * nc + i), ny = ldcs(cf.ny + k * nc + i), l = ldcs(cf.l + k * nc + i);
+        const xd nx(ldcs(c.cf_nx + k * nc + i)), ny(ldcs(c.cf_ny + k * nc + i)), l(ldcs(c.cf_l + k * nc + i));
         const bool side2 = nb >= 0 && (nb & 1);
-        const Prim<T> o = nb >= 0 ? load_prim(W, nb >> 1) : grad_ghost(c, i, -(nb + 1), q, nx, ny);
+        const Prim<xd> o = nb >= 0 ? prim_as<xd>(load_prim(W, nb >> 1)) : grad_ghost(c, i, -(nb + 1), q, nx, ny);
         grad_face(g, q, o, nx, ny, l, side2);
     }
     grad_finish(c, i, g);
-    st8(G_of<T>(c), i, g);
+    st8x(c.G64, i, g);
 }
 
 // The FP64 gradients that minmod reconstructs from (this project's arithmetic, the oracle's
@@ -791,29 +830,43 @@ __device__ __forceinline__ void grad_one(const DevCase& c, int i) {
 __device__ __forceinline__ void grad_one_mm(const DevCase& c, int i) {
     const int nc = c.nc;
     const double* __restrict__ W = c.W64;
-    const Prim<double> q = load_prim(W, i);
-    double g[8];
+    const Prim<xd> q = prim_as<xd>(load_prim(W, i));
+    xd g[8];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         const int nb = ldcs(c.cf_nb + k * nc + i);
         const double ax = ldcs(c.cf_ax + k * nc + i), ay = ldcs(c.cf_ay + k * nc + i);
         const bool side2 = nb >= 0 && (nb & 1);
-        Prim<double> o;
+        Prim<xd> o;
         if (nb >= 0) {
-            o = load_prim(W, nb >> 1);
+            o = prim_as<xd>(load_prim(W, nb >> 1));
         } else {
-            const double nx = ldcs(c.cf_nx + k * nc + i), ny = ldcs(c.cf_ny + k * nc + i);
+            const xd nx(ldcs(c.cf_nx + k * nc + i)), ny(ldcs(c.cf_ny + k * nc + i));
             o = grad_ghost(c, i, -(nb + 1), q, nx, ny);
         }
-        const double sr = q.r + o.r, sp = q.p + o.p, su = q.u + o.u, sv = q.v + o.v;
-        const double v[8] = {sr * ax, sr * ay, sp * ax, sp * ay, su * ax, su * ay, sv * ax, sv * ay};
+        const xd s[4] = {q.r + o.r, q.p + o.p, q.u + o.u, q.v + o.v};
+        // r and p, then u and v each: a velocity that is zero takes only its own products aside
+        double v[8];
+        {
+            const double a[4] = {s[0].v, s[0].v, s[1].v, s[1].v}, b[4] = {ax, ay, ax, ay};
+            ip::muln<4>(v, a, b);
+        }
 #pragma unroll
-        for (int m = 0; m < 8; m++) g[m] = k == 0 ? neg_if(v[m], side2) : g[m] + neg_if(v[m], side2);
+        for (int m = 2; m < 4; m++) {
+            const double a[2] = {s[m].v, s[m].v}, b[2] = {ax, ay};
+            ip::muln<2>(v + 2 * m, a, b);
+        }
+#pragma unroll
+        for (int m = 0; m < 8; m++) g[m] = k == 0 ? neg_if(xd(v[m]), side2) : g[m] + neg_if(xd(v[m]), side2);
     }
     const double y = c.invS[i];
+    double r[8];
 #pragma unroll
-    for (int m = 0; m < 8; m++) g[m] = g[m] * y;
-    st8(c.G64, i, g);
+    for (int m = 0; m < 8; m += 2) {
+        const double a[2] = {g[m].v, g[m + 1].v}, b[2] = {y, y};
+        ip::muln<2>(r + m, a, b);
+    }
+    st8(c.G64, i, r);
 }
 
 // The mixed form's gradients (FP32 faces, every stage path): per face s = q + o and the
@@ -890,13 +943,13 @@ __global__ void __launch_bounds__(256) k_grad(const DevCase c) {
         if (i0 < c.nc) {
             if constexpr (MM) grad_one_mm(c, i0);
             else if constexpr (sizeof(T) == 4) grad_one_w(c, i0);
-            else grad_one<T>(c, i0);
+            else grad_one(c, i0);
         }
     } else {
         for (int i = i0; i < c.nc; i += gridDim.x * blockDim.x) {  // persistent grid
             if constexpr (MM) grad_one_mm(c, i);
             else if constexpr (sizeof(T) == 4) grad_one_w(c, i);
-            else grad_one<T>(c, i);
+            else grad_one(c, i);
         }
     }
 }
@@ -918,12 +971,12 @@ __device__ __forceinline__ unsigned mm_code(T a, T b) {
 }
 // Returns minmod's branches for r, p, u, v (2 bits each, in that order; 0 without minmod),
 // which the adjoint's recorded path reads instead of recomputing them.
-template <typename T, int RECON>
-__device__ __forceinline__ unsigned reconstruct(Prim<T>& q, const T* g, T dx, T dy, const Prim<T>& dq) {
-    T dr = proj<T, RECON>(g[0], g[1], dx, dy);
-    T dp = proj<T, RECON>(g[2], g[3], dx, dy);
-    T du = proj<T, RECON>(g[4], g[5], dx, dy);
-    T dv = proj<T, RECON>(g[6], g[7], dx, dy);
+template <typename T, int RECON, typename G>
+__device__ __forceinline__ unsigned reconstruct(Prim<T>& q, const G* g, T dx, T dy, const Prim<T>& dq) {
+    T dr = proj<T, RECON>(T(g[0]), T(g[1]), dx, dy);
+    T dp = proj<T, RECON>(T(g[2]), T(g[3]), dx, dy);
+    T du = proj<T, RECON>(T(g[4]), T(g[5]), dx, dy);
+    T dv = proj<T, RECON>(T(g[6]), T(g[7]), dx, dy);
     unsigned code = 0;
     if (RECON == RECON_MINMOD) {
         code = mm_code(dr, dq.r) | mm_code(dp, dq.p) << 2 | mm_code(du, dq.u) << 4 | mm_code(dv, dq.v) << 6;
@@ -979,63 +1032,65 @@ __device__ __forceinline__ bool edge_inner(const DevCase& c, int e) {
     return SIDE == EDGE_INNER ? true : (SIDE == EDGE_BOUNDARY ? false : e < c.n_int);
 }
 template <typename T, int FLUX, int RECON, bool REC = false, int SIDE = EDGE_ANY>
-__device__ __forceinline__ void flux_core(const DevCase& c, int e, int c1, const Prim<T>& qL, const T* gL,
-                                          const Prim<T>& qR, const T* gR, T* out, const EdgeGeo<T>& geo,
+__device__ __forceinline__ void flux_core(const DevCase& c, int e, int c1, const Prim<T>& qL_, const T* gL,
+                                          const Prim<T>& qR_, const T* gR, T* out, const EdgeGeo<T>& geo,
                                           const FluxRec& rec = FluxRec{}) {
+    typedef Arith<T> A;
+    const Prim<A> qL = prim_as<A>(qL_), qR = prim_as<A>(qR_);
     static_assert(!REC || FLUX == FLUX_HLLC, "flux records are kept for HLLC");
     // qR: the second cell's primitives on interior edges (e < n_int), qL on boundary edges
-    const T nx = geo.nx, ny = geo.ny, l = geo.l;
-    const T GAM = gam_of<T>(c), IG1 = ig1_of<T>(c);
+    const A nx(geo.nx), ny(geo.ny), l(geo.l);
+    const A GAM = gam_of<A>(c), IG1 = ig1_of<A>(c);
     const bool inner = edge_inner<SIDE>(c, e);
-    Prim<T> gc = qL;
+    Prim<A> gc = qL;
     DevBnd b{};
-    T Tc = T(0), M = T(0);
+    A Tc = A(0), M = A(0);
     if (!inner) {
         b = c.bnds[c.ebnd[e]];
-        const MatT<T> mt = matT_of<T>(c, c1);
+        const MatT<A> mt = matT_of<A>(c, c1);
         Tc = temperature(qL, mt.gm1, mt.Cv);
         M = mt.M;
         if (RECON == RECON_MINMOD) gc = ghost_state(b, qL, Tc, nx, ny, M);
     }
     // minmod's neighbour-minus-centre differences of both sides: formed once per edge in
     // FP64 (the FP64 pipe is the bound there); per Gauss point in FP32 (fewer live registers)
-    Prim<T> dL = qL, dR = qL;
+    Prim<A> dL = qL, dR = qL;
     if (RECON == RECON_MINMOD && sizeof(T) == 8) {
-        const Prim<T>& nb = inner ? qR : gc;
+        const Prim<A>& nb = inner ? qR : gc;
         dL.r = nb.r - qL.r; dL.u = nb.u - qL.u; dL.v = nb.v - qL.v; dL.p = nb.p - qL.p;
         dR.r = neg_if(dL.r, true); dR.u = neg_if(dL.u, true); dR.v = neg_if(dL.v, true); dR.p = neg_if(dL.p, true);
     }
-    T fs[4] = {T(0.0), T(0.0), T(0.0), T(0.0)};
+    A fs[4] = {A(0.0), A(0.0), A(0.0), A(0.0)};
     bool hit = false;
     unsigned codes = 0;
 #pragma unroll
     for (int gp = 0; gp < 2; gp++) {
-        Prim<T> pL = qL, pR;
+        Prim<A> pL = qL, pR;
         if (RECON == RECON_MINMOD && sizeof(T) == 4) {
-            const Prim<T>& nb = inner ? qR : gc;
+            const Prim<A>& nb = inner ? qR : gc;
             dL.r = nb.r - qL.r; dL.u = nb.u - qL.u; dL.v = nb.v - qL.v; dL.p = nb.p - qL.p;
             dR.r = qL.r - qR.r; dR.u = qL.u - qR.u; dR.v = qL.v - qR.v; dR.p = qL.p - qR.p;
         }
         if (RECON != RECON_NONE)
-            codes |= reconstruct<T, RECON>(pL, gL, geo.dl[4 * gp], geo.dl[4 * gp + 1], dL) << (16 * gp);
+            codes |= reconstruct<A, RECON>(pL, gL, A(geo.dl[4 * gp]), A(geo.dl[4 * gp + 1]), dL) << (16 * gp);
         if (inner) {
             pR = qR;
             if (RECON != RECON_NONE)
-                codes |= reconstruct<T, RECON>(pR, gR, geo.dl[4 * gp + 2], geo.dl[4 * gp + 3], dR) << (16 * gp + 8);
+                codes |= reconstruct<A, RECON>(pR, gR, A(geo.dl[4 * gp + 2]), A(geo.dl[4 * gp + 3]), dR) << (16 * gp + 8);
         } else {
             pR = ghost_state(b, pL, Tc, nx, ny, M);
         }
-        T f[4];
+        A f[4];
         if constexpr (REC) {
-            const T cL = hllc_sound(GAM * pL.p, pL.r), cR = hllc_sound(GAM * pR.p, pR.r);
-            T* v = static_cast<T*>(rec.v) + (size_t)(10 * gp) * c.ne + e;
+            const A cL = hllc_sound(GAM * pL.p, pL.r), cR = hllc_sound(GAM * pR.p, pR.r);
+            A* v = static_cast<A*>(rec.v) + (size_t)(10 * gp) * c.ne + e;
             const size_t ne = c.ne;
             v[0] = pL.r; v[ne] = pL.u; v[2 * ne] = pL.v; v[3 * ne] = pL.p;
             v[4 * ne] = pR.r; v[5 * ne] = pR.u; v[6 * ne] = pR.v; v[7 * ne] = pR.p;
             v[8 * ne] = cL; v[9 * ne] = cR;
             flux_hllc_c(f, pL, pR, cL, cR, nx, ny, IG1);
         } else {
-            hit |= num_flux<T, FLUX>(f, pL, pR, nx, ny, GAM, IG1, c.newton_cap, c.rg_flux);
+            hit |= num_flux<A, FLUX>(f, pL, pR, nx, ny, GAM, IG1, c.newton_cap, c.rg_flux);
         }
         // the reference's fluxes sum the Gauss points from +0 (its fSum = 0; fSum += F); this
         // project's own fluxes (HLLC, Roe) start from the first point's flux
@@ -1051,8 +1106,8 @@ __device__ __forceinline__ void flux_core(const DevCase& c, int e, int c1, const
     }
     if constexpr (REC) rec.bits[e] = codes;
     if (hit) atomicOr(c.err, ERRBIT_NEWTON_CAP);
-    const T lh = l * T(0.5);
-    out[0] = fs[0] * lh; out[1] = fs[1] * lh; out[2] = fs[2] * lh; out[3] = fs[3] * lh;
+    const A lh = half(l);
+    out[0] = T(fs[0] * lh); out[1] = T(fs[1] * lh); out[2] = T(fs[2] * lh); out[3] = T(fs[3] * lh);
 }
 
 // The flux of edge e (what F holds for it) from the stage's W and G (with REC: and its record).
@@ -1169,10 +1224,100 @@ __global__ void __launch_bounds__(256, 3) k_flux_pipe(const DevCase c) {
     cp_async_wait<0>();
 }
 
+// The FP64 flux with reconstruction, two lanes per edge: lane gp evaluates Gauss point gp,
+// the pair adds its points' fluxes by shuffle and each lane writes two of the four
+// components. One thread for both points holds twice the state (199 registers, 8 warps on an
+// SM: the FP64 unit then waits for the integer chains of two warps per scheduler); the bits
+// are the same, a sum of two having no order. Called by whole warps; live is false past the
+// last edge. With REC (HLLC) the point leaves its record (FluxRec).
+template <int FLUX, int RECON, bool REC = false>
+__device__ __forceinline__ void flux_lane(const DevCase& c, int e, int gp, bool live, const FluxRec& rec = FluxRec{}) {
+    static_assert(RECON != RECON_NONE && (!REC || FLUX == FLUX_HLLC), "");
+    const double* __restrict__ W = c.W64;
+    const double* __restrict__ G = c.G64;
+    const size_t ne = c.ne;
+    const bool inner = e < c.n_int;
+    const int c1 = ldcs(c.ec1 + e), c2 = inner ? ldcs(c.ec2 + e) : c1;
+    const double* __restrict__ dl = c.dl + (size_t)(4 * gp) * ne + e;
+    const xd nx(ldcs(c.nx + e)), ny(ldcs(c.ny + e));
+    const Prim<xd> qL = prim_as<xd>(load_prim(W, c1));
+    Prim<xd> pL = qL, pR;
+    unsigned codes = 0;
+    xd f[4];
+    bool hit = false;
+    {
+        DevBnd b{};
+        xd Tc(0.0), M(0.0);
+        Prim<xd> o;  // across the edge: the second cell, or the centre state's ghost
+        if (inner) {
+            o = prim_as<xd>(load_prim(W, c2));
+        } else {
+            b = c.bnds[c.ebnd[e]];
+            const MatT<xd> mt = matT_of<xd>(c, c1);
+            Tc = temperature(qL, mt.gm1, mt.Cv);
+            M = mt.M;
+            o = RECON == RECON_MINMOD ? ghost_state(b, qL, Tc, nx, ny, M) : qL;
+        }
+        Prim<xd> d = qL;
+        if (RECON == RECON_MINMOD) d = Prim<xd>{o.r - qL.r, o.u - qL.u, o.v - qL.v, o.p - qL.p};
+        double g[8];
+        ld8(G, c1, g);
+        codes = reconstruct<xd, RECON>(pL, g, xd(ldcs(dl)), xd(ldcs(dl + ne)), d);
+        if (inner) {
+            pR = o;
+            if (RECON == RECON_MINMOD) d = Prim<xd>{-d.r, -d.u, -d.v, -d.p};
+            ld8(G, c2, g);
+            codes |= reconstruct<xd, RECON>(pR, g, xd(ldcs(dl + 2 * ne)), xd(ldcs(dl + 3 * ne)), d) << 8;
+        } else {
+            pR = ghost_state(b, pL, Tc, nx, ny, M);
+        }
+    }
+    const xd GAM = gam_of<xd>(c), IG1 = ig1_of<xd>(c);
+    if constexpr (REC) {
+        const xd cL = hllc_sound(GAM * pL.p, pL.r), cR = hllc_sound(GAM * pR.p, pR.r);
+        if (live) {
+            double* v = static_cast<double*>(rec.v) + (size_t)(10 * gp) * ne + e;
+            v[0] = pL.r.v; v[ne] = pL.u.v; v[2 * ne] = pL.v.v; v[3 * ne] = pL.p.v;
+            v[4 * ne] = pR.r.v; v[5 * ne] = pR.u.v; v[6 * ne] = pR.v.v; v[7 * ne] = pR.p.v;
+            v[8 * ne] = cL.v; v[9 * ne] = cR.v;
+        }
+        flux_hllc_c(f, pL, pR, cL, cR, nx, ny, IG1);
+        const unsigned both = __shfl_xor_sync(0xffffffffu, codes, 1);
+        if (live && gp == 0) rec.bits[e] = codes | both << 16;
+    } else {
+        hit = num_flux<xd, FLUX>(f, pL, pR, nx, ny, GAM, IG1, c.newton_cap, c.rg_flux);
+    }
+    if (hit && live) atomicOr(c.err, ERRBIT_NEWTON_CAP);
+    const xd lh = half(xd(ldcs(c.l + e)));
+    double out[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        double mine = gp ? f[2 + k].v : f[k].v;
+        double other = __shfl_xor_sync(0xffffffffu, gp ? f[k].v : f[2 + k].v, 1);
+        // the reference's fluxes sum the Gauss points from +0 (its fSum = 0; fSum += F); this
+        // project's own fluxes (HLLC, Roe) start from the first point's flux
+        if (FLUX != FLUX_HLLC && FLUX != FLUX_ROE) (gp ? other : mine) = ip::plus_zero(gp ? other : mine);
+        out[k] = ((xd(mine) + xd(other)) * lh).v;
+    }
+    if (live) reinterpret_cast<double2*>(c.F64)[2 * (size_t)e + gp] = make_double2(out[0], out[1]);
+}
+
+template <typename T, int RECON> constexpr int kFluxMinBlocks = sizeof(T) == 8 && RECON != RECON_NONE ? 3 : 0;
+
+// k_flux: FP64 with reconstruction two lanes per edge, else one thread per edge
+template <typename T, int RECON> struct FluxLanes { static constexpr int n = sizeof(T) == 8 && RECON != RECON_NONE ? 2 : 1; };
+
 template <typename T, int FLUX, int RECON, bool STRIDE>
-__global__ void __launch_bounds__(256) k_flux(const DevCase c) {
+__global__ void __launch_bounds__(256, kFluxMinBlocks<T, RECON>) k_flux(const DevCase c) {
     const int e0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if constexpr (!STRIDE) {  // one thread per item
+    if constexpr (FluxLanes<T, RECON>::n == 2) {
+        const int n = 2 * c.ne;
+        for (int t = e0; (t & ~31) < n; t += gridDim.x * blockDim.x) {
+            const bool live = t < n;
+            flux_lane<FLUX, RECON>(c, live ? t >> 1 : c.ne - 1, t & 1, live);
+            if (!STRIDE) break;
+        }
+    } else if constexpr (!STRIDE) {  // one thread per item
         if (e0 < c.ne) flux_one<T, FLUX, RECON>(c, e0);
     } else {
         for (int e = e0; e < c.ne; e += gridDim.x * blockDim.x) flux_one<T, FLUX, RECON>(c, e);  // persistent grid
@@ -1209,14 +1354,16 @@ __device__ __forceinline__ void gather_residual(const DevCase& c, int i, double*
     const int nc = c.nc;
     const T* __restrict__ F = F_of<T>(c);
     if constexpr (sizeof(T) == 8) {
-        R[0] = 0.0; R[1] = 0.0; R[2] = 0.0; R[3] = 0.0;
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const int f = c.face[k * nc + i];
             double v[4];
             ld4(F, f >> 1, v);
 #pragma unroll
-            for (int q = 0; q < 4; q++) R[q] = R[q] + neg_if(v[q], !(f & 1));
+            for (int q = 0; q < 4; q++) {
+                const double t = neg_if(v[q], !(f & 1));
+                R[q] = k == 0 ? ip::plus_zero(t) : ip::fadd(R[q], t);  // 0 -/+ F first
+            }
         }
     } else {
         float t[3][4];
@@ -1247,10 +1394,10 @@ __device__ __forceinline__ Prim<float> prim_face_of<float>(double ro, double ru,
 
 // local time step of one cell (calcTimeStep STEADY branch, src/methods/fvm_tvd.cpp:218-224)
 __device__ __forceinline__ void local_dt(const DevCase& c, int i, const Prim<double>& q, const DevMat& mt) {
-    double cz = sqrt(mt.gam * q.p / q.r);
-    double t = c.cfl_number * c.S[i] / t_max(fabs(q.u) + cz, fabs(q.v) + cz);
-    c.ctau_next[i] = t;
-    c.cfl[i] = t / c.S[i];
+    const xd cz = t_sqrt(xd(mt.gam) * xd(q.p) / xd(q.r)), S(c.S[i]);
+    const xd t = xd(c.cfl_number) * S / t_max(t_abs(xd(q.u)) + cz, t_abs(xd(q.v)) + cz);
+    c.ctau_next[i] = t.v;
+    c.cfl[i] = (t / S).v;
 }
 
 template <typename T>
@@ -1298,29 +1445,29 @@ template <typename T, int SCHEME, int STAGE>
 __device__ __forceinline__ void update_finish(const DevCase& c, int i, const double* R, T* __restrict__ Wout) {
     constexpr bool FINAL = StageKind<SCHEME, STAGE>::FINAL;
     const int nc = c.nc;
-    const double cf = c.cfl[i];
+    // FP64 faces: products on the integer pipes. The mixed form's update streams at the rate of
+    // DRAM and its meshes are often small: there the FP64 unit's shorter latency counts.
+    typedef typename WideArith<T>::type D;
+    const D cf(c.cfl[i]);
     const double* __restrict__ src = STAGE == 0 ? c.A : c.B;
-    double u0 = src[i] + cf * R[0], u1 = src[nc + i] + cf * R[1], u2 = src[2 * nc + i] + cf * R[2],
-           u3 = src[3 * nc + i] + cf * R[3];
     double* dst = FINAL ? c.A : c.B;
-    if (SCHEME == TIME_SSPRK3) {
-        // SSP-RK3 (not in the reference) with fused multiply-adds: X + cf R, then
-        // 3/4 U^n + 1/4 X and 1/3 U^n + 2/3 X (the Euler and Heun stages stay unfused: the
-        // reference's U += cTau/S R)
-        u0 = fma(cf, R[0], src[i]); u1 = fma(cf, R[1], src[nc + i]);
-        u2 = fma(cf, R[2], src[2 * nc + i]); u3 = fma(cf, R[3], src[3 * nc + i]);
-        if (STAGE == 1) {
-            u0 = fma(0.25, u0, 0.75 * c.A[i]); u1 = fma(0.25, u1, 0.75 * c.A[nc + i]);
-            u2 = fma(0.25, u2, 0.75 * c.A[2 * nc + i]); u3 = fma(0.25, u3, 0.75 * c.A[3 * nc + i]);
-        } else if (STAGE == 2) {
-            const double c13 = 1.0 / 3.0, c23 = 2.0 / 3.0;
-            u0 = fma(c23, u0, c13 * c.A[i]); u1 = fma(c23, u1, c13 * c.A[nc + i]);
-            u2 = fma(c23, u2, c13 * c.A[2 * nc + i]); u3 = fma(c23, u3, c13 * c.A[3 * nc + i]);
+    D u[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const D x(src[k * nc + i]), r(R[k]);
+        if (SCHEME == TIME_SSPRK3) {
+            // SSP-RK3 (not in the reference) with fused multiply-adds: X + cf R, then
+            // 3/4 U^n + 1/4 X and 1/3 U^n + 2/3 X (the Euler and Heun stages stay unfused: the
+            // reference's U += cTau/S R)
+            u[k] = t_fma(cf, r, x);
+            if (STAGE == 1) u[k] = t_fma(D(ip::reg(0.25)), u[k], D(0.75) * D(c.A[k * nc + i]));
+            else if (STAGE == 2) u[k] = t_fma(D(ip::reg(2.0 / 3.0)), u[k], D(1.0 / 3.0) * D(c.A[k * nc + i]));
+        } else {
+            u[k] = x + cf * r;
+            if (SCHEME == TIME_HEUN && STAGE == 1) u[k] = half(D(c.A[k * nc + i]) + u[k]);
         }
-    } else if (SCHEME == TIME_HEUN && STAGE == 1) {
-        u0 = 0.5 * (c.A[i] + u0); u1 = 0.5 * (c.A[nc + i] + u1);
-        u2 = 0.5 * (c.A[2 * nc + i] + u2); u3 = 0.5 * (c.A[3 * nc + i] + u3);
     }
+    const double u0(u[0]), u1(u[1]), u2(u[2]), u3(u[3]);
     dst[i] = u0; dst[nc + i] = u1; dst[2 * nc + i] = u2; dst[3 * nc + i] = u3;
     const Prim<T> w = prim_face_of<T>(u0, u1, u2, u3, c, i);
     store_prim(Wout, i, w);

@@ -40,11 +40,10 @@ struct DevBnd {     // one <boundCond>: kind and (Vx, Vy, T, P)
 };
 
 // The constants rim_orig derives from GAM (src/global.cpp:240-250), formed as it forms
-// them; a caller with a fixed gas forms them once. iAGAM, iSGAM, i1DGAM are RN(1/AGAM),
-// RN(1/SGAM), RN(1/(1 + DGAM)) for the quotients by them (div_x), eAGAM is 1/AGAM as the
-// reference writes it in the sonic-rarefaction exponent.
+// them; a caller with a fixed gas forms them once. eAGAM is 1/AGAM as the reference writes it
+// in the sonic-rarefaction exponent.
 template <typename T> struct RimGas {
-    T GAM, AGAM, DGAM, GGAM, HGAM, FGAM, OGAM, QGAM, PGAM, RGAM, SGAM, TGAM, iAGAM, iSGAM, i1DGAM, eAGAM;
+    T GAM, AGAM, DGAM, GGAM, HGAM, FGAM, OGAM, QGAM, PGAM, RGAM, SGAM, TGAM, eAGAM;
 };
 template <typename T>
 __host__ __device__ __forceinline__ RimGas<T> rim_gas(T GAM) {
@@ -65,9 +64,6 @@ __host__ __device__ __forceinline__ RimGas<T> rim_gas(T GAM) {
     g.RGAM = (T(4.0) * GAM);
     g.SGAM = (GAM * g.AGAM);
     g.TGAM = (g.QGAM / T(2.0));
-    g.iAGAM = T(1) / g.AGAM;
-    g.iSGAM = T(1) / g.SGAM;
-    g.i1DGAM = T(1) / (T(1) + g.DGAM);
     g.eAGAM = T(1) / g.AGAM;
     return g;
 }
@@ -247,7 +243,7 @@ void launch_objective_grad(const DevCase& c, const AdjCase& a, const double* w, 
                            cudaStream_t s);
 
 // built-in checks of the arithmetic helpers against the hardware operations
-// (which: 0 div_rn vs '/', 1 widen vs (double), 2 narrow vs (float) within 1 ulp)
+// (which: 0 div_rn vs '/' and the integer-pipe operations of intpipe.cuh, 1 widen vs (double), 2 narrow vs (float) within 1 ulp)
 long long selftest_arith(int which, long long n, unsigned long long seed);
 // deterministic FP64 sums of S*U over cells (mass, x/y momentum, energy)
 void launch_conservation(const DevCase& c, double* partial, int nblocks, cudaStream_t s);

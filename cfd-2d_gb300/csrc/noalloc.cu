@@ -71,14 +71,15 @@ __global__ void __launch_bounds__(256) k_static_edge_flux(const StaticArgs a) {
         const double Tc = temperature(qL, a.mat.gm1, a.mat.Cv);
         qR = ghost_state(a.b[bi], qL, Tc, nx, ny, a.mat.M);
     }
-    double f[4];
-    num_flux<double, FLUX>(f, qL, qR, nx, ny, a.gam, 1.0 / (a.gam - 1.0), 100);
-    const double lh = l * 0.5;
+    xd f[4];
+    num_flux<xd, FLUX>(f, prim_as<xd>(qL), prim_as<xd>(qR), xd(nx), xd(ny), xd(a.gam), xd(1.0 / (a.gam - 1.0)), 100,
+                       rim_gas<double>(a.gam));
+    const xd lh = half(xd(l));
     for (int k = 0; k < 4; k++) {  // both Gauss points see the same states
-        double s = 0.0;
+        xd s(0.0);
         s = s + f[k];
         s = s + f[k];
-        a.F[(size_t)k * ne + e] = s * lh;
+        a.F[(size_t)k * ne + e] = (s * lh).v;
     }
 }
 

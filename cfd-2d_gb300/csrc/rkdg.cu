@@ -1,7 +1,7 @@
 // Device code of FEM_RKDG (src/methods/fem_rkdg.cpp). Built with -fmad=false: every
 // product and sum rounds on its own, in the reference's order, so the FP64 results equal
-// the reference's bit for bit (the quotients by the density and the cell sizes are
-// correctly rounded, div_rn; the polynomial sums start from +0 as VECTOR::SCALAR_PROD's).
+// the reference's bit for bit (products, quotients and roots on the integer pipes are
+// correctly rounded, intpipe.cuh; the polynomial sums start from +0 as VECTOR::SCALAR_PROD's).
 #include "rkdg.hpp"
 
 #include "kernels.cuh"
@@ -14,6 +14,8 @@ __device__ __forceinline__ double pz(double x) {
     const long long b = __double_as_longlong(x);
     return __longlong_as_double(b == (long long)0x8000000000000000ull ? 0ll : b);
 }
+
+__device__ __forceinline__ xd pz(xd x) { return xd(pz(x.v)); }
 
 __device__ __forceinline__ DgMat dmat(const DgCase& c, int cell) { return c.cmat ? c.mats[c.cmat[cell]] : c.mat0; }
 
@@ -32,99 +34,115 @@ __device__ __forceinline__ void store12(double* __restrict__ U, int i, const dou
     for (int k = 0; k < 6; k++) p[k] = make_double2(a[2 * k], a[2 * k + 1]);
 }
 
-struct DgPar { double r, u, v, E, p, y; };
+struct DgPar { xd r, u, v, E, p; ip::Recip y; };
 
 // convertConsToPar (:1420-1430) through URS(0)'s pressure: each variable's polynomial at a
 // point (SCALAR_PROD from s = 0 with the basis (1, F1, F2), src/global.h:128-135), u, v, E
-// by r (:1422-1425), e, p = r e (gam - 1) (src/global.cpp:15-17). y = RN(1/r).
+// by r (:1422-1425), e, p = r e (gam - 1) (src/global.cpp:15-17). y = recip_of(r).
 __device__ __forceinline__ DgPar dg_eval(const double* a, double F1, double F2, double gm1) {
-    double s[4];
+    xd s[4];
 #pragma unroll
     for (int v = 0; v < 4; v++) {
-        double t = pz(a[3 * v]);  // 0 + a0 * 1.0
-        t = t + a[3 * v + 1] * F1;
-        t = t + a[3 * v + 2] * F2;
-        s[v] = t;
+        double pr[2];
+        const double x[2] = {a[3 * v + 1], a[3 * v + 2]}, y[2] = {F1, F2};
+        ip::muln<2>(pr, x, y);
+        s[v] = xd(pz(a[3 * v])) + xd(pr[0]) + xd(pr[1]);  // 0 + a0 * 1.0 first
     }
     DgPar q;
     q.r = s[0];
-    q.y = 1.0 / q.r;
-    q.u = div_rn(s[1], q.r, q.y);
-    q.v = div_rn(s[2], q.r, q.y);
-    q.E = div_rn(s[3], q.r, q.y);
-    const double e = q.E - 0.5 * (q.u * q.u + q.v * q.v);
-    q.p = q.r * e * gm1;
+    q.y = recip_of(q.r);
+    q.u = div_y(s[1], q.r, q.y);
+    q.v = div_y(s[2], q.r, q.y);
+    q.E = div_y(s[3], q.r, q.y);
+    const xd e = q.E - half(q.u * q.u + q.v * q.v);
+    q.p = q.r * e * xd(gm1);
     return q;
 }
 
-// calcConvectionSurf (:995-1122), one thread per edge: both sides at each Gauss point, the
-// flux (calcFlux :918-960; boundaryCond :1324-1343 for a boundary edge), the sides'
-// integrals sum_g (F w) f in Gauss-point order, times edgeJ.
+// calcConvectionSurf (:995-1122), one lane per edge and Gauss point: GE neighbouring lanes
+// share an edge (three points: ten edges and two idle lanes in a warp). A lane evaluates both
+// sides' polynomials at its point and the flux there (calcFlux :918-960; boundaryCond
+// :1324-1343 for a boundary edge); the lanes then exchange their fluxes and divide the sides'
+// integrals sum_g (F w) f, in Gauss-point order, times edgeJ, among themselves: with three
+// lanes one basis function each, with two one side each. One thread for all of an edge's
+// points needs 255 registers (8 warps on an SM) and leaves the FP64 unit waiting.
 template <int FLUX, int GE>
-__global__ void __launch_bounds__(128) k_dg_edge(const DgCase c, const double* __restrict__ U) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= c.ne) return;
+__global__ void __launch_bounds__(128, 5) k_dg_edge(const DgCase c, const double* __restrict__ U) {
+    constexpr int PER_WARP = 32 / GE;  // edges
+    const int lane = threadIdx.x & 31, g = lane % GE, first = lane - g;
+    const long long e0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * PER_WARP + lane / GE;
+    const bool live = lane < PER_WARP * GE && e0 < c.ne;
+    const int e = live ? (int)e0 : c.ne - 1;
     const int c1 = c.ec1[e], c2 = c.ec2[e];
     const bool inner = c2 >= 0;
-    double a1[12], a2[12];
-    load12(U, c1, a1);
-    if (inner) load12(U, c2, a2);
-    const DgMat m1 = dmat(c, c1);
-    const double gm2 = inner ? dmat(c, c2).gm1 : 0.0;
-    const double nx = c.enx[e], ny = c.eny[e];
-    double i1[12], i2[12];
-    bool hit = false;
-#pragma unroll
-    for (int g = 0; g < GE; g++) {
-        const double2* Fp = reinterpret_cast<const double2*>(c.eF + ((size_t)e * GE + g) * 4);
-        const double2 Fa = __ldg(Fp), Fb = __ldg(Fp + 1);
-        const DgPar L = dg_eval(a1, Fa.x, Fa.y, m1.gm1);
-        const Prim<double> qL{L.r, L.u, L.v, L.p};
-        Prim<double> qR;
-        double yR;
+    const xd nx(c.enx[e]), ny(c.eny[e]);
+    const double* eF = c.eF + (size_t)e * GE * 4;
+    xd f[4];
+    {
+        const double2 Fa = __ldg(reinterpret_cast<const double2*>(eF + 4 * g));
+        const DgMat m1 = dmat(c, c1);
+        double a[12];
+        load12(U, c1, a);
+        const DgPar L = dg_eval(a, Fa.x, Fa.y, m1.gm1);
+        const Prim<xd> qL{L.r, L.u, L.v, L.p};
+        Prim<xd> qR;
+        ip::Recip yR;
         if (inner) {
-            const DgPar R = dg_eval(a2, Fb.x, Fb.y, gm2);
-            qR = Prim<double>{R.r, R.u, R.v, R.p};
+            const double2 Fb = __ldg(reinterpret_cast<const double2*>(eF + 4 * g + 2));
+            load12(U, c2, a);
+            const DgPar R = dg_eval(a, Fb.x, Fb.y, dmat(c, c2).gm1);
+            qR = Prim<xd>{R.r, R.u, R.v, R.p};
             yR = R.y;
         } else {
             // URS(1) of pL (:1428) gives the temperature an outlet or wall ghost carries
-            const double Tc = temperature(qL, m1.gm1, m1.Cv);
-            qR = ghost_state(c.bnds[c.ebnd[e]], qL, Tc, nx, ny, m1.M);
-            yR = 1.0 / qR.r;
+            const xd Tc = temperature(qL, xd(m1.gm1), xd(m1.Cv));
+            qR = ghost_state(c.bnds[c.ebnd[e]], qL, Tc, nx, ny, xd(m1.M));
+            yR = recip_of(qR.r);
         }
-        double f[4];
-        if (FLUX == FLUX_GODUNOV) hit |= flux_godunov<double, true>(f, qL, qR, nx, ny, m1.rg, c.newton_cap, L.y, yR);
-        else flux_lax<double, true>(f, qL, qR, nx, ny, m1.gam, m1.ig1, L.y, yR);
-        const double w = c.egw[g];
-        const double w1[3] = {w, GE == 2 ? Fa.x : Fa.x * w, GE == 2 ? Fa.y : Fa.y * w};  // getF(c1, pt) * w (w = 1 for 2 points)
+        bool hit = false;
+        if (FLUX == FLUX_GODUNOV) hit = flux_godunov(f, qL, qR, nx, ny, m1.rg, c.newton_cap, L.y, yR);
+        else flux_lax(f, qL, qR, nx, ny, xd(m1.gam), xd(m1.ig1), L.y, yR);
+        if (hit && live) atomicOr(c.err, ERRBIT_NEWTON_CAP);
+    }
+    // the fluxes of all the edge's points; past the warp's last edge a lane reads its own
+    xd fg[GE][4];
+#pragma unroll
+    for (int q = 0; q < GE; q++)
+#pragma unroll
+        for (int v = 0; v < 4; v++)
+            fg[q][v] = xd(__shfl_sync(0xffffffffu, f[v].v, lane < PER_WARP * GE ? first + q : lane));
+    if (!live) return;
+    const xd J(c.edgeJ[e]);
+    // integral of basis function k over one side (getF(c, pt) * w, w = 1 for two points)
+    auto integral = [&](int side, int k, int v) {
+        xd t(0.0);
+#pragma unroll
+        for (int q = 0; q < GE; q++) {
+            const xd w(c.egw[q]);
+            xd wf = w;
+            if (k > 0) {
+                const xd F(__ldg(eF + 4 * q + 2 * side + k - 1));
+                wf = GE == 2 ? F : F * w;
+            }
+            const xd x = wf * fg[q][v];
+            t = q == 0 ? pz(x) : t + x;
+        }
+        return (t * J).v;
+    };
+    if (GE == 3) {
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+            c.E1[12 * (size_t)e + 3 * v + g] = integral(0, g, v);
+            if (inner) c.E2[12 * (size_t)e + 3 * v + g] = integral(1, g, v);
+        }
+    } else if (g == 0 || inner) {
+        double out[12];
 #pragma unroll
         for (int v = 0; v < 4; v++)
 #pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const double t = w1[k] * f[v];
-                i1[3 * v + k] = g == 0 ? pz(t) : i1[3 * v + k] + t;
-            }
-        if (inner) {
-            const double w2[3] = {w, GE == 2 ? Fb.x : Fb.x * w, GE == 2 ? Fb.y : Fb.y * w};
-#pragma unroll
-            for (int v = 0; v < 4; v++)
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    const double t = w2[k] * f[v];
-                    i2[3 * v + k] = g == 0 ? pz(t) : i2[3 * v + k] + t;
-                }
-        }
+            for (int k = 0; k < 3; k++) out[3 * v + k] = integral(g, k, v);
+        store12(g == 0 ? c.E1 : c.E2, e, out);
     }
-    const double J = c.edgeJ[e];
-#pragma unroll
-    for (int k = 0; k < 12; k++) i1[k] = i1[k] * J;
-    store12(c.E1, e, i1);
-    if (inner) {
-#pragma unroll
-        for (int k = 0; k < 12; k++) i2[k] = i2[k] * J;
-        store12(c.E2, e, i2);
-    }
-    if (hit) atomicOr(c.err, ERRBIT_NEWTON_CAP);
 }
 
 // max over a warp's non-negative doubles (as ordered bits), then one atomic per warp
@@ -155,7 +173,7 @@ __device__ __forceinline__ unsigned long long pos_bits(double x) {
 // calcNewFields (:1216-1242) / calcNewFields2 (:1244-1284). Stage 1 reads A and writes B;
 // stage 2 reads B (and A) and writes A.
 template <int GC>
-__global__ void __launch_bounds__(128) k_dg_cell(const DgCase c, int stage, int with_res) {
+__global__ void __launch_bounds__(128, 5) k_dg_cell(const DgCase c, int stage, int with_res) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = i < c.nc;
     unsigned long long rb[4] = {0, 0, 0, 0};
@@ -163,22 +181,22 @@ __global__ void __launch_bounds__(128) k_dg_cell(const DgCase c, int stage, int 
         double a[12];
         load12(stage == 1 ? c.A : c.B, i, a);
         const DgMat m = dmat(c, i);
-        const double ihx = c.ih[2 * (size_t)i], ihy = c.ih[2 * (size_t)i + 1];
-        double in[12];
+        const xd ihx(c.ih[2 * (size_t)i]), ihy(c.ih[2 * (size_t)i + 1]);
+        xd in[12];
 #pragma unroll
         for (int g = 0; g < GC; g++) {
             const double2 F = __ldg(reinterpret_cast<const double2*>(c.cF) + (size_t)i * GC + g);
             const DgPar q = dg_eval(a, F.x, F.y, m.gm1);
-            const double fr = q.r * q.u;
-            const double fu = fr * q.u + q.p;
-            const double fv = fr * q.v;
-            const double fe = q.u * (q.r * q.E + q.p);
-            const double gr = q.r * q.v;
-            const double gu = gr * q.u;
-            const double gv = gr * q.v + q.p;
-            const double ge = q.v * (q.r * q.E + q.p);
-            const double fx[4] = {fr, fu, fv, fe}, gy[4] = {gr, gu, gv, ge};
-            const double w = c.cgw[g];
+            const xd fr = q.r * q.u;
+            const xd fu = fr * q.u + q.p;
+            const xd fv = fr * q.v;
+            const xd fe = q.u * (q.r * q.E + q.p);
+            const xd gr = q.r * q.v;
+            const xd gu = gr * q.u;
+            const xd gv = gr * q.v + q.p;
+            const xd ge = q.v * (q.r * q.E + q.p);
+            const xd fx[4] = {fr, fu, fv, fe}, gy[4] = {gr, gu, gv, ge};
+            const xd w(c.cgw[g]);
             // tmpInt = 0; += getDFDX * f = (0, 1/HX, 0) f; += getDFDY * g = (0, 0, 1/HY) g; *= w.
             // With finite fluxes the products by 0 are +-0 and every sum with them is exact:
             // component 1 is 0 + f/HX (pz), component 2 is 0 + g/HY, component 0 is +-0 after
@@ -187,25 +205,25 @@ __global__ void __launch_bounds__(128) k_dg_cell(const DgCase c, int stage, int 
             bool finite = true;
 #pragma unroll
             for (int v = 0; v < 4; v++)
-                finite = finite && ((__double2hiint(fx[v]) & 0x7ff00000) != 0x7ff00000) &&
-                         ((__double2hiint(gy[v]) & 0x7ff00000) != 0x7ff00000);
+                finite = finite && ((__double2hiint(fx[v].v) & 0x7ff00000) != 0x7ff00000) &&
+                         ((__double2hiint(gy[v].v) & 0x7ff00000) != 0x7ff00000);
             if (finite) {
 #pragma unroll
                 for (int v = 0; v < 4; v++) {
-                    const double t1 = pz(ihx * fx[v]) * w;
-                    const double t2 = pz(ihy * gy[v]) * w;
-                    if (g == 0) in[3 * v] = 0.0;
+                    const xd t1 = pz(ihx * fx[v]) * w;
+                    const xd t2 = pz(ihy * gy[v]) * w;
+                    if (g == 0) in[3 * v] = xd(0.0);
                     in[3 * v + 1] = g == 0 ? pz(t1) : in[3 * v + 1] + t1;
                     in[3 * v + 2] = g == 0 ? pz(t2) : in[3 * v + 2] + t2;
                 }
             } else {
 #pragma unroll
                 for (int v = 0; v < 4; v++) {
-                    double t0 = 0.0 + 0.0 * fx[v];
-                    double t1 = 0.0 + ihx * fx[v];
-                    double t2 = 0.0 + 0.0 * fx[v];
-                    t0 = t0 + 0.0 * gy[v];
-                    t1 = t1 + 0.0 * gy[v];
+                    xd t0 = xd(0.0) + xd(0.0) * fx[v];
+                    xd t1 = xd(0.0) + ihx * fx[v];
+                    xd t2 = xd(0.0) + xd(0.0) * fx[v];
+                    t0 = t0 + xd(0.0) * gy[v];
+                    t1 = t1 + xd(0.0) * gy[v];
                     t2 = t2 + ihy * gy[v];
                     t0 = t0 * w; t1 = t1 * w; t2 = t2 * w;
                     in[3 * v] = g == 0 ? pz(t0) : in[3 * v] + t0;
@@ -214,8 +232,8 @@ __global__ void __launch_bounds__(128) k_dg_cell(const DgCase c, int stage, int 
                 }
             }
         }
-        const double J = c.cellJ[i];
-        double R[12];
+        const xd J(c.cellJ[i]);
+        xd R[12];
 #pragma unroll
         for (int k = 0; k < 12; k++) R[k] = pz(in[k] * J);  // ro_int (0) += intRO * cellJ
 #pragma unroll
@@ -226,28 +244,28 @@ __global__ void __launch_bounds__(128) k_dg_cell(const DgCase c, int stage, int 
             if (fw & 1) {
                 load12(c.E2, e, s);
 #pragma unroll
-                for (int k = 0; k < 12; k++) R[k] = R[k] + s[k];
+                for (int k = 0; k < 12; k++) R[k] = R[k] + xd(s[k]);
             } else {
                 load12(c.E1, e, s);
 #pragma unroll
-                for (int k = 0; k < 12; k++) R[k] = R[k] - s[k];
+                for (int k = 0; k < 12; k++) R[k] = R[k] - xd(s[k]);
             }
         }
         const double* Mi = c.invA + 9 * (size_t)i;
         double M[9];
 #pragma unroll
         for (int k = 0; k < 9; k++) M[k] = __ldg(Mi + k);
-        const double ct = c.ctau[i];
+        const xd ct(c.ctau[i]);
         double out[12];
 #pragma unroll
         for (int v = 0; v < 4; v++)
 #pragma unroll
             for (int r = 0; r < 3; r++) {
-                double t = pz(M[3 * r] * R[3 * v]);  // VECTOR *= matr: tmp = 0; += m_rj e_j
-                t = t + M[3 * r + 1] * R[3 * v + 1];
-                t = t + M[3 * r + 2] * R[3 * v + 2];
+                xd t = pz(xd(M[3 * r]) * R[3 * v]);  // VECTOR *= matr: tmp = 0; += m_rj e_j
+                t = t + xd(M[3 * r + 1]) * R[3 * v + 1];
+                t = t + xd(M[3 * r + 2]) * R[3 * v + 2];
                 t = t * ct;
-                out[3 * v + r] = a[3 * v + r] + t;
+                out[3 * v + r] = (xd(a[3 * v + r]) + t).v;
             }
         if (stage == 1) {
             store12(c.B, i, out);
@@ -262,7 +280,7 @@ __global__ void __launch_bounds__(128) k_dg_cell(const DgCase c, int stage, int 
 #pragma unroll
             for (int k = 0; k < 12; k++) {
                 const double o = shared ? out[k] : old[k];
-                res[k] = (out[k] + o) * 0.5;
+                res[k] = half(xd(out[k]) + xd(o)).v;
             }
             store12(c.A, i, res);
             // a non-positive or NaN cell-mean density or energy is reported (the state is
@@ -304,9 +322,9 @@ __global__ void __launch_bounds__(128) k_dg_tstep(const DgCase c) {
         double maxU = 0.0;
         auto visit = [&](double F1, double F2) {
             const DgPar q = dg_eval(a, F1, F2, m.gm1);
-            const double cz = sqrt(div_rn(m.gam * q.p, q.r, q.y));  // URS(0)
-            const double Uv = sqrt(q.u * q.u + q.v * q.v) + cz;    // magU() + cz
-            if (maxU < Uv) maxU = Uv;
+            const xd cz = t_sqrt(div_y(xd(m.gam) * q.p, q.r, q.y));    // URS(0)
+            const xd Uv = t_sqrt(q.u * q.u + q.v * q.v) + cz;          // magU() + cz
+            if (maxU < Uv.v) maxU = Uv.v;
         };
 #pragma unroll
         for (int g = 0; g < GC; g++) {
@@ -367,7 +385,7 @@ inline int blocks(long long n, int b) { return (int)((n + b - 1) / b); }
 }  // namespace
 
 void dg_launch_edges(const DgCase& c, int flux, const double* U, cudaStream_t s) {
-    const int nb = blocks(c.ne, 128);
+    const int nb = blocks(c.ne, 4 * (32 / c.ge));  // four warps of 32 / ge edges
     if (flux == FLUX_LAX) {
         if (c.ge == 3) k_dg_edge<FLUX_LAX, 3><<<nb, 128, 0, s>>>(c, U);
         else k_dg_edge<FLUX_LAX, 2><<<nb, 128, 0, s>>>(c, U);
