@@ -310,6 +310,126 @@ IP_FN double sqrt(double x) {
     return sqrt_rare(x);
 }
 
+// ---- x^a
+
+// 64 intervals of the significand m: c = kLogC / 1024 >= 1/m at the interval's left end, so
+// that r = m c - 1 is exact and 0 <= r < 2^-5; kLogT = -log2(c), Q62; kExpT = 2^(i/64), Q63.
+#if defined(__CUDA_ARCH__)
+#define IP_TABLE static __device__ const
+#else
+#define IP_TABLE static const
+#endif
+IP_TABLE unsigned short kLogC[64] = {
+    1024, 1009, 993, 979, 964, 950, 937, 924, 911, 898, 886, 874, 863, 852, 841, 830,
+    820, 810, 800, 790, 781, 772, 763, 754, 745, 737, 729, 721, 713, 705, 698, 690,
+    683, 676, 669, 662, 656, 649, 643, 637, 631, 625, 619, 613, 607, 602, 596, 591,
+    586, 580, 575, 570, 565, 561, 556, 551, 547, 542, 538, 533, 529, 525, 521, 517};
+IP_TABLE u64 kLogT[64] = {
+    0x0000000000000000ull, 0x015ccece78a4a9e2ull, 0x02d6a1c52f5f99c0ull, 0x0426417de5c11ef5ull,
+    0x0593389b019c55adull, 0x06ed040be494e4f1ull, 0x0832b45fc2bb59adull, 0x097cf196adfee84dull,
+    0x0acbdcb3bc4e88faull, 0x0c1f98266e2d535cull, 0x0d5d9654f63a3931ull, 0x0e9feaa1d256ae3dull,
+    0x0fcb4bf9de86679dull, 0x10fa848044b35108ull, 0x122dadc2ab3496d2ull, 0x1364e2511cc820cfull,
+    0x148365e695d796aaull, 0x15a56d7a370ded62ull, 0x16cb0f6865c8ea03ull, 0x17f462e58e168828ull,
+    0x1903372e90bee3f2ull, 0x1a152f142981b3d7ull, 0x1b2a5d6f51ff82b2ull, 0x1c42d5c4c688b3cfull,
+    0x1d5eac4d463d7de1ull, 0x1e5dddf7e46e0a54ull, 0x1f5fd8a9063e3490ull, 0x2064ac1d23cb3bc1ull,
+    0x216c68978eb5cdfaull, 0x22771ee8884eb752ull, 0x2362fd0935b84c2cull, 0x2473772407798668ull,
+    0x25647ca36738f606ull, 0x2657fdc6e1dcd0cbull, 0x274e07ca1f49be5aull, 0x2846a853ae553ba8ull,
+    0x291dde3262f321a8ull, 0x2a1b72da09d5469aull, 0x2af6fd70071f5e6cull, 0x2bd496ee30ab9accull,
+    0x2cb4494dab9de792ull, 0x2d961ed0cb91d406ull, 0x2e7a2205e5813045ull, 0x2f605dca45dfdfb6ull,
+    0x3048dd4d4c00d553ull, 0x310c600e275bf88full, 0x31f92499135908dfull, 0x32c04702422a3142ull,
+    0x33891a8be56a4a25ull, 0x347c5e95887ec06bull, 0x35490566b9539d52ull, 0x361775c932bace07ull,
+    0x36e7b7cd16b43760ull, 0x378fa7d29bdb897aull, 0x386344fba0169378ull, 0x3938cb84d4664657ull,
+    0x39e503e2be17ce3aull, 0x3abe11f27f31124aull, 0x3b6d29207b2970ddull, 0x3c49dd15d3e18a0eull,
+    0x3cfbebfca715669dull, 0x3daf54df46b1e14eull, 0x3e641d088b6533daull, 0x3f1a49e2a175d53aull};
+IP_TABLE u64 kExpT[64] = {
+    0x8000000000000000ull, 0x8164d1f3bc030773ull, 0x82cd8698ac2ba1d7ull, 0x843a28c3acde4046ull,
+    0x85aac367cc487b14ull, 0x871f61969e8d1010ull, 0x88980e8092da8527ull, 0x8a14d575496efd9aull,
+    0x8b95c1e3ea8bd6e6ull, 0x8d1adf5b7e5ba9e5ull, 0x8ea4398b45cd53c0ull, 0x9031dc431466b1dcull,
+    0x91c3d373ab11c336ull, 0x935a2b2f13e6e92bull, 0x94f4efa8fef70961ull, 0x96942d3720185a00ull,
+    0x9837f0518db8a96full, 0x99e0459320b7fa64ull, 0x9b8d39b9d54e5538ull, 0x9d3ed9a72cffb750ull,
+    0x9ef5326091a111adull, 0xa0b0510fb9714fc2ull, 0xa27043030c496818ull, 0xa43515ae09e6809eull,
+    0xa5fed6a9b15138eaull, 0xa7cd93b4e9653569ull, 0xa9a15ab4ea7c0ef8ull, 0xab7a39b5a93ed337ull,
+    0xad583eea42a14ac6ull, 0xaf3b78ad690a4374ull, 0xb123f581d2ac258full, 0xb311c412a9112489ull,
+    0xb504f333f9de6484ull, 0xb6fd91e328d17791ull, 0xb8fbaf4762fb9ee9ull, 0xbaff5ab2133e45fbull,
+    0xbd08a39f580c36beull, 0xbf1799b67a731082ull, 0xc12c4cca66709456ull, 0xc346ccda24976407ull,
+    0xc5672a115506daddull, 0xc78d74c8abb9b15cull, 0xc9b9bd866e2f27a2ull, 0xcbec14fef2727c5cull,
+    0xce248c151f8480e3ull, 0xd06333daef2b2594ull, 0xd2a81d91f12ae45aull, 0xd4f35aabcfedfa1full,
+    0xd744fccad69d6af4ull, 0xd99d15c278afd7b5ull, 0xdbfbb797daf23755ull, 0xde60f4825e0e9123ull,
+    0xe0ccdeec2a94e111ull, 0xe33f8972be8a5a51ull, 0xe5b906e77c8348a8ull, 0xe8396a503c4bdc68ull,
+    0xeac0c6e7dd24392eull, 0xed4f301ed9942b84ull, 0xefe4b99bdcdaf5cbull, 0xf281773c59ffb139ull,
+    0xf5257d152486cc2cull, 0xf7d0df730ad13bb8ull, 0xfa83b2db722a033aull, 0xfd3e0c0cf486c174ull};
+#undef IP_TABLE
+
+// high 64 bits of a b, at most 3 too small
+IP_FN u64 mulhi(u64 a, u64 b) {
+    const u32 ah = (u32)(a >> 32), al = (u32)a, bh = (u32)(b >> 32), bl = (u32)b;
+    return wide(ah, bh) + (u32)(wide(ah, bl) >> 32) + (u32)(wide(al, bh) >> 32);
+}
+IP_FN u32 mulhi32(u32 a, u32 b) { return (u32)(wide(a, b) >> 32); }
+
+// x^a for x in range and positive, 2^-20 <= a < 4 (in [2^-500, 2^500] as a result), within
+// 0.54 units in the last place: log2 and exp2 by tables of 64 entries and polynomials (the
+// scheme of Tang, ACM TOMS 15 (1989) and 16 (1990)) in fixed point, the products of the high
+// terms in 32 bits. The coefficients are Taylor's.
+IP_FN double pow_core(double x, double a) {
+    // a in Q61
+    const u32 ea = hi(a) >> 20;  // 1003 .. 1024
+    const u64 am = ((u64)shl2(lo(a), mant_hi(a), 10) << 32) | (lo(a) << 10);  // Q62 of [1, 2)
+    const u64 A = am >> (1024u - ea);                                           // Q61: a = am 2^(ea-1023-62)
+    // log2(x) = e + F, F in Q62
+    const u32 xh = hi(x), i = (xh >> 14) & 63u, c = kLogC[i];
+    const u64 m0 = wide(lo(x), c);
+    const u64 m1 = wide(mant_hi(x), c) + (u32)(m0 >> 32);
+    const u64 R = ((m1 << 32) | (u32)m0) - (1ull << 62);  // r, Q62
+    const u64 rs = R << 6;                                  // Q68
+    const u32 rh = (u32)(rs >> 32);                         // Q36
+    u32 p = 2626u;                                     // Q14
+    p = 47274u - mulhi32(p, rh);                       // Q18
+    p = 864443u - mulhi32(p, rh);
+    p = 16136271u - mulhi32(p, rh);
+    p = 309816401u - mulhi32(p, rh);                   // Q30
+    u64 P = 0x000171547652b830ull - (wide(p, rh) >> 16);   // Q50
+    P = 0x001ec709dc3a03fdull - mulhi(P, rs);
+    P = 0x02e2a8eca5705fc3ull - mulhi(P, rs);
+    P = 0x5c551d94ae0bf85eull - mulhi(P, rs);              // Q62
+    const u64 F = kLogT[i] + (mulhi(P, rs) >> 4);
+    // y = a (e + F), Q61: a (e + 512) - 512 a + a F over 96 bits
+    const u32 eb = (xh >> 20) - 511u;
+    const u64 y0 = wide((u32)A, eb), aF = mulhi(A, F) << 2;
+    const u64 ylo = (u64)(u32)y0 + (u32)aF;                       // low word of a (e + 512) + a F
+    u64 yh = wide((u32)(A >> 32), eb) + (u32)(y0 >> 32) + (u32)(aF >> 32) + (u32)(ylo >> 32);
+    u64 yl = (u32)ylo;
+    const u64 sub = A << 9;                                        // 512 a modulo 2^64; its top: A >> 55
+    const u64 l2 = yl - (u32)sub;
+    yh = yh - ((A >> 23) + ((l2 >> 32) & 1u));
+    yl = (u32)l2;
+    // 2^y: y = k + i/64 + s
+    const int k = (int)((long long)yh >> 29);
+    const u64 fr = ((yh << 35) | (yl << 3));                       // Q64
+    const u32 j = (u32)(fr >> 58);
+    const u64 s = fr << 6;                                          // Q70
+    const u32 sh = (u32)(s >> 32);
+    u32 q = 4094u;                                     // Q28
+    q = 2646306u + mulhi32(q, sh);
+    q = 1466040222u + mulhi32(q, sh);                   // Q40
+    u64 Q = 0x0000009d955b7dd2ull + mulhi32(q, sh);        // Q46
+    Q = 0x0000e35846b82506ull + mulhi(Q, s);
+    Q = 0x00f5fdeffc162c75ull + mulhi(Q, s);
+    Q = 0xb17217f7d1cf79acull + mulhi(Q, s);               // Q64
+    const u64 T = kExpT[j];
+    const u64 E = T + (mulhi(T, mulhi(Q, s)) >> 6);                // Q63
+    const u32 Eh = (u32)(E >> 32), El = (u32)E;
+    const u32 ql = shr2(El, Eh, 11);
+    return round_pack(Eh >> 11, ql, (El << 21) | (ql & 1u), (u32)(k + 1022) << 20);
+}
+IP_RARE double pow_rare(double x, double a) { return ::exp(::log(x) * a); }
+// x^a; what the fixed-point form does not take goes through exp and log
+IP_FN double pow(double x, double a) {
+    // 2^-120 <= x < 2^120, 2^-20 <= a < 4
+    if (__builtin_expect(hi(x) - 0x38700000u < 0x0f000000u && hi(a) - 0x3eb00000u < 0x01600000u, 1)) return pow_core(x, a);
+    return pow_rare(x, a);
+}
+
 // x / 2: exact for normal results and zeros, by the exponent
 IP_FN double half(double x) {
     const u32 xa = hi(x) & 0x7fffffffu;

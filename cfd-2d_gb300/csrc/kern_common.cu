@@ -183,6 +183,9 @@ __global__ void k_selftest(int which, long long n, unsigned long long seed, unsi
                      differ(ip::rcp(b2), __drcp_rn(b2)) + differ(ip::quot(a2, b2), __ddiv_rn(a2, b2)) +
                      differ(ip::quot(a2, c), __ddiv_rn(a2, c)) + differ(ip::sqrt(s), __dsqrt_rn(s)) +
                      differ(ip::half(c), __dmul_rn(c, 0.5)) + differ(ip::plus_zero(c), __dadd_rn(0.0, c));
+            // x^(1/7), x in [0.5, 1.5): CUDA's pow is within 2 units in the last place, so is the difference
+            const double x = 0.5 + (double)(r1 >> 12) * 0x1p-52, p7 = ::pow(x, 1.0 / 7.0);
+            local += llabs(__double_as_longlong(ip::pow(x, 1.0 / 7.0)) - __double_as_longlong(p7)) > 2;
         } else if (which == 1) {  // widening of random normal floats
             const float f = __uint_as_float((unsigned)(((r1 % 254) + 1) << 23) | (unsigned)(r2 & 0x807fffffu));
             local += __double_as_longlong(widen(f)) != __double_as_longlong((double)f);

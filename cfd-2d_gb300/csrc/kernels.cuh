@@ -34,7 +34,7 @@ __device__ __forceinline__ double t_fma(double a, double b, double c) { return f
 using ip::xd;
 __device__ __forceinline__ xd t_sqrt(xd x) { return xd(ip::sqrt(x.v)); }
 // x^a for positive x (the reference's exp(log(x) a))
-__device__ __forceinline__ xd t_pow(xd x, xd a) { return xd(exp(log(x.v) * a.v)); }
+__device__ __forceinline__ xd t_pow(xd x, xd a) { return xd(ip::pow(x.v, a.v)); }
 __device__ __forceinline__ float t_pow(float x, float a) { return expf(logf(x) * a); }
 __device__ __forceinline__ xd t_abs(xd x) { return xd(ip::make(ip::hi(x.v) & 0x7fffffffu, ip::lo(x.v))); }
 __device__ __forceinline__ xd t_fma(xd a, xd b, xd c) { return xd(__fma_rn(a.v, b.v, c.v)); }

@@ -1,6 +1,7 @@
 """The integer-pipe FP64 arithmetic (csrc/intpipe.cuh) compiled for the host: correctly rounded
 products, sums, reciprocals, quotients and square roots must equal the IEEE operations bit for
-bit on random, nearly equal and special operands, whatever the reciprocal seeds' last bits are."""
+bit on random, nearly equal and special operands, whatever the reciprocal seeds' last bits are;
+x^a lies within 0.55 units in the last place of long double's."""
 import os
 import shutil
 import subprocess
@@ -43,6 +44,10 @@ int main(int argc, char** argv) {
                         same(ip::rcp(b), 1.0 / b) && same(ip::quot(a, b), a / b) && same(ip::sqrt(x), std::sqrt(x)) &&
                         same(ip::half(a), 0.5 * a) && same(ip::plus_zero(a), 0.0 + a);
         if (!ok && bad++ < 5) printf("%a %a %a\n", a, b, x);
+        const double px = dbl((u64)(i % 3 ? 1022 + g() % 2 : 903 + g() % 240) << 52 | (g() & 0xfffffffffffffull));
+        const double e = i % 2 ? 1.0 / 7.0 : 2.5, y = ip::pow(px, e);
+        const long double t = powl((long double)px, (long double)e);
+        if (!((double)fabsl(y - t) <= 0.55 * std::ldexp(1.0, std::ilogb((double)t) - 52)) && bad++ < 5) printf("pow %a %a\n", px, e);
     }
     return bad != 0;
 }
