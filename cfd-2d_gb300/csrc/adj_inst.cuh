@@ -25,38 +25,159 @@ namespace {
 
 inline int adj_nblk(long n, int b) { return (int)((n + b - 1) / b); }
 
+// One side's adjoints of an edge (12 values): primitives, then gradients.
+template <typename T>
+__device__ __forceinline__ void store_bars(T* o, const Prim<T>& q, const T* g) {
+    st4(o, 0, q.r, q.u, q.v, q.p);
+    st8(o + 4, 0, g);
+}
+__device__ __forceinline__ void store_bars(double* o, const Prim<xd>& q, const xd* g) {
+    st4(o, 0, q.r.v, q.u.v, q.v.v, q.p.v);
+    st8x(o + 4, 0, g);
+}
+
+// The flux VJP of an interior edge with FP64 faces and reconstruction, two lanes per edge: lane
+// gp reverses Gauss point gp's flux (its states read from the forward's record with REC, else
+// reconstructed), the pair exchanges the face states' adjoints, and each lane gathers the
+// reconstruction's VJP of one side over both points, in the points' order: the same operations
+// as adj_flux_edge's on the same values. One thread for an edge needs 160 registers (12 warps
+// on an SM) and waits for its own chains. Called by whole warps.
+template <int FLUX, int RECON, bool REC>
+__device__ __forceinline__ void adj_flux_lane(const DevCase& c, const AdjCase& a, const FluxRec& rec, int e, int gp,
+                                              bool live) {
+    const size_t ne = c.ne;
+    const xd nx(c.nx[e]), ny(c.ny[e]);
+    const xd GAM = gam_of<xd>(c), IG1 = ig1_of<xd>(c);
+    const int c1 = c.ec1[e], c2 = c.ec2[e];
+    const double* __restrict__ DL = c.dl + e;
+    unsigned codes = 0;
+    Prim<xd> pL, pR, pb[2][2];  // adjoints of the face states: [point][side]
+    {
+        xd cL, cR;
+        if constexpr (REC) {
+            const double* v = static_cast<const double*>(rec.v) + (size_t)(10 * gp) * ne + e;
+            pL = Prim<xd>{xd(v[0]), xd(v[ne]), xd(v[2 * ne]), xd(v[3 * ne])};
+            pR = Prim<xd>{xd(v[4 * ne]), xd(v[5 * ne]), xd(v[6 * ne]), xd(v[7 * ne])};
+            cL = xd(v[8 * ne]); cR = xd(v[9 * ne]);
+            if (RECON == RECON_MINMOD) codes = rec.bits[e] >> (16 * gp);
+        } else {
+            pL = prim_as<xd>(load_prim(c.W64, c1));
+            pR = prim_as<xd>(load_prim(c.W64, c2));
+            Prim<xd> d = pL;
+            if (RECON == RECON_MINMOD) d = Prim<xd>{pR.r - pL.r, pR.u - pL.u, pR.v - pL.v, pR.p - pL.p};
+            const double* dl = DL + (size_t)(4 * gp) * ne;
+            double g[8];
+            ld8(c.G64, c1, g);
+            codes = reconstruct<xd, RECON>(pL, g, xd(dl[0]), xd(dl[ne]), d);
+            if (RECON == RECON_MINMOD) d = Prim<xd>{-d.r, -d.u, -d.v, -d.p};
+            ld8(c.G64, c2, g);
+            codes |= reconstruct<xd, RECON>(pR, g, xd(dl[2 * ne]), xd(dl[3 * ne]), d) << 8;
+        }
+        xd fb[4];
+        {
+            double m1[4], m2[4];
+            ld4(a.mu, c1, m1);
+            ld4(a.mu, c2, m2);
+            // F = (sum over Gauss points of f) * l/2; R_c1 -= F, R_c2 += F
+            const xd lh = half(xd(c.l[e]));
+#pragma unroll
+            for (int k = 0; k < 4; k++) fb[k] = (xd(m2[k]) - xd(m1[k])) * lh;
+        }
+        Prim<xd> Lb = zero_prim<xd>(), Rb = zero_prim<xd>();
+        if constexpr (REC) vjp_hllc_c(pL, pR, cL, cR, nx, ny, GAM, IG1, fb, Lb, Rb);
+        else vjp_flux<FLUX>(pL, pR, nx, ny, GAM, IG1, fb, Lb, Rb);
+        pb[0][0] = Lb;
+        pb[0][1] = Rb;
+    }
+    // both points' adjoints and branches in both lanes
+    auto swap = [](xd x) { return xd(__shfl_xor_sync(0xffffffffu, x.v, 1)); };
+    unsigned cd[2];
+    {
+        const unsigned oc = __shfl_xor_sync(0xffffffffu, codes, 1);
+        cd[0] = gp ? oc : codes;
+        cd[1] = gp ? codes : oc;
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            const Prim<xd> m = pb[0][s], o{swap(m.r), swap(m.u), swap(m.v), swap(m.p)};
+            pb[0][s] = gp ? o : m;
+            pb[1][s] = gp ? m : o;
+        }
+    }
+    if (!live) return;
+    const int side = gp;  // this lane's side from here on
+    xd qb[4], gb[8];
+#pragma unroll
+    for (int k = 0; k < 4; k++) qb[k] = acc0<xd>();
+#pragma unroll
+    for (int k = 0; k < 8; k++) gb[k] = acc0<xd>();
+#pragma unroll
+    for (int g = 0; g < 2; g++) {
+        const double* dl = DL + (size_t)(4 * g + 2 * side) * ne;
+        const xd dx(dl[0]), dy(dl[ne]);
+        const Prim<xd>&l = pb[g][0], &r = pb[g][1];
+        const xd lv[4] = {l.r, l.p, l.u, l.v}, rv[4] = {r.r, r.p, r.u, r.v};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const unsigned bl = RECON == RECON_LINEAR ? 1u : (cd[g] >> (2 * k)) & 3u;
+            const unsigned br = RECON == RECON_LINEAR ? 1u : (cd[g] >> (8 + 2 * k)) & 3u;
+            const xd own = side ? rv[k] : lv[k];
+            if ((side ? br : bl) == 1u) {  // the projection: into the gradient
+                gb[2 * k] = madd(gb[2 * k], own, dx);
+                gb[2 * k + 1] = madd(gb[2 * k + 1], own, dy);
+            }
+            // the left face state's share, then the right one's: a side keeps its own state's
+            // adjoint unless the difference was taken (2), which passes it to the other side
+            if ((bl == 2u) == (side == 1)) qb[k] = qb[k] + lv[k];
+            if ((br == 2u) == (side == 0)) qb[k] = qb[k] + rv[k];
+        }
+    }
+    store_bars(static_cast<double*>(a.eq) + 24 * (size_t)e + 12 * side, Prim<xd>{qb[0], qb[2], qb[3], qb[1]}, gb);
+}
+// FP64 faces with reconstruction: the interior edges by lanes in the first n_lane blocks, the
+// boundary edges (stored last) one thread each in the others
+template <int RECON> constexpr bool kAdjLanes = RECON != RECON_NONE;
+
 template <typename T, int FLUX, int RECON, int SIDE>
 __device__ __forceinline__ void adj_flux_edge(const DevCase& c, const AdjCase& a, int e);
 template <typename T, int FLUX, int RECON>
 // FP32 faces: at most 128 registers (two 256-thread blocks' worth per SM), measured
-// faster than the compiler's unconstrained choice; FP64 faces: unconstrained. With FP64 faces
-// interior and boundary edges (stored last) run their own instantiations.
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 0) k_adj_flux(const DevCase c, const AdjCase a) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= c.ne) return;
-    if constexpr (sizeof(T) == 8) {  // FP64 faces: no contraction, the same bits in either instantiation
-        if (e < c.n_int) adj_flux_edge<T, FLUX, RECON, EDGE_INNER>(c, a, e);
+// faster than the compiler's unconstrained choice. With FP64 faces interior and boundary edges
+// (stored last) run their own instantiations.
+__global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : 128, sizeof(T) == 4 ? 2 : 4)
+k_adj_flux(const DevCase c, const AdjCase a, int n_lane) {
+    if constexpr (sizeof(T) == 8) {
+        const int t = blockIdx.x * blockDim.x + threadIdx.x;
+        if (kAdjLanes<RECON> && (int)blockIdx.x < n_lane) {
+            const bool live = t < 2 * c.n_int;
+            if constexpr (kAdjLanes<RECON>) adj_flux_lane<FLUX, RECON, false>(c, a, FluxRec{}, live ? t >> 1 : 0, t & 1, live);
+            return;
+        }
+        const int e = t + (kAdjLanes<RECON> ? c.n_int - n_lane * (int)blockDim.x : 0);
+        if (e >= c.ne) return;
+        if (!kAdjLanes<RECON> && e < c.n_int) adj_flux_edge<T, FLUX, RECON, EDGE_INNER>(c, a, e);
         else adj_flux_edge<T, FLUX, RECON, EDGE_BOUNDARY>(c, a, e);
     } else {
-        adj_flux_edge<T, FLUX, RECON, EDGE_ANY>(c, a, e);
+        const int e = blockIdx.x * blockDim.x + threadIdx.x;
+        if (e < c.ne) adj_flux_edge<T, FLUX, RECON, EDGE_ANY>(c, a, e);
     }
 }
 template <typename T, int FLUX, int RECON, int SIDE>
 __device__ __forceinline__ void adj_flux_edge(const DevCase& c, const AdjCase& a, int e) {
+    typedef Arith<T> A;
     const int ne = c.ne;
     const T* W = W_of<T>(c);
     const T* G = G_of<T>(c);
     const T* DL = DL_of<T>(c);
-    const T nx = NX_of<T>(c)[e], ny = NY_of<T>(c)[e], l = L_of<T>(c)[e];
-    const T GAM = gam_of<T>(c), IG1 = ig1_of<T>(c);
+    const A nx(NX_of<T>(c)[e]), ny(NY_of<T>(c)[e]), l(L_of<T>(c)[e]);
+    const A GAM = gam_of<A>(c), IG1 = ig1_of<A>(c);
     const int c1 = c.ec1[e];
     const bool inner = edge_inner<SIDE>(c, e);
     const int c2 = inner ? c.ec2[e] : -1;
-    const Prim<T> qL = load_prim(W, c1);
-    Prim<T> qR = qL, gc = qL;
+    const Prim<A> qL = prim_as<A>(load_prim(W, c1));
+    Prim<A> qR = qL, gc = qL;
     DevBnd b{};
-    T Tc = T(0), M = T(0), gm1 = T(0), Cv = T(0);
-    T fb[4];
+    A Tc = A(0), M = A(0), gm1 = A(0), Cv = A(0);
+    A fb[4];
     {
         double m1[4], m2[4] = {0, 0, 0, 0};
         ld4(a.mu, c1, m1);
@@ -64,45 +185,45 @@ __device__ __forceinline__ void adj_flux_edge(const DevCase& c, const AdjCase& a
         // F = (sum over Gauss points of f) * l/2; R_c1 -= F, R_c2 += F. The difference is
         // formed in FP64 and rounded once into the face precision.
         const double lh = to_wide(l) * (RECON == RECON_NONE ? 1.0 : 0.5);
-        for (int k = 0; k < 4; k++) fb[k] = to_face<T>((m2[k] - m1[k]) * lh);
+        for (int k = 0; k < 4; k++) fb[k] = to_face<A>((m2[k] - m1[k]) * lh);
     }
     if (inner) {
-        qR = load_prim(W, c2);
+        qR = prim_as<A>(load_prim(W, c2));
     } else {
         b = c.bnds[c.ebnd[e]];
-        const MatT<T> mt = matT_of<T>(c, c1);
+        const MatT<A> mt = matT_of<A>(c, c1);
         gm1 = mt.gm1; Cv = mt.Cv; M = mt.M;
         Tc = temperature(qL, gm1, Cv);
         if (RECON == RECON_MINMOD) gc = ghost_state(b, qL, Tc, nx, ny, M);
     }
-    Prim<T> q1b = zero_prim<T>(), q2b = zero_prim<T>(), gcb = zero_prim<T>();
-    T g1b[8], g2b[8], bp[4];
+    Prim<A> q1b = zero_prim<A>(), q2b = zero_prim<A>(), gcb = zero_prim<A>();
+    A g1b[8], g2b[8], bp[4];
 #pragma unroll
-    for (int k = 0; k < 8; k++) { g1b[k] = acc0<T>(); g2b[k] = acc0<T>(); }
+    for (int k = 0; k < 8; k++) { g1b[k] = acc0<A>(); g2b[k] = acc0<A>(); }
 #pragma unroll
-    for (int k = 0; k < 4; k++) bp[k] = acc0<T>();
-    T Tcb = acc0<T>();
+    for (int k = 0; k < 4; k++) bp[k] = acc0<A>();
+    A Tcb = acc0<A>();
     const int ngp = RECON == RECON_NONE ? 1 : 2;
 #pragma unroll 1
     for (int gp = 0; gp < ngp; gp++) {
-        Prim<T> pL = qL, pR = qR;
-        T aL[4] = {T(0), T(0), T(0), T(0)}, aR[4] = {T(0), T(0), T(0), T(0)};
-        T dxL = T(0), dyL = T(0), dxR = T(0), dyR = T(0);
+        Prim<A> pL = qL, pR = qR;
+        A aL[4] = {A(0), A(0), A(0), A(0)}, aR[4] = {A(0), A(0), A(0), A(0)};
+        A dxL = A(0), dyL = A(0), dxR = A(0), dyR = A(0);
         if (RECON != RECON_NONE) {
             T g[8];
-            dxL = DL[(4 * gp) * ne + e]; dyL = DL[(4 * gp + 1) * ne + e];
+            dxL = A(DL[(4 * gp) * ne + e]); dyL = A(DL[(4 * gp + 1) * ne + e]);
             ld8(G, c1, g);
             project<RECON>(g, dxL, dyL, aL);
             pL = recon_a<RECON>(qL, aL, inner ? qR : gc);
             if (inner) {
-                dxR = DL[(4 * gp + 2) * ne + e]; dyR = DL[(4 * gp + 3) * ne + e];
+                dxR = A(DL[(4 * gp + 2) * ne + e]); dyR = A(DL[(4 * gp + 3) * ne + e]);
                 ld8(G, c2, g);
                 project<RECON>(g, dxR, dyR, aR);
                 pR = recon_a<RECON>(qR, aR, qL);
             }
         }
         if (!inner) pR = ghost_state(b, pL, Tc, nx, ny, M);
-        Prim<T> pLb = zero_prim<T>(), pRb = zero_prim<T>();
+        Prim<A> pLb = zero_prim<A>(), pRb = zero_prim<A>();
         vjp_flux<FLUX>(pL, pR, nx, ny, GAM, IG1, fb, pLb, pRb);
         if (!inner) vjp_ghost(b, pL, Tc, nx, ny, M, pRb, pLb, Tcb, bp);
         if (RECON == RECON_NONE) {  // both Gauss points see the cell-centre states: one pass, twice the weight
@@ -122,10 +243,8 @@ __device__ __forceinline__ void adj_flux_edge(const DevCase& c, const AdjCase& a
         o[0] += to_wide(bp[0]); o[1] += to_wide(bp[1]); o[2] += to_wide(bp[2]); o[3] += to_wide(bp[3]);
     }
     T* o = static_cast<T*>(a.eq) + 24 * (size_t)e;
-    st4(o, 0, q1b.r, q1b.u, q1b.v, q1b.p);
-    st8(o + 4, 0, g1b);
-    st4(o + 12, 0, q2b.r, q2b.u, q2b.v, q2b.p);
-    st8(o + 16, 0, g2b);
+    store_bars(o, q1b, g1b);
+    store_bars(o + 12, q2b, g2b);
 }
 
 // The forward flux kernel of a recomputed stage that also keeps the evaluation's record
@@ -150,65 +269,73 @@ __global__ void __launch_bounds__(128) k_flux_rec(const DevCase c, const FluxRec
 template <typename T, int RECON, int SIDE>
 __device__ __forceinline__ void adj_flux_rec_edge(const DevCase& c, const AdjCase& a, const FluxRec& r, int e);
 template <typename T, int RECON>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 0) k_adj_flux_rec(const DevCase c, const AdjCase a,
-                                                                              const FluxRec r) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= c.ne) return;
+__global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : 128, sizeof(T) == 4 ? 2 : 4)
+k_adj_flux_rec(const DevCase c, const AdjCase a, const FluxRec r, int n_lane) {
     if constexpr (sizeof(T) == 8) {
-        if (e < c.n_int) adj_flux_rec_edge<T, RECON, EDGE_INNER>(c, a, r, e);
+        const int t = blockIdx.x * blockDim.x + threadIdx.x;
+        if (kAdjLanes<RECON> && (int)blockIdx.x < n_lane) {
+            const bool live = t < 2 * c.n_int;
+            if constexpr (kAdjLanes<RECON>) adj_flux_lane<FLUX_HLLC, RECON, true>(c, a, r, live ? t >> 1 : 0, t & 1, live);
+            return;
+        }
+        const int e = t + (kAdjLanes<RECON> ? c.n_int - n_lane * (int)blockDim.x : 0);
+        if (e >= c.ne) return;
+        if (!kAdjLanes<RECON> && e < c.n_int) adj_flux_rec_edge<T, RECON, EDGE_INNER>(c, a, r, e);
         else adj_flux_rec_edge<T, RECON, EDGE_BOUNDARY>(c, a, r, e);
     } else {
-        adj_flux_rec_edge<T, RECON, EDGE_ANY>(c, a, r, e);
+        const int e = blockIdx.x * blockDim.x + threadIdx.x;
+        if (e < c.ne) adj_flux_rec_edge<T, RECON, EDGE_ANY>(c, a, r, e);
     }
 }
 template <typename T, int RECON, int SIDE>
 __device__ __forceinline__ void adj_flux_rec_edge(const DevCase& c, const AdjCase& a, const FluxRec& r, int e) {
+    typedef Arith<T> A;
     const int ne = c.ne;
     const T* DL = DL_of<T>(c);
-    const T nx = NX_of<T>(c)[e], ny = NY_of<T>(c)[e], l = L_of<T>(c)[e];
-    const T GAM = gam_of<T>(c), IG1 = ig1_of<T>(c);
+    const A nx(NX_of<T>(c)[e]), ny(NY_of<T>(c)[e]), l(L_of<T>(c)[e]);
+    const A GAM = gam_of<A>(c), IG1 = ig1_of<A>(c);
     const int c1 = c.ec1[e];
     const bool inner = edge_inner<SIDE>(c, e);
     const int c2 = inner ? c.ec2[e] : -1;
-    Prim<T> qL{};
+    Prim<A> qL{};
     DevBnd b{};
-    T Tc = T(0), M = T(0), gm1 = T(0), Cv = T(0);
-    T fb[4];
+    A Tc = A(0), M = A(0), gm1 = A(0), Cv = A(0);
+    A fb[4];
     {
         double m1[4], m2[4] = {0, 0, 0, 0};
         ld4(a.mu, c1, m1);
         if (inner) ld4(a.mu, c2, m2);
         const double lh = to_wide(l) * (RECON == RECON_NONE ? 1.0 : 0.5);
-        for (int k = 0; k < 4; k++) fb[k] = to_face<T>((m2[k] - m1[k]) * lh);
+        for (int k = 0; k < 4; k++) fb[k] = to_face<A>((m2[k] - m1[k]) * lh);
     }
     if (!inner) {
-        qL = load_prim(W_of<T>(c), c1);
+        qL = prim_as<A>(load_prim(W_of<T>(c), c1));
         b = c.bnds[c.ebnd[e]];
-        const MatT<T> mt = matT_of<T>(c, c1);
+        const MatT<A> mt = matT_of<A>(c, c1);
         gm1 = mt.gm1; Cv = mt.Cv; M = mt.M;
         Tc = temperature(qL, gm1, Cv);
     }
-    Prim<T> q1b = zero_prim<T>(), q2b = zero_prim<T>(), gcb = zero_prim<T>();
-    T g1b[8], g2b[8], bp[4];
+    Prim<A> q1b = zero_prim<A>(), q2b = zero_prim<A>(), gcb = zero_prim<A>();
+    A g1b[8], g2b[8], bp[4];
 #pragma unroll
-    for (int k = 0; k < 8; k++) { g1b[k] = acc0<T>(); g2b[k] = acc0<T>(); }
+    for (int k = 0; k < 8; k++) { g1b[k] = acc0<A>(); g2b[k] = acc0<A>(); }
 #pragma unroll
-    for (int k = 0; k < 4; k++) bp[k] = acc0<T>();
-    T Tcb = acc0<T>();
+    for (int k = 0; k < 4; k++) bp[k] = acc0<A>();
+    A Tcb = acc0<A>();
     const unsigned bits = RECON == RECON_MINMOD ? r.bits[e] : 0u;
     const int ngp = RECON == RECON_NONE ? 1 : 2;
 #pragma unroll 1
     for (int gp = 0; gp < ngp; gp++) {
         const T* v = static_cast<const T*>(r.v) + (size_t)(10 * gp) * ne + e;
-        const Prim<T> pL{v[0], v[ne], v[2 * (size_t)ne], v[3 * (size_t)ne]};
-        const Prim<T> pR{v[4 * (size_t)ne], v[5 * (size_t)ne], v[6 * (size_t)ne], v[7 * (size_t)ne]};
-        const T cL = v[8 * (size_t)ne], cR = v[9 * (size_t)ne];
-        T dxL = T(0), dyL = T(0), dxR = T(0), dyR = T(0);
+        const Prim<A> pL{A(v[0]), A(v[ne]), A(v[2 * (size_t)ne]), A(v[3 * (size_t)ne])};
+        const Prim<A> pR{A(v[4 * (size_t)ne]), A(v[5 * (size_t)ne]), A(v[6 * (size_t)ne]), A(v[7 * (size_t)ne])};
+        const A cL(v[8 * (size_t)ne]), cR(v[9 * (size_t)ne]);
+        A dxL = A(0), dyL = A(0), dxR = A(0), dyR = A(0);
         if (RECON != RECON_NONE) {
-            dxL = DL[(4 * gp) * ne + e]; dyL = DL[(4 * gp + 1) * ne + e];
-            if (inner) { dxR = DL[(4 * gp + 2) * ne + e]; dyR = DL[(4 * gp + 3) * ne + e]; }
+            dxL = A(DL[(4 * gp) * ne + e]); dyL = A(DL[(4 * gp + 1) * ne + e]);
+            if (inner) { dxR = A(DL[(4 * gp + 2) * ne + e]); dyR = A(DL[(4 * gp + 3) * ne + e]); }
         }
-        Prim<T> pLb = zero_prim<T>(), pRb = zero_prim<T>();
+        Prim<A> pLb = zero_prim<A>(), pRb = zero_prim<A>();
         vjp_hllc_c(pL, pR, cL, cR, nx, ny, GAM, IG1, fb, pLb, pRb);
         if (!inner) vjp_ghost(b, pL, Tc, nx, ny, M, pRb, pLb, Tcb, bp);
         if (RECON == RECON_NONE) {
@@ -228,10 +355,8 @@ __device__ __forceinline__ void adj_flux_rec_edge(const DevCase& c, const AdjCas
         o[0] += to_wide(bp[0]); o[1] += to_wide(bp[1]); o[2] += to_wide(bp[2]); o[3] += to_wide(bp[3]);
     }
     T* o = static_cast<T*>(a.eq) + 24 * (size_t)e;
-    st4(o, 0, q1b.r, q1b.u, q1b.v, q1b.p);
-    st8(o + 4, 0, g1b);
-    st4(o + 12, 0, q2b.r, q2b.u, q2b.v, q2b.p);
-    st8(o + 16, 0, g2b);
+    store_bars(o, q1b, g1b);
+    store_bars(o + 12, q2b, g2b);
 }
 
 // The three faces' contributions summed exactly (SumAcc): the primitive adjoint is
@@ -262,7 +387,7 @@ __global__ void __launch_bounds__(256) k_adj_gather(const DevCase c, const AdjCa
     const T iSi = invS_of<T>(c)[i];
     T gv[8];
 #pragma unroll
-    for (int m = 0; m < 8; m++) gv[m] = g[m].face() * iSi;
+    for (int m = 0; m < 8; m++) gv[m] = T(Arith<T>(g[m].face()) * Arith<T>(iSi));
     st8(static_cast<T*>(a.gbar), i, gv);
 }
 
@@ -276,93 +401,99 @@ __global__ void __launch_bounds__(256) k_adj_cell(const DevCase c, const AdjCase
     const int nc = c.nc;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nc) return;
-    const MatT<T> mt = matT_of<T>(c, i);
-    const Prim<T> q = load_prim(W_of<T>(c), i);
+    typedef Arith<T> A;
+    typedef typename WideArith<T>::type D;
+    const MatT<A> mt = matT_of<A>(c, i);
+    const Prim<A> q = prim_as<A>(load_prim(W_of<T>(c), i));
     // h = the gradient adjoints divided by the area (k_adj_gather)
     const T* h = static_cast<const T*>(a.gbar);
     // the cell's primitive adjoint: the gathered FP64 value plus the sum of the
     // Green-Gauss products (r, u, v, p)
     SumAcc<T> qs[4];
-    T Tcb = acc0<T>();
-    Prim<T> qb = zero_prim<T>();  // ghost-path contributions (boundary faces only)
+    A Tcb = acc0<A>();
+    Prim<A> qb = zero_prim<A>();  // ghost-path contributions (boundary faces only)
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         const int f = c.face[k * nc + i];
         const int e = f >> 1;
         const bool side2 = f & 1;
-        const T nx = NX_of<T>(c)[e], ny = NY_of<T>(c)[e], l = L_of<T>(c)[e];
+        const A nx(NX_of<T>(c)[e]), ny(NY_of<T>(c)[e]), l(L_of<T>(c)[e]);
         // d g_i / d (neighbour or ghost value) = +-(l/2) n / S_i with n outward from c1; the
         // neighbour's gradient takes q_i with the opposite sign and its own 1/S_j. The own
         // value's direct terms, (1/S_i) sum_k (l_k/2) n_out,k over the three faces, are the
         // outward normals of a closed triangle weighted by their lengths: zero, and left out.
-        const T w = neg_if(T(0.5) * l, side2);
-        const T wx = w * nx, wy = w * ny;
+        const A w = neg_if(half(l), side2);
+        const A wx = w * nx, wy = w * ny;
         const int j = side2 ? c.ec1[e] : c.ec2[e];
         if (j >= 0) {
             T hj[8];
             ld8(h, j, hj);
-            qs[0].add(-madd(wx * hj[0], wy, hj[1]));
-            qs[3].add(-madd(wx * hj[2], wy, hj[3]));
-            qs[1].add(-madd(wx * hj[4], wy, hj[5]));
-            qs[2].add(-madd(wx * hj[6], wy, hj[7]));
+            qs[0].add(-madd(wx * A(hj[0]), wy, A(hj[1])));
+            qs[3].add(-madd(wx * A(hj[2]), wy, A(hj[3])));
+            qs[1].add(-madd(wx * A(hj[4]), wy, A(hj[5])));
+            qs[2].add(-madd(wx * A(hj[6]), wy, A(hj[7])));
         } else {  // boundary face: the ghost of the unreconstructed centre state
             T hi[8];
             ld8(h, i, hi);
-            const T s0 = madd(wx * hi[0], wy, hi[1]), s1 = madd(wx * hi[2], wy, hi[3]);
-            const T s2 = madd(wx * hi[4], wy, hi[5]), s3 = madd(wx * hi[6], wy, hi[7]);
+            const A s0 = madd(wx * A(hi[0]), wy, A(hi[1])), s1 = madd(wx * A(hi[2]), wy, A(hi[3]));
+            const A s2 = madd(wx * A(hi[4]), wy, A(hi[5])), s3 = madd(wx * A(hi[6]), wy, A(hi[7]));
             const DevBnd b = c.bnds[c.ebnd[e]];
-            const T Tc = temperature(q, mt.gm1, mt.Cv);
-            Prim<T> ob;
+            const A Tc = temperature(q, mt.gm1, mt.Cv);
+            Prim<A> ob;
             ob.r = s0; ob.p = s1; ob.u = s2; ob.v = s3;
-            T bp[4] = {acc0<T>(), acc0<T>(), acc0<T>(), acc0<T>()};
+            A bp[4] = {acc0<A>(), acc0<A>(), acc0<A>(), acc0<A>()};
             vjp_ghost(b, q, Tc, nx, ny, mt.M, ob, qb, Tcb, bp);
             double* o = a.eb2 + 4 * (size_t)(e - c.n_int);
             o[0] += to_wide(bp[0]); o[1] += to_wide(bp[1]); o[2] += to_wide(bp[2]); o[3] += to_wide(bp[3]);
         }
     }
-    if (Tcb != T(0.0)) vjp_temperature(q, mt.gm1, mt.Cv, Tcb, qb);
+    if (to_wide(Tcb) != 0.0) vjp_temperature(q, mt.gm1, mt.Cv, Tcb, qb);
     {
         double q0[4];
         ld4(a.qbar, i, q0);  // r, u, v, p
         qs[0].add(qb.r); qs[1].add(qb.u); qs[2].add(qb.v); qs[3].add(qb.p);
-        qb.r = to_face<T>(q0[0] + qs[0].value());
-        qb.u = to_face<T>(q0[1] + qs[1].value());
-        qb.v = to_face<T>(q0[2] + qs[2].value());
-        qb.p = to_face<T>(q0[3] + qs[3].value());
+        qb.r = to_face<A>(to_wide(D(q0[0]) + D(qs[0].value())));
+        qb.u = to_face<A>(to_wide(D(q0[1]) + D(qs[1].value())));
+        qb.v = to_face<A>(to_wide(D(q0[2]) + D(qs[2].value())));
+        qb.p = to_face<A>(to_wide(D(q0[3]) + D(qs[3].value())));
     }
-    T V[4] = {acc0<T>(), acc0<T>(), acc0<T>(), acc0<T>()};
+    A V[4] = {acc0<A>(), acc0<A>(), acc0<A>(), acc0<A>()};
     vjp_cons2prim_q(q, mt.gm1, qb, V);
-    double ux[4];
-    for (int k = 0; k < 4; k++) ux[k] = a.tb[k * nc + i] + to_wide(V[k]);
-    if (first) {  // lambda of the step input, and (coef_t, coef_acc = the last stage's) the next step's start
-        const double cf = c.cfl[i];
-        double t[4];
-        for (int k = 0; k < 4; k++) {
-            const double l = a.acc[k * nc + i] + ux[k];
-            a.lam[k * nc + i] = l;
-            t[k] = coef_t * l;
-            a.tb[k * nc + i] = t[k];
-            a.acc[k * nc + i] = coef_acc * l;
+    D ux[4];
+    for (int k = 0; k < 4; k++) ux[k] = D(a.tb[k * nc + i]) + D(to_wide(V[k]));
+    const D cf(c.cfl[i]), ct(coef_t), ca(coef_acc);
+    double mu[4];
+    for (int k = 0; k < 4; k++) {
+        const size_t q4 = (size_t)k * nc + i;
+        D t;
+        if (first) {  // lambda of the step input, and (coef_t, coef_acc = the last stage's) the next step's start
+            const D l = D(a.acc[q4]) + ux[k];
+            a.lam[q4] = to_wide(l);
+            t = ct * l;
+            a.acc[q4] = to_wide(ca * l);
+        } else {
+            t = ct * ux[k];
+            a.acc[q4] = to_wide(D(a.acc[q4]) + ca * ux[k]);
         }
-        st4(a.mu_out, i, cf * t[0], cf * t[1], cf * t[2], cf * t[3]);
-    } else {
-        const double cf = c.cfl[i];
-        double t[4];
-        for (int k = 0; k < 4; k++) {
-            t[k] = coef_t * ux[k];
-            a.tb[k * nc + i] = t[k];
-            a.acc[k * nc + i] += coef_acc * ux[k];
-        }
-        st4(a.mu_out, i, cf * t[0], cf * t[1], cf * t[2], cf * t[3]);
+        a.tb[q4] = to_wide(t);
+        mu[k] = to_wide(cf * t);
     }
+    st4(a.mu_out, i, mu[0], mu[1], mu[2], mu[3]);
 }
 
+// blocks of 128 threads for the flux VJP: n_lane for the interior edges' lanes, the rest one
+// thread per edge
+inline int adj_flux_grid(const DevCase& c, int recon, int& n_lane) {
+    n_lane = sizeof(KT) == 8 && recon != RECON_NONE ? adj_nblk(2l * c.n_int, 128) : 0;
+    return n_lane ? n_lane + adj_nblk(c.ne - c.n_int, 128) : adj_nblk(c.ne, 128);
+}
 template <int FLUX>
 void adj_flux_by_recon(const DevCase& c, const AdjCase& a, int recon, cudaStream_t s) {
-    const int g = adj_nblk(c.ne, 128);
-    if (recon == RECON_NONE) k_adj_flux<KT, FLUX, RECON_NONE><<<g, 128, 0, s>>>(c, a);
-    else if (recon == RECON_LINEAR) k_adj_flux<KT, FLUX, RECON_LINEAR><<<g, 128, 0, s>>>(c, a);
-    else k_adj_flux<KT, FLUX, RECON_MINMOD><<<g, 128, 0, s>>>(c, a);
+    int n_lane;
+    const int g = adj_flux_grid(c, recon, n_lane);
+    if (recon == RECON_NONE) k_adj_flux<KT, FLUX, RECON_NONE><<<g, 128, 0, s>>>(c, a, n_lane);
+    else if (recon == RECON_LINEAR) k_adj_flux<KT, FLUX, RECON_LINEAR><<<g, 128, 0, s>>>(c, a, n_lane);
+    else k_adj_flux<KT, FLUX, RECON_MINMOD><<<g, 128, 0, s>>>(c, a, n_lane);
 }
 }  // namespace
 
@@ -378,10 +509,11 @@ void KFN(flux_rec)(const DevCase& c, int recon, const FluxRec& r, cudaStream_t s
     else k_flux_rec<KT, RECON_MINMOD><<<g, 128, 0, s>>>(c, r);
 }
 void KFN(adj_flux_rec)(const DevCase& c, const AdjCase& a, int recon, const FluxRec& r, cudaStream_t s) {
-    const int g = adj_nblk(c.ne, 128);
-    if (recon == RECON_NONE) k_adj_flux_rec<KT, RECON_NONE><<<g, 128, 0, s>>>(c, a, r);
-    else if (recon == RECON_LINEAR) k_adj_flux_rec<KT, RECON_LINEAR><<<g, 128, 0, s>>>(c, a, r);
-    else k_adj_flux_rec<KT, RECON_MINMOD><<<g, 128, 0, s>>>(c, a, r);
+    int n_lane;
+    const int g = adj_flux_grid(c, recon, n_lane);
+    if (recon == RECON_NONE) k_adj_flux_rec<KT, RECON_NONE><<<g, 128, 0, s>>>(c, a, r, n_lane);
+    else if (recon == RECON_LINEAR) k_adj_flux_rec<KT, RECON_LINEAR><<<g, 128, 0, s>>>(c, a, r, n_lane);
+    else k_adj_flux_rec<KT, RECON_MINMOD><<<g, 128, 0, s>>>(c, a, r, n_lane);
 }
 void KFN(adj_gather)(const DevCase& c, const AdjCase& a, cudaStream_t s) {
     k_adj_gather<KT><<<adj_nblk(c.nc, 128), 128, 0, s>>>(c, a);

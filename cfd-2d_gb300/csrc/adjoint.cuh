@@ -30,7 +30,9 @@ template <typename T> __device__ __forceinline__ Prim<T> zero_prim() {
 template <typename T> __device__ __forceinline__ T to_face(double x);
 template <> __device__ __forceinline__ double to_face<double>(double x) { return x; }
 template <> __device__ __forceinline__ float to_face<float>(double x) { return narrow(x); }
+template <> __device__ __forceinline__ xd to_face<xd>(double x) { return xd(x); }
 __device__ __forceinline__ double to_wide(double x) { return x; }
+__device__ __forceinline__ double to_wide(xd x) { return x.v; }
 __device__ __forceinline__ double to_wide(float x) { return widen(x); }
 
 // A running sum in the face precision kept exact for FP32 (Knuth's TwoSum into a
@@ -39,7 +41,8 @@ __device__ __forceinline__ double to_wide(float x) { return widen(x); }
 template <typename T> struct SumAcc;
 template <> struct SumAcc<double> {
     double s = -0.0;
-    __device__ __forceinline__ void add(double x) { s += x; }
+    __device__ __forceinline__ void add(double x) { s = ip::fadd(s, x); }
+    __device__ __forceinline__ void add(xd x) { add(x.v); }
     __device__ __forceinline__ double value() const { return s; }
     __device__ __forceinline__ double face() const { return s; }
 };
@@ -202,6 +205,12 @@ __device__ __forceinline__ double star_speed(double num, double den, double& ide
     iden = hllc_in_range(den) ? hllc_rcp1(den) : 1.0 / den;
     return hllc_quot(num, den);
 }
+__device__ __forceinline__ xd star_speed(xd num, xd den, xd& iden) {
+    double y;
+    const double s = star_speed(num.v, den.v, y);
+    iden = xd(y);
+    return xd(s);
+}
 __device__ __forceinline__ float star_speed(float num, float den, float& iden) {
     iden = 1.0f / den;
     return num / den;
@@ -311,10 +320,9 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<T>& L, const Prim<T>& R, T
 // FP64 faces: the VJP of the FP64 forward's arrangement (flux_hllc_c<double> in kernels.cuh:
 // S_K U_K - F_K from m_K = rho_K d_K, d_K = S_K - un_K, and only the used side's energy),
 // recomputing the forward's values and branches with its own expressions.
-__device__ __forceinline__ void vjp_hllc_c(const Prim<double>& L, const Prim<double>& R, double cL, double cR,
-                                           double nx, double ny, double GAM, double IG1, const double* fb,
-                                           Prim<double>& Lb, Prim<double>& Rb) {
-    typedef double T;
+__device__ __forceinline__ void vjp_hllc_c(const Prim<xd>& L, const Prim<xd>& R, xd cL, xd cR, xd nx, xd ny, xd GAM,
+                                           xd IG1, const xd* fb, Prim<xd>& Lb, Prim<xd>& Rb) {
+    typedef xd T;
     const T unL = dot2(L.u, nx, L.v, ny), unR = dot2(R.u, nx, R.v, ny);
     const T sl1 = unL - cL, sl2 = unR - cR, sr1 = unL + cL, sr2 = unR + cR;
     const bool l1 = sl1 < sl2, r1 = sr1 > sr2;
@@ -323,7 +331,7 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<double>& L, const Prim<dou
     // E = p IG1 + .5 r (u^2 + v^2): the adjoint Eb of one side's energy into its state
     auto energy_bar = [&](const Prim<T>& q, T Eb, Prim<T>& qb) {
         const T e = Eb * q.r;
-        qb.p = madd(qb.p, Eb, IG1); qb.r = madd(qb.r, Eb * T(0.5), t_fma(q.u, q.u, q.v * q.v));
+        qb.p = madd(qb.p, Eb, IG1); qb.r = madd(qb.r, half(Eb), t_fma(q.u, q.u, q.v * q.v));
         qb.u = madd(qb.u, e, q.u); qb.v = madd(qb.v, e, q.v);
     };
     if (SL >= T(0.0) || SR <= T(0.0)) {  // supersonic: the upwind side's physical flux
@@ -408,12 +416,12 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<double>& L, const Prim<dou
     Lb.u = madd(Lb.u, unLb, nx); Lb.v = madd(Lb.v, unLb, ny);
     Rb.u = madd(Rb.u, unRb, nx); Rb.v = madd(Rb.v, unRb, ny);
     // c = sqrt(GAM p / r) = sqrt(a): dc = (GAM dp - a dr) / (2 c r), a = c^2
-    if (cLb != T(0.0)) {
-        const T ab = hllc_quot(T(0.5) * cLb, cL * L.r);
+    if (cLb.v != 0.0) {
+        const T ab = hllc_quot(half(cLb), cL * L.r);
         Lb.p = madd(Lb.p, ab, GAM); Lb.r = madd(Lb.r, -ab, cL * cL);
     }
-    if (cRb != T(0.0)) {
-        const T ab = hllc_quot(T(0.5) * cRb, cR * R.r);
+    if (cRb.v != 0.0) {
+        const T ab = hllc_quot(half(cRb), cR * R.r);
         Rb.p = madd(Rb.p, ab, GAM); Rb.r = madd(Rb.r, -ab, cR * cR);
     }
 }
@@ -482,12 +490,12 @@ __device__ __forceinline__ void vjp_reconstruct_code(unsigned code, T dx, T dy, 
 }
 
 // Projections a = g . dl of one side's four gradients, as reconstruct() forms them.
-template <int RECON, typename T>
-__device__ __forceinline__ void project(const T* g, T dx, T dy, T* a) {
-    a[0] = proj<T, RECON>(g[0], g[1], dx, dy);
-    a[1] = proj<T, RECON>(g[2], g[3], dx, dy);
-    a[2] = proj<T, RECON>(g[4], g[5], dx, dy);
-    a[3] = proj<T, RECON>(g[6], g[7], dx, dy);
+template <int RECON, typename G, typename T>
+__device__ __forceinline__ void project(const G* g, T dx, T dy, T* a) {
+    a[0] = proj<T, RECON>(T(g[0]), T(g[1]), dx, dy);
+    a[1] = proj<T, RECON>(T(g[2]), T(g[3]), dx, dy);
+    a[2] = proj<T, RECON>(T(g[4]), T(g[5]), dx, dy);
+    a[3] = proj<T, RECON>(T(g[6]), T(g[7]), dx, dy);
 }
 
 // The forward reconstruction from the projections (kernels.cuh reconstruct).

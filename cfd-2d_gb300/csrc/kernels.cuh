@@ -201,6 +201,7 @@ __device__ __forceinline__ xd neg_if(xd x, bool s) { return xd(neg_if(x.v, s)); 
 __device__ __forceinline__ float neg_if(float x, bool s) { return __int_as_float(__float_as_int(x) ^ (s ? (int)0x80000000 : 0)); }
 // a / b given y = RN(1/b): the correctly rounded quotient in FP64, a * y in the FP32 faces.
 __device__ __forceinline__ double div_by(double a, double b, double y) { return div_rn(a, b, y); }
+__device__ __forceinline__ xd div_by(xd a, xd b, xd) { return a / b; }
 __device__ __forceinline__ float div_by(float a, float, float y) { return a * y; }
 // Quotients by a shared divisor: recip_of the divisor once, div_y per dividend (FP32 divides).
 struct NoRecip {};
