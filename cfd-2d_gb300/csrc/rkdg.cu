@@ -113,35 +113,43 @@ __global__ void __launch_bounds__(128, 5) k_dg_edge(const DgCase c, const double
             fg[q][v] = xd(__shfl_sync(0xffffffffu, f[v].v, lane < PER_WARP * GE ? first + q : lane));
     if (!live) return;
     const xd J(c.edgeJ[e]);
-    // integral of basis function k over one side (getF(c, pt) * w, w = 1 for two points)
-    auto integral = [&](int side, int k, int v) {
+    // getF(c, pt)'s component 1 or 2 at point q, times its weight (1 for two points)
+    auto basis = [&](int side, int k, int q) {
+        const xd F(__ldg(eF + 4 * q + 2 * side + k - 1));
+        return GE == 2 ? F : F * xd(c.egw[q]);
+    };
+    // integral over a side of the basis function with weighted values wf
+    auto integral = [&](const xd* wf, int v) {
         xd t(0.0);
 #pragma unroll
         for (int q = 0; q < GE; q++) {
-            const xd w(c.egw[q]);
-            xd wf = w;
-            if (k > 0) {
-                const xd F(__ldg(eF + 4 * q + 2 * side + k - 1));
-                wf = GE == 2 ? F : F * w;
-            }
-            const xd x = wf * fg[q][v];
+            const xd x = wf[q] * fg[q][v];
             t = q == 0 ? pz(x) : t + x;
         }
         return (t * J).v;
     };
     if (GE == 3) {
+        xd wf[GE];
+#pragma unroll 1
+        for (int side = 0; side < (inner ? 2 : 1); side++) {
+            if (side == 0 || g > 0) {
 #pragma unroll
-        for (int v = 0; v < 4; v++) {
-            c.E1[12 * (size_t)e + 3 * v + g] = integral(0, g, v);
-            if (inner) c.E2[12 * (size_t)e + 3 * v + g] = integral(1, g, v);
+                for (int q = 0; q < GE; q++) wf[q] = g == 0 ? xd(c.egw[q]) : basis(side, g, q);
+            }
+            double* o = (side ? c.E2 : c.E1) + 12 * (size_t)e + g;
+#pragma unroll
+            for (int v = 0; v < 4; v++) o[3 * v] = integral(wf, v);
         }
     } else if (g == 0 || inner) {
-        double out[12];
+        double* o = (g == 0 ? c.E1 : c.E2) + 12 * (size_t)e;
+#pragma unroll 1
+        for (int k = 0; k < 3; k++) {
+            xd wf[GE];
 #pragma unroll
-        for (int v = 0; v < 4; v++)
+            for (int q = 0; q < GE; q++) wf[q] = k == 0 ? xd(c.egw[q]) : basis(g, k, q);
 #pragma unroll
-            for (int k = 0; k < 3; k++) out[3 * v + k] = integral(g, k, v);
-        store12(g == 0 ? c.E1 : c.E2, e, out);
+            for (int v = 0; v < 4; v++) o[3 * v + k] = integral(wf, v);
+        }
     }
 }
 
@@ -184,6 +192,8 @@ __global__ void __launch_bounds__(128, 5) k_dg_cell(const DgCase c, int stage, i
         const xd ihx(c.ih[2 * (size_t)i]), ihy(c.ih[2 * (size_t)i + 1]);
         xd in[12];
 #pragma unroll
+        for (int k = 0; k < 12; k++) in[k] = xd(0.0);
+#pragma unroll 1  // (unrolled, the kernel no longer fits the instruction cache)
         for (int g = 0; g < GC; g++) {
             const double2 F = __ldg(reinterpret_cast<const double2*>(c.cF) + (size_t)i * GC + g);
             const DgPar q = dg_eval(a, F.x, F.y, m.gm1);
@@ -212,9 +222,8 @@ __global__ void __launch_bounds__(128, 5) k_dg_cell(const DgCase c, int stage, i
                 for (int v = 0; v < 4; v++) {
                     const xd t1 = pz(ihx * fx[v]) * w;
                     const xd t2 = pz(ihy * gy[v]) * w;
-                    if (g == 0) in[3 * v] = xd(0.0);
-                    in[3 * v + 1] = g == 0 ? pz(t1) : in[3 * v + 1] + t1;
-                    in[3 * v + 2] = g == 0 ? pz(t2) : in[3 * v + 2] + t2;
+                    in[3 * v + 1] = in[3 * v + 1] + t1;
+                    in[3 * v + 2] = in[3 * v + 2] + t2;
                 }
             } else {
 #pragma unroll
@@ -226,9 +235,9 @@ __global__ void __launch_bounds__(128, 5) k_dg_cell(const DgCase c, int stage, i
                     t1 = t1 + xd(0.0) * gy[v];
                     t2 = t2 + ihy * gy[v];
                     t0 = t0 * w; t1 = t1 * w; t2 = t2 * w;
-                    in[3 * v] = g == 0 ? pz(t0) : in[3 * v] + t0;
-                    in[3 * v + 1] = g == 0 ? pz(t1) : in[3 * v + 1] + t1;
-                    in[3 * v + 2] = g == 0 ? pz(t2) : in[3 * v + 2] + t2;
+                    in[3 * v] = in[3 * v] + t0;
+                    in[3 * v + 1] = in[3 * v + 1] + t1;
+                    in[3 * v + 2] = in[3 * v + 2] + t2;
                 }
             }
         }
