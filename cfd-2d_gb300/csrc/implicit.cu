@@ -156,120 +156,98 @@ __device__ __forceinline__ xd mul_half_l(xd s, xd hl, xd l) {
 }
 __device__ __forceinline__ xd plus_zero(xd x) { return xd(ip::plus_zero(x.v)); }
 
-// One face's 0.5 l R diag(lam+-) L (eigenValues / rightEigenVector / leftEigenVector /
-// calcAP / calcAM, :335-406, scaled by l in run, :572-600) from the Roe state (u, v, c,
-// H), with the normal (nx, ny) of the side being assembled. The reference forms
-// R diag(lam+) and R diag(lam-) as full 4x4 products and multiplies each by L, summing
-// four products from 0 per entry. An entry of R diag(lam+) is R[i][k] lam+_k or zero, and
-// a zero term never changes such a sum (started from +0 it cannot become -0), so column k
-// contributes to A+ only where lam_k > 0 and to A- only where lam_k < 0, in the
-// reference's order of k: the same bits with half the products.
-// Adds A+ into dg (the cell's diagonal block); returns A- in am.
-__device__ __forceinline__ void face_jacobians(xd u, xd v, xd c, xd H, xd GAM, xd nx, xd ny, xd l, xd* dg, xd* am) {
-    const xd hl = half(l);
-    const xd qn = u * nx + v * ny;
-    const xd q2 = u * u + v * v;
-    const xd lx = -ny, ly = nx;
-    const xd ql = u * lx + v * ly;
-    const xd g1 = GAM - xd(1.0), c2 = c * c;
-    // the quotients of leftEigenVector
-    const ip::Recip yc2 = recip_of(c2), yc = recip_of(c);
-    const xd A0 = div_y(half(q2) * g1, c2, yc2);
-    const xd B0 = div_y(qn, c, yc);
-    const xd Cu = div_y(g1 * u, c2, yc2);
-    const xd Dn = div_y(nx, c, yc);
-    const xd Ev = div_y(g1 * v, c2, yc2);
-    const xd Fn = div_y(ny, c, yc);
-    const xd G0 = div_y(half(g1), c2, yc2);
-    const xd Hg = div_y(g1, c2, yc2);
-    const xd L[16] = {half(A0 + B0), -half(Cu + Dn), -half(Ev + Fn), G0,
-                          xd(1.0) - A0,    Cu,               Ev,               neg_if(Hg, true),
-                          half(A0 - B0),  -half(Cu - Dn), -half(Ev - Fn), G0,
-                          neg_if(ql, true), lx,              ly,               xd(0.0)};
-    const xd lam[4] = {qn - c, qn, qn + c, qn};
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        xd Rr[4];
-        if (i == 0) { Rr[0] = xd(1.0); Rr[1] = xd(1.0); Rr[2] = xd(1.0); Rr[3] = xd(0.0); }
-        if (i == 1) { Rr[0] = u - c * nx; Rr[1] = u; Rr[2] = u + c * nx; Rr[3] = lx; }
-        if (i == 2) { Rr[0] = v - c * ny; Rr[1] = v; Rr[2] = v + c * ny; Rr[3] = ly; }
-        if (i == 3) { Rr[0] = H - qn * c; Rr[1] = half(q2); Rr[2] = H + qn * c; Rr[3] = ql; }
-        xd sp[4] = {xd(0.0), xd(0.0), xd(0.0), xd(0.0)}, sm[4] = {xd(0.0), xd(0.0), xd(0.0), xd(0.0)};
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const xd t = i == 0 && k < 3 ? lam[k] : Rr[k] * lam[k];  // 1.0 * lam
-            if (lam[k].v > 0) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) sp[j] = sp[j] + t * L[4 * k + j];
-            } else if (lam[k].v < 0) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) sm[j] = sm[j] + t * L[4 * k + j];
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const xd ap = mul_half_l(sp[j], hl, l);
-            dg[4 * i + j] = dg[4 * i + j] + ap;
-            am[4 * i + j] = plus_zero(mul_half_l(sm[j], hl, l));
-        }
-    }
-}
-
-// One block row of the system per cell (run's edge loop, :541-634, gathered per
-// cell in ascending edge order, and the diagonal S/cTau of :640-664): the Roe
-// average of the face's two centre states, the spectral radius (steady), A+ into
-// the diagonal block, A- as the face's block, and the right-hand side -sum F l/2.
-__global__ void __launch_bounds__(128, 4) k_imp_assemble(const ImpCase c) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.nc) return;
-    const int nc = c.nc;
-    const xd GAM(c.gam_flux);
-    xd dg[16];
-#pragma unroll
-    for (int m = 0; m < 16; m++) dg[m] = xd(0.0);
-    xd rhs[4] = {xd(0.0), xd(0.0), xd(0.0), xd(0.0)};
-    xd lam(0.0);
+// One block row of the system per cell (run's edge loop, :541-634, gathered per cell in
+// ascending edge order, and the diagonal S/cTau of :640-664), four lanes per cell, one per row:
+// per face the Roe average of its two centre states (k_imp_roe), A+ into the diagonal block, A-
+// as the face's block, and the right-hand side -sum F l/2; steady also the spectral radius.
+//
+// A+- = 0.5 l R diag(lam+-) L (eigenValues / rightEigenVector / leftEigenVector / calcAP /
+// calcAM, :335-406, scaled by l in run, :572-600), with the normal of the side being assembled.
+// The reference forms R diag(lam+) and R diag(lam-) as full 4x4 products and multiplies each by
+// L, summing four products from 0 per entry. An entry of R diag(lam+) is R[i][k] lam+_k or zero,
+// and a zero term never changes such a sum (started from +0 it cannot become -0), so column k
+// contributes to A+ only where lam_k > 0 and to A- only where lam_k < 0, in the reference's
+// order of k: the same bits with half the products.
+//
+// One thread per cell held L, A- and the diagonal block (192 registers) in a body larger than
+// the instruction cache; a lane holds one row of each, and the lanes divide L's quotients.
+__global__ void __launch_bounds__(128) k_imp_assemble(const ImpCase c) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if ((t & ~31) >= 4 * c.nc) return;
+    const bool live = t < 4 * c.nc;
+    const int i = live ? t >> 2 : c.nc - 1, row = t & 3, nc = c.nc;
+    const xd GAM(c.gam_flux), g1 = GAM - xd(1.0);
+    xd dg[4] = {xd(0.0), xd(0.0), xd(0.0), xd(0.0)}, rhs(0.0), lsum(0.0);
 #pragma unroll 1
     for (int k = 0; k < 3; k++) {
         const int f = c.face[k * nc + i], e = f >> 1;
         const bool side2 = f & 1;
-        double fe[4];
-        ld4(c.F, e, fe);
-#pragma unroll
-        for (int m = 0; m < 4; m++) rhs[m] = rhs[m] + xd(neg_if(fe[m], !side2));
-        const xd nx(c.nx[e]), ny(c.ny[e]), l(c.l[e]);
-        double ra[4];  // the edge's Roe state (u, v, c, H), formed once by k_imp_roe
+        rhs = rhs + xd(neg_if(c.F[4 * (size_t)e + row], !side2));
+        const xd nx(neg_if(c.nx[e], side2)), ny(neg_if(c.ny[e], side2)), l(c.l[e]), hl = half(l);
+        double ra[4];  // the edge's Roe state
         ld4(c.R, e, ra);
-        const xd a[4] = {xd(ra[0]), xd(ra[1]), xd(ra[2]), xd(ra[3])};
-        if (c.steady) lam = lam + (t_sqrt(a[0] * a[0] + a[1] * a[1]) + a[2]) * l;
-        xd am[16];
-        face_jacobians(a[0], a[1], a[2], a[3], GAM, neg_if(nx, side2), neg_if(ny, side2), l, dg, am);
-        const bool inner = e < c.n_int;
+        const xd u(ra[0]), v(ra[1]), cz(ra[2]), H(ra[3]);
+        if (c.steady) lsum = lsum + (t_sqrt(u * u + v * v) + cz) * l;
+        const xd qn = u * nx + v * ny, q2 = u * u + v * v;
+        const xd lx = -ny, ly = nx, ql = u * lx + v * ly;
+        // leftEigenVector's quotients: by c^2 in lanes 0-2, by c in lane 3
+        const xd d = row == 3 ? cz : cz * cz;
+        const ip::Recip y = recip_of(d);
+        const xd n0 = row == 0 ? half(q2) * g1 : row == 1 ? g1 * u : row == 2 ? g1 * v : qn;
+        const xd n1 = row == 0 ? half(g1) : row == 1 ? g1 : nx;
+        const xd r0 = div_y(n0, d, y), r1 = div_y(n1, d, y), r2 = div_y(ny, d, y);
+        auto from = [&](xd x, int lane) { return xd(__shfl_sync(0xffffffffu, x.v, lane, 4)); };
+        const xd G0 = from(r1, 0), Hg = from(r1, 1), Cu = from(r0, 1), Ev = from(r0, 2), A0 = from(r0, 0);
+        // A0 +- B0, Cu +- Dn, Ev +- Fn in lanes 0-2, 1 - A0 in lane 3
+        const xd B0 = from(r0, 3), Dn = from(r1, 3), Fn = from(r2, 3);
+        const xd x = row == 3 ? xd(1.0) : r0, z = row == 0 ? B0 : row == 1 ? Dn : row == 2 ? Fn : A0;
+        const xd hp = half(x + z), dm = x - z, hm = half(dm);
+        const xd L[16] = {from(hp, 0),  -from(hp, 1), -from(hp, 2), G0,
+                          from(dm, 3),  Cu,           Ev,           -Hg,
+                          from(hm, 0),  -from(hm, 1), -from(hm, 2), G0,
+                          -ql,          lx,           ly,           xd(0.0)};
+        const xd lam[4] = {qn - cz, qn, qn + cz, qn};
+        // this lane's row of R
+        const xd w = row == 1 ? nx : row == 2 ? ny : qn, b = row == 1 ? u : row == 2 ? v : H;
+        const xd cw = cz * w;
+        xd R[4] = {b - cw, b, b + cw, ly};
+        if (row == 0) { R[0] = xd(1.0); R[1] = xd(1.0); R[2] = xd(1.0); R[3] = xd(0.0); }
+        if (row == 1) R[3] = lx;
+        if (row == 3) { R[1] = half(q2); R[3] = ql; }
+        xd sp[4] = {xd(0.0), xd(0.0), xd(0.0), xd(0.0)}, sm[4] = {xd(0.0), xd(0.0), xd(0.0), xd(0.0)};
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            double2* o = reinterpret_cast<double2*>(c.O + oblk(nc, i, k, 0, q));
-            o[0] = inner ? make_double2(am[q].v, am[4 + q].v) : make_double2(0.0, 0.0);
-            o[1] = inner ? make_double2(am[8 + q].v, am[12 + q].v) : make_double2(0.0, 0.0);
+            const xd s = R[q] * lam[q];
+            // one sum, into the side the eigenvalue's sign names (cells of a warp differ in it)
+            const bool plus = lam[q].v > 0, minus = lam[q].v < 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const xd t = (plus ? sp[j] : sm[j]) + s * L[4 * q + j];
+                if (plus) sp[j] = t;
+                if (minus) sm[j] = t;
+            }
+        }
+        const bool inner = e < c.n_int;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            dg[j] = dg[j] + mul_half_l(sp[j], hl, l);
+            const xd am = plus_zero(mul_half_l(sm[j], hl, l));
+            if (live) c.O[oblk(nc, i, k, row, j)] = inner ? am.v : 0.0;
         }
     }
     const xd S(c.S[i]);
     xd tau;
     if (c.steady) {
-        tau = xd(2.0) * xd(*c.cfl) * S / (lam + xd(1.0e-100));
-        c.ctau[i] = tau.v;
+        tau = xd(2.0) * xd(*c.cfl) * S / (lsum + xd(1.0e-100));
+        if (live && row == 0) c.ctau[i] = tau.v;
     } else {
         tau = xd(c.ctau[i]);
     }
     const xd sd = S / tau;
+    if (!live) return;
 #pragma unroll
-    for (int m = 0; m < 16; m++) dg[m] = (m % 5) == 0 ? dg[m] + sd : plus_zero(dg[m]);  // + 0.0 off the diagonal
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        double2* d = reinterpret_cast<double2*>(c.D + dblk(nc, i, 0, q));
-        d[0] = make_double2(dg[q].v, dg[4 + q].v);
-        d[1] = make_double2(dg[8 + q].v, dg[12 + q].v);
-    }
-    st4(c.b, i, rhs[0].v, rhs[1].v, rhs[2].v, rhs[3].v);
+    for (int j = 0; j < 4; j++) c.D[dblk(nc, i, row, j)] = (j == row ? dg[j] + sd : plus_zero(dg[j])).v;  // + 0.0 off the diagonal
+    c.b[4 * (size_t)i + row] = rhs.v;
 }
 
 __device__ __forceinline__ bool solve_ok(const GmresCtl* g) { return g->final_ && !g->restart && g->status == 0; }
@@ -425,7 +403,7 @@ void imp_launch_flux(const ImpCase& c, cudaStream_t s) {
     k_imp_roe<<<blocks(c.ne, 128), 128, 0, s>>>(c);
 }
 void imp_launch_assemble(const ImpCase& c, cudaStream_t s) {
-    k_imp_assemble<<<blocks(c.nc, 128), 128, 0, s>>>(c);
+    k_imp_assemble<<<blocks(4 * c.nc, 128), 128, 0, s>>>(c);
 }
 void imp_launch_post(const ImpCase& c, cudaStream_t s) {
     k_imp_post_begin<<<1, 1, 0, s>>>(c);
