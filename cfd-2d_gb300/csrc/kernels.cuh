@@ -936,8 +936,9 @@ __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) 
 
 // MM: this project's arithmetic for minmod (FP64 only, grad_one_mm); FP32 faces the mixed
 // form's (grad_one_w); else the reference's
+// FP64 faces: 64 registers (32 warps on an SM; 80 and 24 without the bound, 1-2% slower)
 template <typename T, bool STRIDE, bool MM = false>
-__global__ void __launch_bounds__(256) k_grad(const DevCase c) {
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 0) k_grad(const DevCase c) {
     static_assert(!MM || sizeof(T) == 8, "the minmod gradient arithmetic is FP64's");
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (!STRIDE) {  // one thread per item
