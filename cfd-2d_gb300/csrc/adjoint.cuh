@@ -85,8 +85,7 @@ __device__ __forceinline__ void vjp_cons2prim(const T* U, T gm1, const Prim<T>& 
 // (E = p/(r gm1) + (u^2 + v^2)/2): no read of the FP64 state.
 template <typename T>
 __device__ __forceinline__ void vjp_cons2prim_q(const Prim<T>& q, T gm1, const Prim<T>& pb, T* Ub) {
-    // derivative factors only: Newton-refined reciprocal and quotient (FP64; FP32 divides)
-    const T ro = q.r, iro = hllc_recip(ro), u = q.u, v = q.v;
+        const T ro = q.r, iro = hllc_recip(ro), u = q.u, v = q.v;
     const T e = hllc_quot(q.p, ro * gm1);
     const T E = madd(e, T(0.5), t_fma(u, u, v * v));
     T rb = madd(pb.r, pb.p * e, gm1);
@@ -198,18 +197,10 @@ __device__ __forceinline__ void vjp_lax(const Prim<T>& L, const Prim<T>& R, T nx
     Lb.u += unlb * nx; Lb.v += unlb * ny; Rb.u += unrb * nx; Rb.v += unrb * ny;
 }
 
-// Ss = num / den as the forward forms it (hllc_quot: the forward's quotient bit for bit),
-// with an approximation of 1/den for the derivatives (the Newton reciprocal hllc_quot
-// starts from; FP32: a division)
-__device__ __forceinline__ double star_speed(double num, double den, double& iden) {
-    iden = hllc_in_range(den) ? hllc_rcp1(den) : 1.0 / den;
-    return hllc_quot(num, den);
-}
+// Ss = num / den as the forward forms it (hllc_quot), and 1/den for the derivatives
 __device__ __forceinline__ xd star_speed(xd num, xd den, xd& iden) {
-    double y;
-    const double s = star_speed(num.v, den.v, y);
-    iden = xd(y);
-    return xd(s);
+    iden = hllc_recip(den);
+    return hllc_quot(num, den);
 }
 __device__ __forceinline__ float star_speed(float num, float den, float& iden) {
     iden = 1.0f / den;
@@ -325,7 +316,7 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<xd>& L, const Prim<xd>& R,
     typedef xd T;
     const T unL = dot2(L.u, nx, L.v, ny), unR = dot2(R.u, nx, R.v, ny);
     const T sl1 = unL - cL, sl2 = unR - cR, sr1 = unL + cL, sr2 = unR + cR;
-    const bool l1 = sl1 < sl2, r1 = sr1 > sr2;
+    const bool l1 = ip::less(sl1.v, sl2.v), r1 = ip::less(sr2.v, sr1.v);
     const T SL = l1 ? sl1 : sl2, SR = r1 ? sr1 : sr2;
     T unLb = acc0<T>(), unRb = acc0<T>(), SLb = acc0<T>(), SRb = acc0<T>(), cLb = acc0<T>(), cRb = acc0<T>();
     // E = p IG1 + .5 r (u^2 + v^2): the adjoint Eb of one side's energy into its state
@@ -334,9 +325,9 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<xd>& L, const Prim<xd>& R,
         qb.p = madd(qb.p, Eb, IG1); qb.r = madd(qb.r, half(Eb), t_fma(q.u, q.u, q.v * q.v));
         qb.u = madd(qb.u, e, q.u); qb.v = madd(qb.v, e, q.v);
     };
-    if (SL >= T(0.0) || SR <= T(0.0)) {  // supersonic: the upwind side's physical flux
+    if (not_negative(SL) || not_negative(-SR)) {  // supersonic: the upwind side's physical flux
         T Eb = acc0<T>();
-        if (SL >= T(0.0)) {
+        if (not_negative(SL)) {
             vjp_phys(L.r, L.u, L.v, L.p, energy(L.r, L.u, L.v, L.p, IG1), unL, nx, ny, fb, Lb.r, Lb.u, Lb.v, Lb.p,
                      Eb, unLb);
             energy_bar(L, Eb, Lb);
@@ -351,7 +342,7 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<xd>& L, const Prim<xd>& R,
         const T num = t_fma(-mR, unR, t_fma(mL, unL, R.p - L.p)), den = mL - mR;
         T iden;
         const T Ss = star_speed(num, den, iden);
-        const bool left = Ss >= T(0.0);
+        const bool left = not_negative(Ss);
         const Prim<T>& K = left ? L : R;
         const T SK = left ? SL : SR, unK = left ? unL : unR, dK = left ? dL : dR, mK = left ? mL : mR;
         const T EK = energy(K.r, K.u, K.v, K.p, IG1);

@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(128) k_imp_assemble(const ImpCase c) {
         for (int q = 0; q < 4; q++) {
             const xd s = R[q] * lam[q];
             // one sum, into the side the eigenvalue's sign names (cells of a warp differ in it)
-            const bool plus = lam[q].v > 0, minus = lam[q].v < 0;
+            const bool plus = ip::positive(lam[q].v), minus = ip::positive((-lam[q]).v);
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const xd t = (plus ? sp[j] : sm[j]) + s * L[4 * q + j];

@@ -430,6 +430,27 @@ IP_FN double pow(double x, double a) {
     return pow_rare(x, a);
 }
 
+// a < b and x >= 0 (false for NaN) without an FP64 comparison
+#if defined(__CUDA_ARCH__)
+static __device__ __noinline__ bool less_rare(double a, double b) { return a < b; }
+#else
+static inline bool less_rare(double a, double b) { return a < b; }
+#endif
+IP_FN bool less(double a, double b) {
+    // the bits of a negative number inverted below its sign: ordered as integers
+    const u32 na = (u32)((int)hi(a) >> 31), nb = (u32)((int)hi(b) >> 31);
+    const int ah = (int)(hi(a) ^ (na >> 1)), bh = (int)(hi(b) ^ (nb >> 1));
+    if (__builtin_expect(in_range(a) && in_range(b), 1)) return ah < bh || (ah == bh && (lo(a) ^ na) < (lo(b) ^ nb));
+    return less_rare(a, b);
+}
+IP_FN bool positive(double x) {  // 0 < x
+    const long long b = (long long)(((u64)hi(x) << 32) | lo(x));
+    return b > 0 && b <= 0x7ff0000000000000ll;
+}
+IP_FN bool not_negative(double x) {  // 0 <= x, -0 too
+    const u64 b = ((u64)hi(x) << 32) | lo(x);
+    return b <= 0x7ff0000000000000ull || b == 0x8000000000000000ull;
+}
 // x / 2: exact for normal results and zeros, by the exponent
 IP_FN double half(double x) {
     const u32 xa = hi(x) & 0x7fffffffu;

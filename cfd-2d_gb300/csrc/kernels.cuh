@@ -24,14 +24,14 @@ struct Prim { T r, u, v, p; };
 template <typename A, typename T>
 __device__ __forceinline__ Prim<A> prim_as(const Prim<T>& q) { return Prim<A>{A(q.r), A(q.u), A(q.v), A(q.p)}; }
 
+// FP64 face arithmetic: sums on the FP64 unit, products, quotients and square roots on the
+// integer pipes (intpipe.cuh; the same bits as double's)
+using ip::xd;
 __device__ __forceinline__ double t_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float t_sqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double t_abs(double x) { return fabs(x); }
 __device__ __forceinline__ float t_abs(float x) { return fabsf(x); }
 __device__ __forceinline__ double t_fma(double a, double b, double c) { return fma(a, b, c); }
-// FP64 face arithmetic: sums on the FP64 unit, products, quotients and square roots on the
-// integer pipes (intpipe.cuh; the same bits as double's)
-using ip::xd;
 __device__ __forceinline__ xd t_sqrt(xd x) { return xd(ip::sqrt(x.v)); }
 // x^a for positive x (the reference's exp(log(x) a))
 __device__ __forceinline__ xd t_pow(xd x, xd a) { return xd(ip::pow(x.v, a.v)); }
@@ -52,6 +52,11 @@ template <> struct WideArith<double> { typedef xd type; };
 __device__ __forceinline__ float t_fma(float a, float b, float c) { return fmaf(a, b, c); }
 template <typename T> __device__ __forceinline__ T t_max(T a, T b) { return a > b ? a : b; }  // _max_, src/mesh/grid.h:102
 template <typename T> __device__ __forceinline__ T t_min(T a, T b) { return a < b ? a : b; }
+// FP64 faces compare on the integer pipes
+__device__ __forceinline__ xd t_max(xd a, xd b) { return ip::less(b.v, a.v) ? a : b; }
+__device__ __forceinline__ xd t_min(xd a, xd b) { return ip::less(a.v, b.v) ? a : b; }
+__device__ __forceinline__ bool not_negative(xd x) { return ip::not_negative(x.v); }  // x >= 0
+__device__ __forceinline__ bool not_negative(float x) { return x >= 0.0f; }
 
 template <typename T> __device__ __forceinline__ const T* W_of(const DevCase& c);
 template <> __device__ __forceinline__ const double* W_of<double>(const DevCase& c) { return c.W64; }
@@ -508,74 +513,14 @@ template <typename T> __device__ __forceinline__ T energy(T r, T u, T v, T p, T 
     return t_fma(p, IG1, half(r) * t_fma(u, u, v * v));
 }
 
-// Newton-refined quotient, reciprocal and sound speed of the FP64 HLLC flux. HLLC has no
-// counterpart in the reference, so its arithmetic is this project's definition and the
-// oracle performs the very same operations (same bits): a binary32 seed, then FP64 Newton
-// steps with fused multiply-adds (Newton-Raphson for 1/b and for sqrt(a/r), the final
-// quotient corrected as in Markstein, "IA-64 and Elementary Functions", 2000). The seed
-// is x truncated to binary32 (sign, rebiased exponent, top 23 fraction bits: integer
-// operations) and the binary32 operations are correctly rounded (IEEE), so every step is
-// defined bit for bit. Within |x| in [2^-60, 2^60) every binary32 value stays normal and
-// every result is within about one ulp of the exact one; other operands take the IEEE
-// expression. Each costs 4-6 FP64 instructions where a division or square root costs ~9.
-__device__ __forceinline__ bool hllc_in_range(double x) {  // 2^-60 <= |x| < 2^60
-    const int e = (int)((__double_as_longlong(x) >> 52) & 0x7ff);
-    return e >= 1023 - 60 && e < 1023 + 60;
-}
-__device__ __forceinline__ float hllc_seed(double x) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    const unsigned sgn = (unsigned)(b >> 32) & 0x80000000u;
-    const unsigned ex = (unsigned)((b >> 52) & 0x7ff) - (1023u - 127u);
-    return __uint_as_float(sgn | (ex << 23) | ((unsigned)(b >> 29) & 0x7fffffu));
-}
-// 1/b to ~2^-46 (one Newton step from the binary32 reciprocal of the seed)
-__device__ __forceinline__ double hllc_rcp1(double b) {
-    const double y0 = widen(__frcp_rn(hllc_seed(b)));
-    return fma(y0, fma(-b, y0, ip::one()), y0);
-}
-// a / b: one Newton step for 1/b, then q = a y corrected once (|a|, |b| in range; a = 0
-// gives the IEEE signed zero)
-// (the IEEE fallbacks sit in functions of their own so that the compiler branches to them
-// instead of issuing them, predicated off, beside the common path)
-static __device__ __noinline__ double recip_outright(double b) { return 1.0 / b; }
-static __device__ __noinline__ double sound_outright(double a, double r) { return sqrt(a / r); }
-__device__ __forceinline__ double hllc_quot(double a, double b) {
-    if (hllc_in_range(b)) {
-        if (__builtin_expect(hllc_in_range(a), 1)) {
-            const double y = hllc_rcp1(b);
-            const double q = ip::mul(a, y);
-            return fma(fma(-q, b, a), y, q);
-        }
-        const long long ia = __double_as_longlong(a);
-        if ((ia & 0x7fffffffffffffffll) == 0)
-            return __longlong_as_double((ia ^ __double_as_longlong(b)) & (long long)0x8000000000000000ull);
-    }
-    return div_outright(a, b);
-}
-__device__ __forceinline__ xd hllc_quot(xd a, xd b) { return xd(hllc_quot(a.v, b.v)); }
+// Quotient, reciprocal and sound speed sqrt(a / r) of the HLLC and Roe fluxes: IEEE, on the
+// integer pipes with FP64 faces. (Newton sequences of FP64 multiply-adds from binary32 seeds,
+// 4 to 6 instructions each, held the FP64 unit longer: a flux evaluation had 16 of them.)
+__device__ __forceinline__ xd hllc_quot(xd a, xd b) { return a / b; }
 __device__ __forceinline__ float hllc_quot(float a, float b) { return a / b; }
-// 1/b: two Newton steps
-__device__ __forceinline__ double hllc_recip(double b) {
-    if (__builtin_expect(!hllc_in_range(b), 0)) return recip_outright(b);
-    const double y = hllc_rcp1(b);
-    return fma(y, fma(-b, y, ip::one()), y);
-}
-__device__ __forceinline__ xd hllc_recip(xd b) { return xd(hllc_recip(b.v)); }
+__device__ __forceinline__ xd hllc_recip(xd b) { return xd(ip::rcp(b.v)); }
 __device__ __forceinline__ float hllc_recip(float b) { return 1.0f / b; }
-// sqrt(a / r) for a = GAMMA p, r the density (both positive and in range): s0 and
-// h = 1/(2 r s0) from binary32, then two steps s <- s + (a - (r s) s) h
-__device__ __forceinline__ double hllc_sound(double a, double r) {
-    const long long ia = __double_as_longlong(a), ir = __double_as_longlong(r);
-    if (__builtin_expect(ia < 0 || ir < 0 || !hllc_in_range(a) || !hllc_in_range(r), 0)) return sound_outright(a, r);
-    const float af = hllc_seed(a), rf = hllc_seed(r);
-    const float sf = __fsqrt_rn(__fdiv_rn(af, rf));
-    const double h = widen(__fdiv_rn(0.5f, __fmul_rn(rf, sf)));
-    double s = widen(sf);
-    s = fma(fma(ip::neg(ip::mul(r, s)), s, a), h, s);
-    s = fma(fma(ip::neg(ip::mul(r, s)), s, a), h, s);
-    return s;
-}
-__device__ __forceinline__ xd hllc_sound(xd a, xd r) { return xd(hllc_sound(a.v, r.v)); }
+__device__ __forceinline__ xd hllc_sound(xd a, xd r) { return t_sqrt(a / r); }
 __device__ __forceinline__ float hllc_sound(float a, float r) { return t_sqrt(a / r); }
 
 // HLLC (Toro, Riemann Solvers and Numerical Methods for Fluid Dynamics, sec. 10.4-10.6),
@@ -583,8 +528,7 @@ __device__ __forceinline__ float hllc_sound(float a, float r) { return t_sqrt(a 
 // F*_K = [S*(S_K U_K - F_K) + S_K p* D*] / (S_K - S*), D* = (0, nx, ny, S*),
 // p* = p_K + rho_K (S_K - un_K)(S* - un_K): one division instead of Toro's star state;
 // S_K U_K - F_K is formed from m_K = rho_K (S_K - un_K) and only the side that is used
-// forms its energy. FP64: c = hllc_sound(GAMMA p, rho), S* = hllc_quot,
-// 1/(S_K - S*) = hllc_recip.
+// forms its energy.
 // FP32 faces (the mixed form): both energies up front and the star flux from the physical
 // flux F_K; without branches on the energies this measured faster there (124 against
 // 151 us per flux launch at 2.1M triangles).
@@ -617,12 +561,12 @@ template <typename T>
 __device__ __forceinline__ void flux_hllc_c(T* f, const Prim<T>& L, const Prim<T>& R, T cL, T cR, T nx, T ny, T IG1) {
     T unL = dot2(L.u, nx, L.v, ny), unR = dot2(R.u, nx, R.v, ny);
     T SL = t_min(unL - cL, unR - cR), SR = t_max(unL + cL, unR + cR);
-    if (SL >= T(0.0)) { phys_flux(f, L.r, L.u, L.v, L.p, energy(L.r, L.u, L.v, L.p, IG1), unL, nx, ny); return; }
-    if (SR <= T(0.0)) { phys_flux(f, R.r, R.u, R.v, R.p, energy(R.r, R.u, R.v, R.p, IG1), unR, nx, ny); return; }
+    if (not_negative(SL)) { phys_flux(f, L.r, L.u, L.v, L.p, energy(L.r, L.u, L.v, L.p, IG1), unL, nx, ny); return; }
+    if (not_negative(-SR)) { phys_flux(f, R.r, R.u, R.v, R.p, energy(R.r, R.u, R.v, R.p, IG1), unR, nx, ny); return; }
     T dL = SL - unL, dR = SR - unR;
     T mL = L.r * dL, mR = R.r * dR;
     T Ss = hllc_quot(t_fma(-mR, unR, t_fma(mL, unL, R.p - L.p)), mL - mR);
-    const bool left = Ss >= T(0.0);
+    const bool left = not_negative(Ss);
     const Prim<T>& K = left ? L : R;
     T SK = left ? SL : SR, unK = left ? unL : unR, dK = left ? dL : dR, mK = left ? mL : mR;
     T EK = energy(K.r, K.u, K.v, K.p, IG1);
@@ -691,44 +635,22 @@ __device__ __forceinline__ void flux_roe(T* f, const Prim<T>& L, const Prim<T>& 
     f[3] = T(0.5) * (FL[3] + FR[3] - D3);
 }
 
-// 1/sqrt(x) for x > 0 in [2^-60, 2^60): t = RN32(1 / RN32(sqrt(x truncated to binary32))),
-// then two Newton steps t <- t + (t/2)(1 - x t t); other operands: IEEE
-static __device__ __noinline__ double rsqrt_outright(double x) { return 1.0 / sqrt(x); }
-__device__ __forceinline__ double roe_rsqrt(double x) {
-    if (__builtin_expect(__double_as_longlong(x) <= 0 || !hllc_in_range(x), 0)) return rsqrt_outright(x);
-    double t = widen(__fdiv_rn(1.0f, __fsqrt_rn(hllc_seed(x))));
-    t = fma(ip::half(t), fma(ip::neg(ip::mul(x, t)), t, ip::one()), t);
-    t = fma(ip::half(t), fma(ip::neg(ip::mul(x, t)), t, ip::one()), t);
-    return t;
-}
-__device__ __forceinline__ xd roe_rsqrt(xd x) { return xd(roe_rsqrt(x.v)); }
-static __device__ __noinline__ double sqrt_outright(double x) { return sqrt(x); }
-
 // The Roe flux with FP64 faces, this project's arithmetic (the oracle's flux_roe does the
 // same): the Roe averages from t = 1/sqrt(rho) (sqrt(rho) = rho t, sqrt(rho) H = (E + p) t),
-// c~ = c~^2 t~ and 1/c~^2 = t~^2 with t~ = 1/sqrt(c~^2), the side sound speeds as HLLC's,
-// 1/(sqrt(rho_L) + sqrt(rho_R)) Newton-refined, and the wave sums fused.
+// the side sound speeds as HLLC's, and the wave sums fused.
 __device__ __forceinline__ void flux_roe(xd* f, const Prim<xd>& L, const Prim<xd>& R, xd nx, xd ny, xd GAM,
                                          xd IG1) {
     const xd G1 = GAM - xd(1.0);
     const xd unL = dot2(L.u, nx, L.v, ny), unR = dot2(R.u, nx, R.v, ny);
     const xd EL = energy(L.r, L.u, L.v, L.p, IG1), ER = energy(R.r, R.u, R.v, R.p, IG1);
-    const xd tL = roe_rsqrt(L.r), tR = roe_rsqrt(R.r);
+    const xd tL = hllc_recip(t_sqrt(L.r)), tR = hllc_recip(t_sqrt(R.r));
     const xd sL = L.r * tL, sR = R.r * tR;
     const xd w = hllc_recip(sL + sR);
     const xd ut = t_fma(sL, L.u, sR * R.u) * w, vt = t_fma(sL, L.v, sR * R.v) * w;
     const xd Ht = t_fma(EL + L.p, tL, (ER + R.p) * tR) * w;
     const xd q2 = t_fma(ut, ut, vt * vt);
     const xd c2 = G1 * t_fma(xd(ip::reg(-0.5)), q2, Ht);
-    xd c, ic2;
-    if (__builtin_expect(c2.v > 0.0 && hllc_in_range(c2.v), 1)) {
-        const xd t = roe_rsqrt(c2);
-        c = c2 * t;
-        ic2 = t * t;
-    } else {
-        c = xd(sqrt_outright(c2.v));
-        ic2 = xd(recip_outright(c2.v));
-    }
+    const xd c = t_sqrt(c2), ic2 = hllc_recip(c2);
     const xd unt = dot2(ut, nx, vt, ny);
     const xd rt = sL * sR;
     const xd dr = R.r - L.r, dp = R.p - L.p, dun = unR - unL;

@@ -467,61 +467,8 @@ static double energy(double r, double u, double v, double p, double IG1) {
     return fma(p, IG1, (0.5 * r) * fma(u, u, v * v));
 }
 
-/* Newton-refined quotient, reciprocal and sound speed of the FP64 HLLC flux: this
- * project's definition of that flux's arithmetic, the same operations as the GPU
- * (hllc_quot / hllc_recip / hllc_sound in the library's kernels). A binary32 seed
- * (x truncated: sign, rebiased exponent, top 23 fraction bits), correctly rounded
- * binary32 operations, then FP64 Newton steps with fma (Newton-Raphson for 1/b and
- * sqrt(a/r); the quotient corrected as in Markstein, "IA-64 and Elementary
- * Functions", 2000). Within |x| in [2^-60, 2^60) every binary32 value is normal;
- * other operands take the IEEE expression. */
-static int hllc_in_range(double x) {
-    uint64_t b;
-    memcpy(&b, &x, 8);
-    int e = (int)((b >> 52) & 0x7ff);
-    return e >= 1023 - 60 && e < 1023 + 60;
-}
-static float hllc_seed(double x) {
-    uint64_t b;
-    memcpy(&b, &x, 8);
-    uint32_t sgn = (uint32_t)(b >> 32) & 0x80000000u;
-    uint32_t ex = (uint32_t)((b >> 52) & 0x7ff) - (1023u - 127u);
-    uint32_t f = sgn | (ex << 23) | ((uint32_t)(b >> 29) & 0x7fffffu);
-    float r;
-    memcpy(&r, &f, 4);
-    return r;
-}
-static double hllc_rcp1(double b) {
-    double y0 = (double)(1.0f / hllc_seed(b));  /* a correctly rounded binary32 division */
-    return fma(y0, fma(-b, y0, 1.0), y0);
-}
-static double hllc_quot(double a, double b) {
-    if (hllc_in_range(b)) {
-        if (hllc_in_range(a)) {
-            double y = hllc_rcp1(b), q = a * y;
-            return fma(fma(-q, b, a), y, q);
-        }
-        if (a == 0.0) return copysign(0.0, a) * copysign(1.0, b);
-    }
-    return a / b;
-}
-static double hllc_recip(double b) {
-    if (!hllc_in_range(b)) return 1.0 / b;
-    double y = hllc_rcp1(b);
-    return fma(y, fma(-b, y, 1.0), y);
-}
-static double hllc_sound(double a, double r) {
-    if (!(a > 0.0) || !(r > 0.0) || !hllc_in_range(a) || !hllc_in_range(r)) return sqrt(a / r);
-    float af = hllc_seed(a), rf = hllc_seed(r);
-    float qf = af / rf;
-    float sf = sqrtf(qf);
-    float tf = rf * sf;
-    float hf = 0.5f / tf;
-    double h = (double)hf, s = (double)sf;
-    s = fma(fma(-(r * s), s, a), h, s);
-    s = fma(fma(-(r * s), s, a), h, s);
-    return s;
-}
+/* Sound speed of the HLLC and Roe fluxes: the IEEE quotient and square root. */
+static double hllc_sound(double a, double r) { return sqrt(a / r); }
 
 /* HLLC flux (Toro, Riemann Solvers and Numerical Methods for Fluid Dynamics,
  * 3rd ed., sec. 10.4-10.6) with Davis wave-speed estimates
@@ -532,8 +479,7 @@ static double hllc_sound(double a, double r) {
  * which equals F_K + S_K (U*_K - U_K) for Toro's star state U*_K, with
  *   S_K U_K - F_K = (m_K, m_K u - p nx, m_K v - p ny, E_K (S_K - un_K) - p un_K),
  *   m_K = rho_K (S_K - un_K); only the side used forms its energy. Energies use
- * p/(gamma-1) as p * (1/(gamma-1)). c = hllc_sound(GAMMA p, rho), S* = hllc_quot,
- * 1/(S_K - S*) = hllc_recip. */
+ * p/(gamma-1) as p * (1/(gamma-1)). c = hllc_sound(GAMMA p, rho). */
 static void flux_hllc(double* f, const Par* pL, const Par* pR, double nx, double ny, double GAM) {
     double IG1 = 1.0 / (GAM - 1.0);
     double cL = hllc_sound(GAM * pL->p, pL->r), cR = hllc_sound(GAM * pR->p, pR->r);
@@ -549,7 +495,7 @@ static void flux_hllc(double* f, const Par* pL, const Par* pR, double nx, double
     }
     double dL = SL - unL, dR = SR - unR;
     double mL = pL->r * dL, mR = pR->r * dR;
-    double Ss = hllc_quot(fma(-mR, unR, fma(mL, unL, pR->p - pL->p)), mL - mR);
+    double Ss = fma(-mR, unR, fma(mL, unL, pR->p - pL->p)) / (mL - mR);
     const Par* K; double SK, unK, dK, mK;
     if (Ss >= 0.0) { K = pL; SK = SL; unK = unL; dK = dL; mK = mL; }
     else { K = pR; SK = SR; unK = unR; dK = dR; mK = mR; }
@@ -557,7 +503,7 @@ static void flux_hllc(double* f, const Par* pL, const Par* pR, double nx, double
     /* S_K U_K - F_K = (m_K, m_K u - p nx, m_K v - p ny, E_K (S_K - un_K) - p un_K) */
     double A1 = fma(mK, K->u, -(K->p * nx)), A2 = fma(mK, K->v, -(K->p * ny)), A3 = fma(EK, dK, -(K->p * unK));
     double ps = fma(mK, Ss - unK, K->p);
-    double inv = hllc_recip(SK - Ss);
+    double inv = 1.0 / (SK - Ss);
     double sp = SK * ps;
     f[0] = (Ss * mK) * inv;
     f[1] = fma(Ss, A1, sp * nx) * inv;
@@ -565,47 +511,26 @@ static void flux_hllc(double* f, const Par* pL, const Par* pR, double nx, double
     f[3] = fma(Ss, A3, sp * Ss) * inv;
 }
 
-/* 1/sqrt(x) for x > 0 in [2^-60, 2^60): t = RN32(1 / RN32(sqrt(x truncated to binary32))),
- * then two Newton steps t <- t + (t/2)(1 - x t t); other operands: IEEE. */
-static double roe_rsqrt(double x) {
-    if (!(x > 0.0) || !hllc_in_range(x)) return 1.0 / sqrt(x);
-    float sf = sqrtf(hllc_seed(x));
-    float tf = 1.0f / sf;
-    double t = (double)tf;
-    t = fma(0.5 * t, fma(-(x * t), t, 1.0), t);
-    t = fma(0.5 * t, fma(-(x * t), t, 1.0), t);
-    return t;
-}
-
 /* Roe flux (Roe, J. Comput. Phys. 43, 1981) in the face-normal frame with the
  * Harten-Hyman entropy fix on the acoustic waves (Harten & Hyman, J. Comput.
  * Phys. 50, 1983): delta = max(0, lam~ - lam_L, lam_R - lam~), |lam~| -> delta
  * where |lam~| < delta. Roe averages as in the reference's roe_orig
  * (src/global.cpp:407-441). This project's arithmetic: the averages from
- * t = 1/sqrt(rho) (sqrt(rho) = rho t, sqrt(rho) H = (E + p) t), c~ = c~^2 t~ and
- * 1/c~^2 = t~^2 with t~ = 1/sqrt(c~^2), the side sound speeds as HLLC's,
- * 1/(sqrt(rho_L) + sqrt(rho_R)) Newton-refined, the wave sums fused. */
+ * t = 1/sqrt(rho) (sqrt(rho) = rho t, sqrt(rho) H = (E + p) t), the side sound speeds
+ * as HLLC's, the wave sums fused. */
 static void flux_roe(double* f, const Par* pL, const Par* pR, double nx, double ny, double GAM) {
     double G1 = GAM - 1.0, IG1 = 1.0 / (GAM - 1.0);
     double unL = dot2(pL->u, nx, pL->v, ny), unR = dot2(pR->u, nx, pR->v, ny);
     double EL = energy(pL->r, pL->u, pL->v, pL->p, IG1);
     double ER = energy(pR->r, pR->u, pR->v, pR->p, IG1);
-    double tL = roe_rsqrt(pL->r), tR = roe_rsqrt(pR->r);
+    double tL = 1.0 / sqrt(pL->r), tR = 1.0 / sqrt(pR->r);
     double sL = pL->r * tL, sR = pR->r * tR;
-    double w = hllc_recip(sL + sR);
+    double w = 1.0 / (sL + sR);
     double ut = fma(sL, pL->u, sR * pR->u) * w, vt = fma(sL, pL->v, sR * pR->v) * w;
     double Ht = fma(EL + pL->p, tL, (ER + pR->p) * tR) * w;
     double q2 = fma(ut, ut, vt * vt);
     double c2 = G1 * fma(-0.5, q2, Ht);
-    double c, ic2;
-    if (c2 > 0.0 && hllc_in_range(c2)) {
-        double t = roe_rsqrt(c2);
-        c = c2 * t;
-        ic2 = t * t;
-    } else {
-        c = sqrt(c2);
-        ic2 = 1.0 / c2;
-    }
+    double c = sqrt(c2), ic2 = 1.0 / c2;
     double unt = dot2(ut, nx, vt, ny);
     double rt = sL * sR;
     double dr = pR->r - pL->r, dp = pR->p - pL->p, dun = unR - unL;
