@@ -63,6 +63,7 @@ ImplicitSolver::ImplicitSolver(const TaskConfig& t, Topo&& topo, const std::vect
         c.smoothing = task_.smoothing;
         c.newton_cap = task_.newton_cap;
         c.kdim = task_.gmres_kdim;
+        c.red = imp_red_blocks(nc);
         c.maxit = task_.gmres_maxit;
         c.eps = task_.gmres_eps;
         c.smoothing_par = task_.smoothing_par;
@@ -416,12 +417,12 @@ void ImplicitSolver::profile_steps(int n, double ms[4], int launches[4]) {
     for (int k = 0; k < 4; k++) { ms[k] = 0.0; launches[k] = 0; }
     cudaEvent_t ev[5];
     for (auto& e : ev) CUDA_CHECK(cudaEventCreate(&e));
-    // kernels of one GMRES cycle and the update: reset, |src|, v0; per column spmv, the
-    // inner-product passes (12 vectors each), hcol, orth, givens; solve, x, residual,
-    // finish; post_begin, [smoothing], update, remediation, count
+    // kernels of one GMRES cycle and the update: |src|, v0; per column the product with its
+    // first 12 inner products, further ones 12 at a time, orth; solve, x, residual, finish;
+    // [smoothing], update, remediation, count
     const int jmax = std::min(ic_.kdim, ic_.maxit);
-    int gm_launches = 3 + 4 + 4 + (task_.smoothing ? 1 : 0);
-    for (int j = 0; j < jmax; j++) gm_launches += 4 + (j + 12) / 12;
+    int gm_launches = 2 + 4 + 3 + (task_.smoothing ? 1 : 0);
+    for (int j = 0; j < jmax; j++) gm_launches += 2 + j / 12;
     for (int s = 0; s < n; s++) {
         if (!task_.steady) t_ += task_.tau;
         if (!solver_err_) steps_++;

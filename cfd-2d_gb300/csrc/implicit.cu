@@ -372,11 +372,6 @@ __global__ void __launch_bounds__(256) k_imp_count(const ImpCase c) {
     if (threadIdx.x == 0 && n && solve_ok(c.ctl)) atomicAdd(&c.ctl->n_lim, n);
 }
 
-__global__ void k_imp_post_begin(const ImpCase c) {
-    *c.n_lim = 0;
-    c.ctl->n_lim = 0;
-}
-
 // storage -> reference cell order of the block system: which 0 = D (16 per cell),
 // 1 = O (48 per cell), 2 = b (4 per cell)
 __global__ void __launch_bounds__(256) k_imp_permute(const ImpCase c, double* __restrict__ dst, int which) {
@@ -406,7 +401,6 @@ void imp_launch_assemble(const ImpCase& c, cudaStream_t s) {
     k_imp_assemble<<<blocks(4 * c.nc, 128), 128, 0, s>>>(c);
 }
 void imp_launch_post(const ImpCase& c, cudaStream_t s) {
-    k_imp_post_begin<<<1, 1, 0, s>>>(c);
     const double* dx = c.x;
     if (c.smoothing) {
         k_imp_smooth<<<blocks(c.nc, 256), 256, 0, s>>>(c);

@@ -37,18 +37,22 @@ enum ImpBndKind { IBND_INLET = 1, IBND_OUTLET = 2, IBND_WALL = 3 };
 enum : int { SOLVE_OK = 0, SOLVE_MAX_ITER = 0x2, SOLVE_CONVERG = 0x4 };
 
 constexpr int kGmresMaxKdim = 64;   // Krylov dimension bound of the device control block
-constexpr int kRedBlocks = 608;     // blocks of every reduction kernel (4 per SM)
+constexpr int kRedBlocks = 456;     // most blocks of a reduction kernel (3 per SM)
+
+constexpr int kNotDone = 1 << 30;   // GmresCtl::done_col while the Arnoldi loop runs
 
 // GMRES state shared by the kernels of one solve (device memory).
 struct GmresCtl {
     double bnorm, eps_abs, rnorm, rel;
     double H[(kGmresMaxKdim + 1) * kGmresMaxKdim];  // H[i * kdim + j]
-    double cs[kGmresMaxKdim], sn[kGmresMaxKdim], g[kGmresMaxKdim + 1], y[kGmresMaxKdim];
+    // rotations; g: the residual estimates (g[0] = beta), gr: the rotated right-hand side
+    double cs[kGmresMaxKdim], sn[kGmresMaxKdim], g[kGmresMaxKdim + 1], gr[kGmresMaxKdim], y[kGmresMaxKdim];
     double s[kGmresMaxKdim + 1];     // Krylov vector k is s[k] V_k (V_k stored unscaled)
-    double coef[kGmresMaxKdim];      // h_ij s_i of the column being orthogonalised
+    double hraw[kGmresMaxKdim];      // h_ij of the column being orthogonalised
     int it;        // iterations over all cycles
+    int it0;       // iterations before the current cycle
     int cols;      // columns of the current cycle
-    int done;      // the cycle's Arnoldi loop has ended
+    int done_col;  // the column that ended the cycle's Arnoldi loop (-2: none was needed)
     int status;    // SOLVE_* bits once final
     int restart;   // the true residual asks for another cycle
     int final_;    // the solve has ended (converged, failed or out of iterations)
@@ -62,6 +66,7 @@ struct ImpCase {
     int flux;                 // FLUX_GODUNOV or FLUX_LAX
     int steady, smoothing, newton_cap;
     int kdim, maxit;
+    int red;                  // blocks of the reduction kernels (imp_red_blocks)
     double eps;               // GMRES relative tolerance
     double smoothing_par;
     double tau_xml;
@@ -115,6 +120,7 @@ void imp_launch_flux(const ImpCase& c, cudaStream_t s);
 void imp_launch_assemble(const ImpCase& c, cudaStream_t s);
 void imp_launch_post(const ImpCase& c, cudaStream_t s);   // smoothing, update + limits, remediation, count
 void imp_launch_gmres_cycle(const ImpCase& c, bool first, cudaStream_t s);
+int imp_red_blocks(int nc);
 void imp_launch_permute_blocks(const ImpCase& c, double* dst, int which, cudaStream_t s);
 
 class ImplicitSolver {

@@ -100,28 +100,6 @@ IP_FN double mul_core(double a, double b) {
     return round_pack2(qh, ql, rm | (ql & 1u), low, E);
 }
 
-// a + b for operands in range whose exponents differ by less than 32; ok: the sum was formed
-// (it was not when 32 or more leading bits cancelled)
-IP_FN double add_core(double a, double b, bool& ok) {
-    const u32 xa = hi(a) & 0x7fffffffu, xb = hi(b) & 0x7fffffffu, al = lo(a), bl = lo(b);
-    const bool sw = xa < xb || (xa == xb && al < bl);
-    const u32 ph = sw ? xb : xa, pl = sw ? bl : al, qh0 = sw ? xa : xb, ql0 = sw ? al : bl;
-    const u32 sgn = (sw ? hi(b) : hi(a)) & 0x80000000u;
-    const u32 e = ph >> 20, d = e - (qh0 >> 20);
-    const u32 mh = (ph & 0xfffffu) | 0x100000u, sh0 = (qh0 & 0xfffffu) | 0x100000u;
-    const u32 Mh = shl2(pl, mh, 10), Ml = pl << 10, sh1 = shl2(ql0, sh0, 10), sl1 = ql0 << 10;
-    const u32 rh = sh1 >> (d & 31u), ext = shr2(0u, sl1, d);
-    const u32 rl = shr2(sl1, sh1, d) | (ext < 1u ? ext : 1u);
-    const u32 neg = (u32)((int)(hi(a) ^ hi(b)) >> 31);
-    const u64 S = (((u64)Mh << 32) | Ml) + (((u64)(rh ^ neg) << 32) | (rl ^ neg)) + (neg & 1u);
-    const u32 Sh = (u32)(S >> 32), Sl = (u32)S;
-    ok = d < 32u && Sh != 0;
-    const u32 z = (u32)clz32(Sh) & 31u;
-    const u32 Nh = shl2(Sl, Sh, z), Nl = Sl << z;
-    const u32 ql = shr2(Nl, Nh, 11), qh = Nh >> 11;
-    return round_pack(qh, ql, (Nl << 21) | (ql & 1u), ((e - z) << 20) + sgn);
-}
-
 // ---- any operands: what the branches above leave to
 
 #if defined(__CUDA_ARCH__)
@@ -143,32 +121,12 @@ IP_FN double mul_any(double a, double b) {
     if (zero_product(a, b)) return make((hi(a) ^ hi(b)) & 0x80000000u, 0u);
     return mul_rare(a, b);
 }
-IP_RARE double add_rare(double a, double b) {
-    const u32 xa = hi(a) & 0x7fffffffu, xb = hi(b) & 0x7fffffffu;
-    if ((xb | lo(b)) == 0 && xa - 1u < 0x7fefffffu) return a;  // a finite and not zero: a + 0
-    if ((xa | lo(a)) == 0 && xb - 1u < 0x7fefffffu) return b;
-    if (in_range(a) && in_range(b)) {
-        if (xa == xb && lo(a) == lo(b) && ((hi(a) ^ hi(b)) >> 31)) return make(0u, 0u);
-        const u32 ea = xa >> 20, eb = xb >> 20;
-        if (ea >= eb + 55u) return a;  // below a quarter of the last place
-        if (eb >= ea + 55u) return b;
-    }
-    return a + b;
-}
-
-// a b and a + b for any operands
+// a b for any operands
 IP_FN double mul(double a, double b) {
     if (__builtin_expect(in_range(a) && in_range(b), 1)) return mul_core(a, b);
     return mul_any(a, b);
 }
-IP_FN double add(double a, double b) {
-    bool ok;
-    const double s = add_core(a, b, ok);
-    if (__builtin_expect(ok && in_range(a) && in_range(b), 1)) return s;
-    return add_rare(a, b);
-}
 IP_FN double neg(double x) { return make(hi(x) ^ 0x80000000u, lo(x)); }
-IP_FN double sub(double a, double b) { return add(a, neg(b)); }
 
 // N products behind one branch: the compiler interleaves them
 template <int N>

@@ -1,5 +1,5 @@
 """The integer-pipe FP64 arithmetic (csrc/intpipe.cuh) compiled for the host: correctly rounded
-products, sums, reciprocals, quotients and square roots must equal the IEEE operations bit for
+products, reciprocals, quotients and square roots must equal the IEEE operations bit for
 bit on random, nearly equal and special operands, whatever the reciprocal seeds' last bits are;
 x^a lies within 0.55 units in the last place of long double's."""
 import os
@@ -36,11 +36,11 @@ int main(int argc, char** argv) {
     for (long i = 0; i < n; i++) {
         const unsigned m = (unsigned)(g() % 100000);
         double a = rnd(m), b = rnd(m / 7);
-        if (i % 4 == 1) b = dbl((bits(a) ^ (g() << 63)) + g() % 5 - 2);  // sums that cancel
+        if (i % 4 == 1) b = dbl((bits(a) ^ (g() << 63)) + g() % 5 - 2);  // nearly equal
         if (i % 8 == 3) a = rnd(0) * b;                                   // quotients near a double
         ip::seed_ulps() = (int)(g() % 5) - 2;
         const double x = i % 5 == 0 ? b * b : i % 5 == 1 ? dbl(bits(b * b) + g() % 3 - 1) : a;  // roots near a double
-        const bool ok = same(ip::mul(a, b), a * b) && same(ip::add(a, b), a + b) && same(ip::sub(a, b), a - b) &&
+        const bool ok = same(ip::mul(a, b), a * b) && ip::less(a, b) == (a < b) && ip::not_negative(a) == (a >= 0) && ip::positive(a) == (a > 0) &&
                         same(ip::rcp(b), 1.0 / b) && same(ip::quot(a, b), a / b) && same(ip::sqrt(x), std::sqrt(x)) &&
                         same(ip::half(a), 0.5 * a) && same(ip::plus_zero(a), 0.0 + a);
         if (!ok && bad++ < 5) printf("%a %a %a\n", a, b, x);
