@@ -46,6 +46,9 @@ __device__ __forceinline__ xd half(xd x) { return xd(ip::half(x.v)); }
 template <typename T> struct ArithOf { typedef T type; };
 template <> struct ArithOf<double> { typedef xd type; };
 template <typename T> using Arith = typename ArithOf<T>::type;
+// product of the state update by a constant: xd's, or one multiply-add of three registers
+__device__ __forceinline__ xd w_mul(xd k, xd x) { return k * x; }
+__device__ __forceinline__ double w_mul(double k, double x) { return __fma_rn(ip::reg(k), x, ip::reg(-0.0)); }
 // the FP64 type of a form's state update
 template <typename T> struct WideArith { typedef double type; };
 template <> struct WideArith<double> { typedef xd type; };
@@ -132,6 +135,17 @@ __device__ __forceinline__ void st8x(double* __restrict__ p, int i, const xd* v)
 // geometry, face lists) is loaded with the evict-first hint, so the L2 keeps the cell
 // records the neighbour gathers hit.
 template <typename T> __device__ __forceinline__ T ldcs(const T* p) { return __ldcs(p); }
+
+// What a kernel streams through once (geometry, face lists, state) is fetched into L2 some items
+// ahead of its use: about half of what the chip has in flight at one item per thread. Threads
+// start in the order of their items, and their first loads then hit L2 instead of waiting for
+// DRAM, ahead of the gathers that depend on them.
+constexpr int kAhead = 76800;
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+// line `line` of the items from `item` on
+__device__ __forceinline__ void prefetch_lines(const void* base, size_t item, int bytes, int line) {
+    prefetch_l2(static_cast<const char*>(base) + item * bytes + 128 * line);
+}
 
 template <typename T>
 __device__ __forceinline__ Prim<T> load_prim(const T* __restrict__ W, int i) {
@@ -1384,8 +1398,8 @@ __device__ __forceinline__ void update_finish(const DevCase& c, int i, const dou
             // 3/4 U^n + 1/4 X and 1/3 U^n + 2/3 X (the Euler and Heun stages stay unfused: the
             // reference's U += cTau/S R)
             u[k] = t_fma(cf, r, x);
-            if (STAGE == 1) u[k] = t_fma(D(ip::reg(0.25)), u[k], D(0.75) * D(c.A[k * nc + i]));
-            else if (STAGE == 2) u[k] = t_fma(D(ip::reg(2.0 / 3.0)), u[k], D(1.0 / 3.0) * D(c.A[k * nc + i]));
+            if (STAGE == 1) u[k] = t_fma(D(ip::reg(0.25)), u[k], w_mul(D(0.75), D(c.A[k * nc + i])));
+            else if (STAGE == 2) u[k] = t_fma(D(ip::reg(2.0 / 3.0)), u[k], w_mul(D(1.0 / 3.0), D(c.A[k * nc + i])));
         } else {
             u[k] = x + cf * r;
             if (SCHEME == TIME_HEUN && STAGE == 1) u[k] = half(D(c.A[k * nc + i]) + u[k]);
@@ -1412,6 +1426,16 @@ __device__ __forceinline__ void update_finish(const DevCase& c, int i, const dou
 // SCHEME/STAGE: Euler (0), Heun (0,1; src/methods/fvm_tvd.cpp:366-447), SSP-RK3 Shu-Osher (0,1,2).
 template <typename T, int SCHEME, int STAGE>
 __device__ __forceinline__ void update_one(const DevCase& c, int i) {
+    const int a = (i & ~31) + kAhead / 2;
+    if (a + 32 <= c.nc) {  // the warp's next 32 cells that far ahead, a line per lane
+        const int lane = threadIdx.x & 31;
+        const size_t nc = c.nc;
+        if (lane < 8) prefetch_lines(c.A + (lane >> 1) * nc, a, 8, lane & 1);
+        else if (lane < 16) { if (STAGE > 0) prefetch_lines(c.B + ((lane - 8) >> 1) * nc, a, 8, lane & 1); }
+        else if (lane < 19) prefetch_lines(c.face + (lane - 16) * nc, a, 4, 0);
+        else if (lane < 21) prefetch_lines(c.cfl, a, 8, lane - 19);
+        else if (lane == 21) prefetch_lines(c.flags, a, 4, 0);
+    }
     if (!update_begin<SCHEME, STAGE>(c, i)) return;
     double R[4];
     gather_residual<T>(c, i, R);
@@ -1557,6 +1581,15 @@ __global__ void __launch_bounds__(256, 4) k_flux_grad(const DevCase c) {
     if (e >= c.ne) return;
     const float* __restrict__ W = c.W32;
     const int c1 = ldcs(c.ec1 + e);
+    if (e + kAhead < c.ne) {  // the cell of an edge that far ahead lies about two thirds as far
+        const int ea = e + kAhead, ca = c1 + kAhead / 3 * 2;
+        prefetch_l2(c.geo32 + 3 * (size_t)ea);
+        if (ca < c.nc) prefetch_l2(c.cfrec32 + 3 * (size_t)ca);
+        if ((threadIdx.x & 31) == 0) {
+            prefetch_l2(c.ec1 + ea);
+            prefetch_l2(c.ec2 + ea);
+        }
+    }
     const bool inner = e < c.n_int;
     const Prim<float> qL = load_prim(W, c1);
     float gL[8], gR[8];
