@@ -507,7 +507,7 @@ RkdgSolver::RkdgSolver(const TaskConfig& t, DgMesh&& mesh) : task_(t), mesh_(std
         c.res = dalloc<unsigned long long>(4);
         c.err = dalloc<unsigned>(1);
         stage_ = dalloc<double>(12 * (size_t)nc);
-        CUDA_CHECK(cudaMallocHost(&host_bits_, 5 * sizeof(unsigned long long)));
+        CUDA_CHECK(cudaMallocHost(&host_bits_, 6 * sizeof(unsigned long long)));
         CUDA_CHECK(cudaMemsetAsync(c.err, 0, sizeof(unsigned), stream_));
         CUDA_CHECK(cudaMemsetAsync(c.res, 0, 4 * sizeof(unsigned long long), stream_));
         CUDA_CHECK(cudaMemsetAsync(c.E2, 0, 12 * (size_t)ne * sizeof(double), stream_));
@@ -605,10 +605,11 @@ void RkdgSolver::one_step(bool with_res) {
 }
 
 int RkdgSolver::read_status() {
-    unsigned e = 0;
-    CUDA_CHECK(cudaMemcpyAsync(&e, c_.err, sizeof e, cudaMemcpyDeviceToHost, stream_));
-    CUDA_CHECK(cudaMemsetAsync(c_.err, 0, sizeof(unsigned), stream_));
+    unsigned* e_host = reinterpret_cast<unsigned*>(host_bits_ + 5);
+    CUDA_CHECK(cudaMemcpyAsync(e_host, c_.err, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_));
     CUDA_CHECK(cudaStreamSynchronize(stream_));
+    const unsigned e = *e_host;
+    if (e) CUDA_CHECK(cudaMemsetAsync(c_.err, 0, sizeof(unsigned), stream_));
     if (e & ERRBIT_NONPHYSICAL) return CFD2D_ERR_NONPHYSICAL;
     if (e & ERRBIT_NEWTON_CAP) return CFD2D_ERR_NEWTON_CAP;
     return CFD2D_OK;

@@ -176,7 +176,7 @@ private:
     std::vector<void*> allocs_;
     size_t bytes_ = 0;
     double* stage_ = nullptr;               // 12*nc staging for permutations
-    unsigned long long* host_bits_ = nullptr;  // pinned: tmin, res[4]
+    unsigned long long* host_bits_ = nullptr;  // pinned: tmin, res[4], the error word
     double t_ = 0, tau_ = 0;
     int steps_ = 0;
     bool res_valid_ = false;

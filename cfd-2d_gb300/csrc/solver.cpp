@@ -211,6 +211,8 @@ Solver::Solver(const TaskConfig& t, Topo&& topo, const std::vector<int>& cell_re
         stage_ = dalloc<double>(4 * (size_t)nc);
         dtmin_ = dalloc<unsigned long long>(1);
         partial_ = dalloc<double>(4 * kConservationBlocks);
+        CUDA_CHECK(cudaMallocHost(&status_host_, sizeof(unsigned)));
+        CUDA_CHECK(cudaEventCreateWithFlags(&copied_, cudaEventDisableTiming));
         CUDA_CHECK(cudaMemsetAsync(c.flags, 0, sizeof(unsigned) * nc, stream_));
         CUDA_CHECK(cudaMemsetAsync(c.n_lim, 0, sizeof(int), stream_));
         CUDA_CHECK(cudaMemsetAsync(c.err, 0, sizeof(unsigned), stream_));
@@ -234,6 +236,11 @@ Solver::Solver(const TaskConfig& t, Topo&& topo, const std::vector<int>& cell_re
     } catch (...) {
         for (void* p : allocs_) cudaFree(p);
         allocs_.clear();
+        if (gexec_) cudaGraphExecDestroy(gexec_);
+        if (gexec_many_) cudaGraphExecDestroy(gexec_many_);
+        if (graph_) cudaGraphDestroy(graph_);
+        if (status_host_) cudaFreeHost(status_host_);
+        if (copied_) cudaEventDestroy(copied_);
         if (stream_) cudaStreamDestroy(stream_);
         stream_ = nullptr;
         throw;
@@ -265,8 +272,11 @@ Solver::~Solver() {
     }
     drop_record_graphs();
     if (gexec_) cudaGraphExecDestroy(gexec_);
+    if (gexec_many_) cudaGraphExecDestroy(gexec_many_);
     if (graph_) cudaGraphDestroy(graph_);
     if (stream_) cudaStreamSynchronize(stream_);
+    if (status_host_) cudaFreeHost(status_host_);
+    if (copied_) cudaEventDestroy(copied_);
     for (void* p : allocs_) cudaFree(p);
     if (stream_) cudaStreamDestroy(stream_);
 }
@@ -372,9 +382,9 @@ double Solver::timed_steps(int n) {
     CUDA_CHECK(cudaEventRecord(a, stream_));
     for (int k = 0; k < n; k++) {
         if (!task_.steady) t_ += tau_;
-        CUDA_CHECK(cudaGraphLaunch(gexec_, stream_));
         steps_++;
     }
+    launch_steps(n);
     CUDA_CHECK(cudaEventRecord(b, stream_));
     CUDA_CHECK(cudaEventSynchronize(b));
     float ms = 0;
@@ -407,24 +417,37 @@ void Solver::profile_steps(int n, double ms[4], int launches[4]) {
 }
 
 void Solver::build_graph() {
-    CUDA_CHECK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    try {
-        enqueue_step();
-    } catch (...) {
-        cudaGraph_t g;
-        cudaStreamEndCapture(stream_, &g);
-        if (g) cudaGraphDestroy(g);
-        throw;
-    }
-    CUDA_CHECK(cudaStreamEndCapture(stream_, &graph_));
+    auto capture = [&](int steps) {
+        cudaGraph_t g = nullptr;
+        CUDA_CHECK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+        try {
+            for (int k = 0; k < steps; k++) enqueue_step();
+        } catch (...) {
+            cudaStreamEndCapture(stream_, &g);
+            if (g) cudaGraphDestroy(g);
+            throw;
+        }
+        CUDA_CHECK(cudaStreamEndCapture(stream_, &g));
+        return g;
+    };
+    graph_ = capture(1);
     CUDA_CHECK(cudaGraphInstantiate(&gexec_, graph_, 0));
+    cudaGraph_t many = capture(kGraphSteps);
+    const cudaError_t e = cudaGraphInstantiate(&gexec_many_, many, 0);
+    cudaGraphDestroy(many);
+    CUDA_CHECK(e);
+}
+
+void Solver::launch_steps(int n) {
+    for (; n >= kGraphSteps; n -= kGraphSteps) CUDA_CHECK(cudaGraphLaunch(gexec_many_, stream_));
+    for (; n > 0; n--) CUDA_CHECK(cudaGraphLaunch(gexec_, stream_));
 }
 
 int Solver::read_status() {
-    unsigned e = 0;
-    CUDA_CHECK(cudaMemcpyAsync(&e, dc_.err, sizeof e, cudaMemcpyDeviceToHost, stream_));
-    CUDA_CHECK(cudaMemsetAsync(dc_.err, 0, sizeof(unsigned), stream_));
+    CUDA_CHECK(cudaMemcpyAsync(status_host_, dc_.err, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_));
     CUDA_CHECK(cudaStreamSynchronize(stream_));
+    const unsigned e = *status_host_;
+    if (e) CUDA_CHECK(cudaMemsetAsync(dc_.err, 0, sizeof(unsigned), stream_));
     if (e & ERRBIT_NEWTON_CAP) return CFD2D_ERR_NEWTON_CAP;
     if (e & ERRBIT_NONPHYSICAL) return CFD2D_ERR_NONPHYSICAL;
     return CFD2D_OK;
@@ -436,9 +459,9 @@ int Solver::step(int n) {
         if (!task_.steady) t_ += tau_;  // src/methods/fvm_tvd.cpp:312-316
         if (!task_.steady)
             for (auto& in : inst_) in.t += in.tau;
-        CUDA_CHECK(cudaGraphLaunch(gexec_, stream_));
         steps_++;
     }
+    launch_steps(n);
     return read_status();
 }
 
@@ -534,12 +557,13 @@ void Solver::set_state(const double* ro, const double* ru, const double* rv, con
                                        stream_));
         launch_gather_state(dc_, stage_, dc_.A, stream_);
     }
+    CUDA_CHECK(cudaEventRecord(copied_, stream_));
     launch_prims(dc_, task_.precision, stream_);
     if (reset_tau) {
         tau_ = task_.tau;
         compute_tau();
     }
-    CUDA_CHECK(cudaStreamSynchronize(stream_));
+    CUDA_CHECK(cudaEventSynchronize(copied_));  // the primitives follow on the stream
 }
 
 void Solver::get_ctau(double* out) {

@@ -189,6 +189,13 @@ private:
     cudaStream_t stream_ = nullptr;
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t gexec_ = nullptr;
+    cudaGraphExec_t gexec_many_ = nullptr;  // kGraphSteps steps
+    // steps of one graph launch: between graphs the GPU waits 2-3 us longer than between a
+    // graph's kernels, a tenth of a step on a small mesh
+    static constexpr int kGraphSteps = 8;
+    void launch_steps(int n);               // n steps' kernels
+    unsigned* status_host_ = nullptr;       // pinned: the device error word
+    cudaEvent_t copied_ = nullptr;          // the caller's arrays have been read
     std::vector<Instance> inst_;
     void compute_tau_batch();
     void rebuild_graph();

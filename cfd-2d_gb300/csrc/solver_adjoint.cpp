@@ -181,9 +181,9 @@ double Solver::forward(int nsteps, int k, int* status) {
         }
         for (int j = 0; j < n; j++) {
             if (!task_.steady) t_ += tau_;
-            CUDA_CHECK(cudaGraphLaunch(gexec_, stream_));
             steps_++;
         }
+        launch_steps(n);
     }
     fw_steps_ = nsteps;
     fw_k_ = k;

@@ -139,8 +139,9 @@ void Solver::compute_tau_batch() {
 
 void Solver::rebuild_graph() {
     if (gexec_) cudaGraphExecDestroy(gexec_);
+    if (gexec_many_) cudaGraphExecDestroy(gexec_many_);
     if (graph_) cudaGraphDestroy(graph_);
-    gexec_ = nullptr;
+    gexec_ = gexec_many_ = nullptr;
     graph_ = nullptr;
     build_graph();
 }
