@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(256) k_adj_cell(const DevCase c, const AdjCase
         // outward normals of a closed triangle weighted by their lengths: zero, and left out.
         const A w = neg_if(half(l), side2);
         const A wx = w * nx, wy = w * ny;
-        const int j = side2 ? c.ec1[e] : c.ec2[e];
+        const int j = c.cf_nb[k * nc + i] >> 1;  // the neighbour, beside the face's load (negative: none)
         if (j >= 0) {
             T hj[8];
             ld8(h, j, hj);
