@@ -412,31 +412,53 @@ __global__ void __launch_bounds__(256) k_adj_cell(const DevCase c, const AdjCase
     SumAcc<T> qs[4];
     A Tcb = acc0<A>();
     Prim<A> qb = zero_prim<A>();  // ghost-path contributions (boundary faces only)
+    // every load before the first branch and the first store: the faces and neighbours, then
+    // their geometry, gradient adjoints and the cell's own state (one after another they took
+    // two thirds of the FP32 form's time on a small mesh; with FP64 faces the neighbours'
+    // gradient adjoints stay in the loop, 48 registers less)
+    constexpr bool AHEAD = sizeof(T) == 4;
+    int fc[3], nb[3];
+    T ge[3][3], hv[AHEAD ? 3 : 1][8];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const int f = c.face[k * nc + i];
-        const int e = f >> 1;
-        const bool side2 = f & 1;
-        const A nx(NX_of<T>(c)[e]), ny(NY_of<T>(c)[e]), l(L_of<T>(c)[e]);
+        fc[k] = c.face[k * nc + i];
+        nb[k] = c.cf_nb[k * nc + i];
+    }
+    double q0[4], tb[4], ac[4];
+    ld4(a.qbar, i, q0);  // r, u, v, p
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        tb[k] = a.tb[k * nc + i];
+        ac[k] = a.acc[k * nc + i];
+    }
+    const double cfl = c.cfl[i];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int e = fc[k] >> 1;
+        ge[k][0] = NX_of<T>(c)[e]; ge[k][1] = NY_of<T>(c)[e]; ge[k][2] = L_of<T>(c)[e];
+        if (AHEAD) ld8(h, nb[k] >= 0 ? nb[k] >> 1 : i, hv[AHEAD ? k : 0]);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int e = fc[k] >> 1;
+        const bool side2 = fc[k] & 1;
+        const A nx(ge[k][0]), ny(ge[k][1]), l(ge[k][2]);
         // d g_i / d (neighbour or ghost value) = +-(l/2) n / S_i with n outward from c1; the
         // neighbour's gradient takes q_i with the opposite sign and its own 1/S_j. The own
         // value's direct terms, (1/S_i) sum_k (l_k/2) n_out,k over the three faces, are the
         // outward normals of a closed triangle weighted by their lengths: zero, and left out.
         const A w = neg_if(half(l), side2);
         const A wx = w * nx, wy = w * ny;
-        const int j = c.cf_nb[k * nc + i] >> 1;  // the neighbour, beside the face's load (negative: none)
-        if (j >= 0) {
-            T hj[8];
-            ld8(h, j, hj);
-            qs[0].add(-madd(wx * A(hj[0]), wy, A(hj[1])));
-            qs[3].add(-madd(wx * A(hj[2]), wy, A(hj[3])));
-            qs[1].add(-madd(wx * A(hj[4]), wy, A(hj[5])));
-            qs[2].add(-madd(wx * A(hj[6]), wy, A(hj[7])));
+        if (!AHEAD) ld8(h, nb[k] >= 0 ? nb[k] >> 1 : i, hv[0]);
+        const T* hj = hv[AHEAD ? k : 0];
+        const A s0 = madd(wx * A(hj[0]), wy, A(hj[1])), s1 = madd(wx * A(hj[2]), wy, A(hj[3]));
+        const A s2 = madd(wx * A(hj[4]), wy, A(hj[5])), s3 = madd(wx * A(hj[6]), wy, A(hj[7]));
+        if (nb[k] >= 0) {
+            qs[0].add(-s0);
+            qs[3].add(-s1);
+            qs[1].add(-s2);
+            qs[2].add(-s3);
         } else {  // boundary face: the ghost of the unreconstructed centre state
-            T hi[8];
-            ld8(h, i, hi);
-            const A s0 = madd(wx * A(hi[0]), wy, A(hi[1])), s1 = madd(wx * A(hi[2]), wy, A(hi[3]));
-            const A s2 = madd(wx * A(hi[4]), wy, A(hi[5])), s3 = madd(wx * A(hi[6]), wy, A(hi[7]));
             const DevBnd b = c.bnds[c.ebnd[e]];
             const A Tc = temperature(q, mt.gm1, mt.Cv);
             Prim<A> ob;
@@ -449,8 +471,6 @@ __global__ void __launch_bounds__(256) k_adj_cell(const DevCase c, const AdjCase
     }
     if (to_wide(Tcb) != 0.0) vjp_temperature(q, mt.gm1, mt.Cv, Tcb, qb);
     {
-        double q0[4];
-        ld4(a.qbar, i, q0);  // r, u, v, p
         qs[0].add(qb.r); qs[1].add(qb.u); qs[2].add(qb.v); qs[3].add(qb.p);
         qb.r = to_face<A>(to_wide(D(q0[0]) + D(qs[0].value())));
         qb.u = to_face<A>(to_wide(D(q0[1]) + D(qs[1].value())));
@@ -460,20 +480,20 @@ __global__ void __launch_bounds__(256) k_adj_cell(const DevCase c, const AdjCase
     A V[4] = {acc0<A>(), acc0<A>(), acc0<A>(), acc0<A>()};
     vjp_cons2prim_q(q, mt.gm1, qb, V);
     D ux[4];
-    for (int k = 0; k < 4; k++) ux[k] = D(a.tb[k * nc + i]) + D(to_wide(V[k]));
-    const D cf(c.cfl[i]), ct(coef_t), ca(coef_acc);
+    for (int k = 0; k < 4; k++) ux[k] = D(tb[k]) + D(to_wide(V[k]));
+    const D cf(cfl), ct(coef_t), ca(coef_acc);
     double mu[4];
     for (int k = 0; k < 4; k++) {
         const size_t q4 = (size_t)k * nc + i;
         D t;
         if (first) {  // lambda of the step input, and (coef_t, coef_acc = the last stage's) the next step's start
-            const D l = D(a.acc[q4]) + ux[k];
+            const D l = D(ac[k]) + ux[k];
             a.lam[q4] = to_wide(l);
             t = ct * l;
             a.acc[q4] = to_wide(ca * l);
         } else {
             t = ct * ux[k];
-            a.acc[q4] = to_wide(D(a.acc[q4]) + ca * ux[k]);
+            a.acc[q4] = to_wide(D(ac[k]) + ca * ux[k]);
         }
         a.tb[q4] = to_wide(t);
         mu[k] = to_wide(cf * t);

@@ -829,20 +829,22 @@ __device__ __forceinline__ void grad_one_w(const DevCase& c, int i) {
     const int nc = c.nc;
     const float* __restrict__ W = c.W32;
     const Prim<float> q = load_prim(W, i);
-    float g[8];
+    float g[8], ax[3], ay[3];
+    int nb[3];
+    Prim<float> o[3];  // every load before the first branch
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const int nb = ldcs(c.cf_nb + k * nc + i);
-        const float ax = ldcs(c.cf_ax32 + k * nc + i), ay = ldcs(c.cf_ay32 + k * nc + i);
-        const bool side2 = nb >= 0 && (nb & 1);
-        Prim<float> o;
-        if (nb >= 0) {
-            o = load_prim(W, nb >> 1);
-        } else {
-            const int e = -(nb + 1);
-            o = grad_ghost(c, i, e, q, c.nx32[e], c.ny32[e]);
-        }
-        grad_face_w(g, q, o, ax, ay, side2, k == 0);
+        nb[k] = ldcs(c.cf_nb + k * nc + i);
+        ax[k] = ldcs(c.cf_ax32 + k * nc + i);
+        ay[k] = ldcs(c.cf_ay32 + k * nc + i);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) o[k] = load_prim(W, nb[k] >= 0 ? nb[k] >> 1 : i);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int e = -(nb[k] + 1);
+        if (nb[k] < 0) o[k] = grad_ghost(c, i, e, q, c.nx32[e], c.ny32[e]);
+        grad_face_w(g, q, o[k], ax[k], ay[k], nb[k] >= 0 && (nb[k] & 1), k == 0);
     }
     grad_finish_w(c, i, g);
     st8(c.G32, i, g);
@@ -1554,19 +1556,22 @@ __global__ void __launch_bounds__(256, 5) k_stage_fused(const DevCase c, const D
 __device__ __forceinline__ void grad_of_cell(const DevCase& c, int i, const Prim<float>& q, float* g) {
     const float4* __restrict__ rec = c.cfrec32 + 3 * (size_t)i;
     const float* __restrict__ W = c.W32;
+    // the three records, then the three neighbours, without a branch between the loads (across a
+    // boundary face the cell itself is read, and replaced by the ghost below)
+    float4 r[3];
+    Prim<float> o[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) r[k] = __ldg(rec + k);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const float4 r = __ldg(rec + k);
-        const int nb = __float_as_int(r.x);
-        const bool side2 = nb >= 0 && (nb & 1);
-        Prim<float> o;
-        if (nb >= 0) {
-            o = load_prim(W, nb >> 1);
-        } else {
-            const int e = -(nb + 1);
-            o = grad_ghost(c, i, e, q, c.nx32[e], c.ny32[e]);
-        }
-        grad_face_w(g, q, o, r.y, r.z, side2, k == 0);
+        const int nb = __float_as_int(r[k].x);
+        o[k] = load_prim(W, nb >= 0 ? nb >> 1 : i);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int nb = __float_as_int(r[k].x);
+        if (nb < 0) o[k] = grad_ghost(c, i, -(nb + 1), q, c.nx32[-(nb + 1)], c.ny32[-(nb + 1)]);
+        grad_face_w(g, q, o[k], r[k].y, r[k].z, nb >= 0 && (nb & 1), k == 0);
     }
     grad_finish_w(c, i, g);
 }
