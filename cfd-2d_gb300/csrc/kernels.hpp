@@ -67,10 +67,6 @@ __host__ __device__ __forceinline__ RimGas<T> rim_gas(T GAM) {
     g.eAGAM = T(1) / g.AGAM;
     return g;
 }
-// Launch shape of one kernel kind: threads per block and blocks (0 = one
-// thread per item; otherwise a persistent grid that strides over the items).
-// Default: 64-thread blocks, one thread per item (measured best for the single
-// four-quadrant workload in both precisions; the autotuner can override it).
 // What a forward HLLC flux evaluation leaves for the adjoint's recorded path, per edge (SoA,
 // face precision): v[(10 g + j) ne + e] for Gauss point g, j 0-3 the left face state (r, u,
 // v, p), 4-7 the right one, 8-9 the left and right sound speeds; bits[e] minmod's branches
@@ -80,6 +76,9 @@ struct FluxRec {
     unsigned* bits = nullptr;
 };
 
+// Launch shape of one kernel kind: threads per block and blocks (0 = one
+// thread per item; otherwise a persistent grid that strides over the items).
+// Default: 64-thread blocks, one thread per item; the autotuner can override it.
 struct LaunchShape { int block = 64, grid = 0; };
 enum { KIND_GRAD = 0, KIND_FLUX = 1, KIND_UPDATE = 2, N_TUNED_KINDS = 3 };
 

@@ -191,6 +191,15 @@ Solver::Solver(const TaskConfig& t, Topo&& topo, const std::vector<int>& cell_re
         c.newton_cap = task_.newton_cap;
         c.flux_pipe = mixed && task_.flux_pipe != 0 ? 1 : 0;
         if (c.flux_pipe) launch_flux_prepare_mixed();
+        // FP64 face kernels are long (the flux up to 100 KB of code): warps of one block run
+        // through it together and share the instruction cache, so large blocks are faster once
+        // they fill the chip three times (flux, 152 SMs x 3 blocks of 256 lanes: 7% at 130k
+        // triangles, 1.8% at 2.1M); on a smaller mesh (1.7 fillings: 1.5% slower) their last,
+        // partly filled round costs more than that
+        if (!mixed && task_.recon != RECON_NONE) {
+            if (2ll * ne >= 3 * 152 * 3 * 256) c.shape[KIND_FLUX].block = 256;
+            if (nc >= 152 * 4 * 256) c.shape[KIND_GRAD].block = 128;
+        }
         c.A = dalloc<double>(4 * (size_t)nc);
         c.B = dalloc<double>(4 * (size_t)nc);
         c.cfl = dalloc<double>(nc);
