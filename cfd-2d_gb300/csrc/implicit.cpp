@@ -82,9 +82,6 @@ ImplicitSolver::ImplicitSolver(const TaskConfig& t, Topo&& topo, const std::vect
         c.l = upload(lay_.l);
         c.dl = upload(lay_.dl);
         c.S = upload(lay_.S);
-        std::vector<double> is(nc);
-        for (int i = 0; i < nc; i++) is[i] = 1.0 / lay_.S[i];
-        c.invS = upload(is);
         {  // the matrix-vector product's neighbours; a boundary face's block is zero, so it reads the cell itself
             std::vector<int> nb(3 * (size_t)nc);
             for (int k = 0; k < 3; k++)

@@ -9,8 +9,8 @@
 //
 // Layout in HBM (storage = RCM cell order, faces of a cell in ascending original edge
 // order as Cell::edgesInd lists them): diagonal blocks D[column][nc][row] and face
-// blocks O[face][column][nc][row] (the matrix-vector product runs four threads per
-// cell, one per row, and every load of a block column is one contiguous run across a
+// blocks O[face][column][nc][row] (the assembly runs four lanes per
+// cell, one per row, and every access to a block column is one contiguous run across a
 // warp), right-hand side and every Krylov vector as [nc][4] (x[4c + k], the
 // reference's numbering of unknowns).
 #pragma once
@@ -83,7 +83,6 @@ struct ImpCase {
     const double* l;
     const double* dl;         // 8*ne Gauss-point offsets (gp0: dxL dyL dxR dyR, gp1: ...)
     const double* S;          // nc
-    const double* invS;       // nc, RN(1/S)
     const int* nbr;           // 3*nc the cell across each face (storage), or the cell itself on the boundary
     const int* iperm;         // original -> storage
     const uint8_t* cmat;      // nc or nullptr

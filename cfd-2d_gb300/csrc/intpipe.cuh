@@ -8,8 +8,13 @@
 // the very bits of the FP64 instruction or of the IEEE quotient and square root, so a kernel may
 // form any of its operations on either side.
 //
-// Measured on one SM with all warps resident (clocks per warp operation): product 16.9 native,
-// 13.8 here; with both kinds in flight 8.9 per product.
+// Measured on one SM with all warps resident (clocks per warp operation): product or sum 20
+// native (17 as a multiply-add of three registers; an operand from the constant bank or an
+// immediate costs the 20), product 10.9 here, 8.3 per product with two native to three here;
+// reciprocal 24 (90 native), quotient 34 (144), square root 34 (170). A sum formed here takes
+// 22.6 and lost in every kernel it was tried in (two steps at 2.1M triangles 6.48 -> 7.17 ms),
+// so sums stay native. Kernels: k_flux at 2.1M triangles 1.42 -> 0.7 ms, with a lane per Gauss
+// point; the same arithmetic in one thread per edge gained nothing (200-255 registers).
 //
 // The common path takes operands with 2^-510 <= |x| < 2^510, whose products and quotients
 // stay normal; zeros, and anything else, leave it by a branch.
@@ -34,7 +39,6 @@ __device__ __forceinline__ double make(u32 h, u32 l) { return __hiloint2double((
 // low word of (h:l) >> s, 0 <= s < 32
 __device__ __forceinline__ u32 shr2(u32 l, u32 h, u32 s) { return __funnelshift_r(l, h, s); }
 __device__ __forceinline__ u32 shl2(u32 l, u32 h, u32 s) { return __funnelshift_l(l, h, s); }
-__device__ __forceinline__ int clz32(u32 x) { return __clz((int)x); }
 // approximations of 1/x and 1/sqrt(x), within a few units of the 23rd fraction bit
 __device__ __forceinline__ float rcp_seed(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float rsqrt_seed(float x) { float y; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
@@ -64,7 +68,6 @@ inline u32 lo(double x) { return (u32)bits(x); }
 inline double make(u32 h, u32 l) { const u64 b = ((u64)h << 32) | l; double x; std::memcpy(&x, &b, 8); return x; }
 inline u32 shr2(u32 l, u32 h, u32 s) { return (u32)((((u64)h << 32) | l) >> (s & 31)); }
 inline u32 shl2(u32 l, u32 h, u32 s) { return (u32)(((((u64)h << 32) | l) << (s & 31)) >> 32); }
-inline int clz32(u32 x) { return x ? __builtin_clz(x) : 32; }
 inline u32 f2u(float x) { return (u32)x; }
 inline float u2f_bits(u32 b) { float x; std::memcpy(&x, &b, 4); return x; }
 // off by seed_ulps units in the last place: the results must not depend on the seed

@@ -159,7 +159,7 @@ __global__ void k_selftest(int which, long long n, unsigned long long seed, unsi
     unsigned long long local = 0;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
         const unsigned long long r1 = mix64(seed ^ (2 * k)), r2 = mix64(seed ^ (2 * k + 1));
-        if (which == 0) {  // quotients of random doubles over a wide exponent range, by the reciprocal form
+        if (which == 0) {  // operations on random doubles over a wide exponent range, on the integer pipes
             const double a = __longlong_as_double((long long)(((r1 % 1400) + 324ull) << 52 | (r2 & 0xfffffffffffffull) |
                                                               (r1 & 0x8000000000000000ull)));
             const double b = __longlong_as_double((long long)((((r2 >> 52) % 1400) + 324ull) << 52 |
@@ -167,10 +167,7 @@ __global__ void k_selftest(int which, long long n, unsigned long long seed, unsi
             double a2 = a, b2 = b;
             if ((r1 & 0xf0) == 0) a2 = (r1 & 0x100) ? -0.0 : 0.0;      // zero dividends, both signs
             if ((r2 & 0xf00) == 0) b2 = __longlong_as_double((long long)(r2 & 0xfff0000000000000ull));  // any exponent
-            const double y = 1.0 / b2;
-            const double q1 = div_rn(a2, b2, y), q2 = a2 / b2;
-            local += __double_as_longlong(q1) != __double_as_longlong(q2);
-            // the integer-pipe operations; c: near a in magnitude, for sums that cancel
+            // c: near a in magnitude, for sums that cancel
             const unsigned long long r3 = mix64(r2);
             const unsigned ea = (unsigned)(((unsigned long long)__double_as_longlong(a2) >> 52) & 0x7ff);
             double c = __longlong_as_double((long long)(((r3 & 1) << 63) | (unsigned long long)((ea + (r3 >> 1) % 70 - 35) & 0x7ff) << 52 |

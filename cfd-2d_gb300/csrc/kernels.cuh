@@ -187,31 +187,6 @@ template <> __device__ __forceinline__ double ig1_of<double>(const DevCase& c) {
 template <> __device__ __forceinline__ xd ig1_of<xd>(const DevCase& c) { return xd(ip::reg(c.ig1_flux)); }
 template <> __device__ __forceinline__ float ig1_of<float>(const DevCase& c) { return c.ig1_flux_f; }
 
-// a / b correctly rounded from y = RN(1/b): q = RN(a y), r = a - b q exactly
-// (one FMA), result RN(q + r y) (Markstein, "IA-64 and Elementary Functions",
-// 2000, the division theorem). Three FP64 instructions instead of a full
-// division; the exponent guard keeps a, y and the quotient far from underflow
-// and overflow, where the theorem needs no extra conditions. A zero dividend
-// over a finite y (b nonzero, not NaN) gives the zero with the sign of a XOR b,
-// built on the integer pipe (zero gradients and velocities are common). Other
-// operands (subnormal, huge, inf, NaN, b zero) divide outright.
-// The outright division sits in a function of its own so that the compiler
-// branches to it instead of evaluating it beside the common path.
-static __device__ __noinline__ double div_outright(double a, double b) { return a / b; }
-__device__ __forceinline__ double div_rn(double a, double b, double y) {
-    const long long ia = __double_as_longlong(a), iy = __double_as_longlong(y);
-    const int ea = (int)((ia >> 52) & 0x7ff);
-    const int ey = (int)((iy >> 52) & 0x7ff);
-    const int eq = ea + ey - 1023;
-    if (__builtin_expect(ea > 0x100 && ea < 0x700 && ey > 0x100 && ey < 0x700 && eq > 0x100 && eq < 0x700, 1)) {
-        const double q = a * y;
-        const double r = fma(-q, b, a);
-        return fma(r, y, q);
-    }
-    if ((ia & 0x7fffffffffffffffll) == 0 && ey < 0x7ff)
-        return __longlong_as_double((ia ^ iy) & (long long)0x8000000000000000ull);
-    return div_outright(a, b);
-}
 // -x when s, else x: a sign-bit flip on the integer pipe (x - y is x + (-y) in IEEE).
 __device__ __forceinline__ double neg_if(double x, bool s) {
     return __hiloint2double(__double2hiint(x) ^ (s ? (int)0x80000000 : 0), __double2loint(x));
@@ -219,7 +194,6 @@ __device__ __forceinline__ double neg_if(double x, bool s) {
 __device__ __forceinline__ xd neg_if(xd x, bool s) { return xd(neg_if(x.v, s)); }
 __device__ __forceinline__ float neg_if(float x, bool s) { return __int_as_float(__float_as_int(x) ^ (s ? (int)0x80000000 : 0)); }
 // a / b given y = RN(1/b): the correctly rounded quotient in FP64, a * y in the FP32 faces.
-__device__ __forceinline__ double div_by(double a, double b, double y) { return div_rn(a, b, y); }
 __device__ __forceinline__ xd div_by(xd a, xd b, xd) { return a / b; }
 __device__ __forceinline__ float div_by(float a, float, float y) { return a * y; }
 // Quotients by a shared divisor: recip_of the divisor once, div_y per dividend (FP32 divides).

@@ -1,9 +1,9 @@
 // The explicit discontinuous Galerkin method FEM_RKDG (src/methods/fem_rkdg.cpp) on the GPU.
 //
 // P1 basis per triangle (1, (x-xc)/HX, (y-yc)/HY), cell quadrature of 3 or 4 points, edge
-// quadrature of 2 or 3 points, two Runge-Kutta stages. Per stage two kernels: one thread
-// per edge evaluates both sides' polynomials at the edge's Gauss points, the Riemann flux
-// (GODUNOV or LAX) and the two sides' surface integrals; one thread per cell evaluates the
+// quadrature of 2 or 3 points, two Runge-Kutta stages. Per stage two kernels: one lane
+// per Gauss point of an edge evaluates both sides' polynomials and the Riemann flux (GODUNOV
+// or LAX) there, and the edge's lanes share the two sides' surface integrals; one thread per cell evaluates the
 // volume integral at the cell's Gauss points, gathers its three edges' integrals in
 // ascending original edge number (the order of the reference's edge loop), multiplies by
 // the inverse mass matrix and cTau and forms the stage result. One CUDA graph per step.
@@ -34,7 +34,7 @@ enum DgRkMode { DG_RK_REFERENCE = 0, DG_RK_HEUN = 1 };
 
 // A material with the constants the method derives from it (Material::URS, getGamma).
 struct DgMat {
-    double M, Cv, gam, gm1, ig1, iCv;  // ig1 = RN(1/(gam-1)), iCv = RN(1/Cv)
+    double M, Cv, gam, gm1, ig1;  // ig1 = RN(1/(gam-1))
     RimGas<double> rg;                 // the exact Riemann solver's constants of gam
 };
 

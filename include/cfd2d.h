@@ -184,9 +184,9 @@ int cfd2d_timed_steps(cfd2d_t* h, int nsteps, double* device_ms);
 int cfd2d_profile_steps(cfd2d_t* h, int nsteps, double kernel_ms[4], int kernel_launches[4]);
 
 /* Built-in check of the device arithmetic helpers on n seeded random operands,
- * against the hardware operation on the current device: which = 0 FP64 division
- * through a precomputed reciprocal and the FP64 operations formed on the integer pipes
- * (must equal the hardware's bit for bit; x^(1/7) within 2 units in the last place of pow's), 1 FP32->FP64
+ * against the hardware operation on the current device: which = 0 the FP64
+ * operations formed on the integer pipes (product, quotient, reciprocal, root: must equal the
+ * hardware's bit for bit; x^(1/7) within 2 units in the last place of pow's), 1 FP32->FP64
  * widening on the integer pipe (must equal the conversion), 2 FP64->FP32
  * narrowing on the integer pipe (within 1 ulp), 3 FP64 minmod with its
  * integer-pipe sign test (must equal a*b > 0 ? (|a| < |b| ? a : b) : 0 bit for
