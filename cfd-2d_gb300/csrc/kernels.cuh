@@ -293,19 +293,21 @@ __device__ __forceinline__ Prim<T> ghost_state(const DevBnd& b, const Prim<T>& q
 // (0, 0x7ff0...0]). mm_first is |a| < |b| on magnitude bits, which orders non-NaN
 // values like fabs does. Bit for bit the reference's result.
 static __device__ __noinline__ double mul_outright(double a, double b) { return a * b; }
+// The magnitudes are put together from 32-bit words: a 64-bit mask of a double's bits is compiled
+// to an FP64 absolute value, an instruction of the FP64 unit (eight per reconstruction of a side).
+__device__ __forceinline__ unsigned long long mm_mag(double x) {
+    return (unsigned long long)((unsigned)__double2hiint(x) & 0x7fffffffu) << 32 | (unsigned)__double2loint(x);
+}
 __device__ __forceinline__ bool mm_pos(double a, double b) {
-    const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
-    const long long ma = ia & 0x7fffffffffffffffll, mb = ib & 0x7fffffffffffffffll;
+    const unsigned long long ma = mm_mag(a), mb = mm_mag(b);
     if (ma == 0 || mb == 0) return false;
     const int ea = (int)(ma >> 52), eb = (int)(mb >> 52);
     if (__builtin_expect(ea >= 1 && eb >= 1 && ea + eb >= 972, 1))
-        return (ia ^ ib) >= 0 && ma <= 0x7ff0000000000000ll && mb <= 0x7ff0000000000000ll;
+        return (__double2hiint(a) ^ __double2hiint(b)) >= 0 && ma <= 0x7ff0000000000000ull && mb <= 0x7ff0000000000000ull;
     const long long pb = __double_as_longlong(mul_outright(a, b));  // a branch, not a predicated multiply
     return pb > 0 && pb <= 0x7ff0000000000000ll;
 }
-__device__ __forceinline__ bool mm_first(double a, double b) {
-    return (__double_as_longlong(a) & 0x7fffffffffffffffll) < (__double_as_longlong(b) & 0x7fffffffffffffffll);
-}
+__device__ __forceinline__ bool mm_first(double a, double b) { return mm_mag(a) < mm_mag(b); }
 __device__ __forceinline__ bool mm_pos(xd a, xd b) { return mm_pos(a.v, b.v); }
 __device__ __forceinline__ bool mm_first(xd a, xd b) { return mm_first(a.v, b.v); }
 __device__ __forceinline__ bool mm_pos(float a, float b) {
