@@ -122,8 +122,8 @@ __device__ __forceinline__ void adj_flux_lane(const DevCase& c, const AdjCase& a
             const unsigned br = RECON == RECON_LINEAR ? 1u : (cd[g] >> (8 + 2 * k)) & 3u;
             const xd own = side ? rv[k] : lv[k];
             if ((side ? br : bl) == 1u) {  // the projection: into the gradient
-                gb[2 * k] = madd(gb[2 * k], own, dx);
-                gb[2 * k + 1] = madd(gb[2 * k + 1], own, dy);
+                gb[2 * k] = g == 0 ? own * dx : madd(gb[2 * k], own, dx);
+                gb[2 * k + 1] = g == 0 ? own * dy : madd(gb[2 * k + 1], own, dy);
             }
             // the left face state's share, then the right one's: a side keeps its own state's
             // adjoint unless the difference was taken (2), which passes it to the other side

@@ -310,7 +310,9 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<T>& L, const Prim<T>& R, T
 
 // FP64 faces: the VJP of the FP64 forward's arrangement (flux_hllc_c<double> in kernels.cuh:
 // S_K U_K - F_K from m_K = rho_K d_K, d_K = S_K - un_K, and only the used side's energy),
-// recomputing the forward's values and branches with its own expressions.
+// recomputing the forward's values and branches with its own expressions. A sum's first product
+// is written as one (Lb and Rb are empty on entry): on the integer pipes, where a multiply-add
+// onto the empty sum would be an FP64 product.
 __device__ __forceinline__ void vjp_hllc_c(const Prim<xd>& L, const Prim<xd>& R, xd cL, xd cR, xd nx, xd ny, xd GAM,
                                            xd IG1, const xd* fb, Prim<xd>& Lb, Prim<xd>& Rb) {
     typedef xd T;
@@ -320,9 +322,9 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<xd>& L, const Prim<xd>& R,
     const T SL = l1 ? sl1 : sl2, SR = r1 ? sr1 : sr2;
     T unLb = acc0<T>(), unRb = acc0<T>(), SLb = acc0<T>(), SRb = acc0<T>(), cLb = acc0<T>(), cRb = acc0<T>();
     // E = p IG1 + .5 r (u^2 + v^2): the adjoint Eb of one side's energy into its state
-    auto energy_bar = [&](const Prim<T>& q, T Eb, Prim<T>& qb) {
-        const T e = Eb * q.r;
-        qb.p = madd(qb.p, Eb, IG1); qb.r = madd(qb.r, half(Eb), t_fma(q.u, q.u, q.v * q.v));
+    auto energy_bar = [&](const Prim<T>& q, T Eb, Prim<T>& qb, bool first) {
+        const T e = Eb * q.r, k = t_fma(q.u, q.u, q.v * q.v);
+        qb.p = madd(qb.p, Eb, IG1); qb.r = first ? half(Eb) * k : madd(qb.r, half(Eb), k);
         qb.u = madd(qb.u, e, q.u); qb.v = madd(qb.v, e, q.v);
     };
     if (not_negative(SL) || not_negative(-SR)) {  // supersonic: the upwind side's physical flux
@@ -330,11 +332,11 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<xd>& L, const Prim<xd>& R,
         if (not_negative(SL)) {
             vjp_phys(L.r, L.u, L.v, L.p, energy(L.r, L.u, L.v, L.p, IG1), unL, nx, ny, fb, Lb.r, Lb.u, Lb.v, Lb.p,
                      Eb, unLb);
-            energy_bar(L, Eb, Lb);
+            energy_bar(L, Eb, Lb, false);
         } else {
             vjp_phys(R.r, R.u, R.v, R.p, energy(R.r, R.u, R.v, R.p, IG1), unR, nx, ny, fb, Rb.r, Rb.u, Rb.v, Rb.p,
                      Eb, unRb);
-            energy_bar(R, Eb, Rb);
+            energy_bar(R, Eb, Rb, false);
         }
     } else {
         const T dL = SL - unL, dR = SR - unR;
@@ -366,14 +368,13 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<xd>& L, const Prim<xd>& R,
         SKb = madd(SKb, spb, ps);
         const T psb = spb * SK;
         // ps = pK + mK (Ss - unK)
-        T Krb = acc0<T>(), Kub = acc0<T>(), Kvb = acc0<T>(), Kpb = psb;
+        T Kpb = psb;
         T unKb = -psb * mK;
         mKb = madd(mKb, psb, Ss - unK);
         Ssb = madd(Ssb, psb, mK);
         // A1 = mK u - p nx, A2 = mK v - p ny, A3 = EK dK - p unK
         mKb = madd(madd(mKb, A1b, K.u), A2b, K.v);
-        Kub = madd(Kub, A1b, mK);
-        Kvb = madd(Kvb, A2b, mK);
+        const T Kub = A1b * mK, Kvb = A2b * mK;
         Kpb = madd(madd(madd(Kpb, -A1b, nx), -A2b, ny), -A3b, unK);
         const T EKb = A3b * dK;
         T dKb = A3b * EK;
@@ -382,17 +383,17 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<xd>& L, const Prim<xd>& R,
         const T numb = Ssb * iden, denb = -Ssb * Ss * iden;
         Rb.p += numb; Lb.p -= numb;
         T mLb = madd(denb, numb, unL), mRb = madd(-denb, -numb, unR);
-        unLb = madd(unLb, numb, mL); unRb = madd(unRb, -numb, mR);
+        unLb = numb * mL; unRb = -numb * mR;
         T dLb = acc0<T>(), dRb = acc0<T>();
         // route the K side (its m, d, state, energy and speeds) to L or R
         if (left) {
             mLb += mKb; dLb += dKb; unLb += unKb; SLb += SKb;
-            Lb.r += Krb; Lb.u += Kub; Lb.v += Kvb; Lb.p += Kpb;
-            energy_bar(L, EKb, Lb);
+            Lb.u += Kub; Lb.v += Kvb; Lb.p += Kpb;
+            energy_bar(L, EKb, Lb, true);
         } else {
             mRb += mKb; dRb += dKb; unRb += unKb; SRb += SKb;
-            Rb.r += Krb; Rb.u += Kub; Rb.v += Kvb; Rb.p += Kpb;
-            energy_bar(R, EKb, Rb);
+            Rb.u += Kub; Rb.v += Kvb; Rb.p += Kpb;
+            energy_bar(R, EKb, Rb, true);
         }
         // mL = rL dL, dL = SL - unL (and R)
         Lb.r = madd(Lb.r, mLb, dL); dLb = madd(dLb, mLb, L.r);
@@ -407,11 +408,11 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<xd>& L, const Prim<xd>& R,
     Lb.u = madd(Lb.u, unLb, nx); Lb.v = madd(Lb.v, unLb, ny);
     Rb.u = madd(Rb.u, unRb, nx); Rb.v = madd(Rb.v, unRb, ny);
     // c = sqrt(GAM p / r) = sqrt(a): dc = (GAM dp - a dr) / (2 c r), a = c^2
-    if (cLb.v != 0.0) {
+    if (!ip::zero(cLb.v)) {
         const T ab = hllc_quot(half(cLb), cL * L.r);
         Lb.p = madd(Lb.p, ab, GAM); Lb.r = madd(Lb.r, -ab, cL * cL);
     }
-    if (cRb.v != 0.0) {
+    if (!ip::zero(cRb.v)) {
         const T ab = hllc_quot(half(cRb), cR * R.r);
         Rb.p = madd(Rb.p, ab, GAM); Rb.r = madd(Rb.r, -ab, cR * cR);
     }

@@ -412,6 +412,7 @@ IP_FN bool not_negative(double x) {  // 0 <= x, -0 too
     const u64 b = ((u64)hi(x) << 32) | lo(x);
     return b <= 0x7ff0000000000000ull || b == 0x8000000000000000ull;
 }
+IP_FN bool zero(double x) { return ((hi(x) << 1) | lo(x)) == 0; }
 // x / 2: exact for normal results and zeros, by the exponent
 IP_FN double half(double x) {
     const u32 xa = hi(x) & 0x7fffffffu;
