@@ -1218,13 +1218,17 @@ __device__ __forceinline__ void flux_lane(const DevCase& c, int e, int gp, bool 
     if (live) reinterpret_cast<double2*>(c.F64)[2 * (size_t)e + gp] = make_double2(out[0], out[1]);
 }
 
-template <typename T, int RECON> constexpr int kFluxMinBlocks = sizeof(T) == 8 && RECON != RECON_NONE ? 3 : 0;
+// Registers of the two-lane flux: 80 (three blocks of 256 threads on an SM), with HLLC 64 (four):
+// two steps at 2.1M triangles 5.51 ms with 80, 5.27 with 64, 6.45 with 128; the exact Riemann solver
+// holds more at once (two steps at 130k triangles 728 us with 80, 737 with 64), Roe's gain is 0.4%.
+template <typename T, int FLUX, int RECON>
+constexpr int kFluxMinBlocks = sizeof(T) == 8 && RECON != RECON_NONE ? (FLUX == FLUX_HLLC ? 4 : 3) : 0;
 
 // k_flux: FP64 with reconstruction two lanes per edge, else one thread per edge
 template <typename T, int RECON> struct FluxLanes { static constexpr int n = sizeof(T) == 8 && RECON != RECON_NONE ? 2 : 1; };
 
 template <typename T, int FLUX, int RECON, bool STRIDE>
-__global__ void __launch_bounds__(256, kFluxMinBlocks<T, RECON>) k_flux(const DevCase c) {
+__global__ void __launch_bounds__(256, kFluxMinBlocks<T, FLUX, RECON>) k_flux(const DevCase c) {
     const int e0 = blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (FluxLanes<T, RECON>::n == 2) {
         const int n = 2 * c.ne;
