@@ -1323,8 +1323,8 @@ __device__ __forceinline__ void local_dt(const DevCase& c, int i, const Prim<dou
 template <typename T>
 __device__ __forceinline__ bool outside_limits(const DevCase& c, const Prim<T>& q) {  // :439-446
     if constexpr (sizeof(T) == 8)
-        return q.r < c.lim_rmin || q.r > c.lim_rmax || q.p < c.lim_pmin || q.p > c.lim_pmax ||
-               fabs(q.u) > c.lim_umax || fabs(q.v) > c.lim_umax;
+        return ip::less(q.r, c.lim_rmin) || ip::less(c.lim_rmax, q.r) || ip::less(q.p, c.lim_pmin) ||
+               ip::less(c.lim_pmax, q.p) || fabs(q.u) > c.lim_umax || fabs(q.v) > c.lim_umax;
     else
         return q.r < c.lim_f[0] || q.r > c.lim_f[1] || q.p < c.lim_f[2] || q.p > c.lim_f[3] ||
                fabsf(q.u) > c.lim_f[4] || fabsf(q.v) > c.lim_f[4];
