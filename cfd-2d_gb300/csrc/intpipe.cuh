@@ -13,7 +13,7 @@
 // immediate costs the 20), product 10.9 here, 8.3 per product with two native to three here;
 // reciprocal 24 (90 native), quotient 34 (144), square root 34 (170). A sum formed here takes
 // 22.6 and lost in every kernel it was tried in (two steps at 2.1M triangles 6.48 -> 7.17 ms),
-// so sums stay native. Kernels: k_flux at 2.1M triangles 1.42 -> 0.7 ms, with a lane per Gauss
+// so sums stay native. Kernels: k_flux at 2.1M triangles 1.42 -> 0.62 ms, with a lane per Gauss
 // point; the same arithmetic in one thread per edge gained nothing (200-255 registers).
 //
 // The common path takes operands with 2^-510 <= |x| < 2^510, whose products and quotients

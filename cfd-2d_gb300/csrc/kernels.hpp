@@ -242,7 +242,7 @@ void launch_objective_grad(const DevCase& c, const AdjCase& a, const double* w, 
                            cudaStream_t s);
 
 // built-in checks of the arithmetic helpers against the hardware operations
-// (which: 0 div_rn vs '/' and the integer-pipe operations of intpipe.cuh, 1 widen vs (double), 2 narrow vs (float) within 1 ulp)
+// (which: 0 the integer-pipe operations of intpipe.cuh, 1 widen vs (double), 2 narrow vs (float) within 1 ulp)
 long long selftest_arith(int which, long long n, unsigned long long seed);
 // deterministic FP64 sums of S*U over cells (mass, x/y momentum, energy)
 void launch_conservation(const DevCase& c, double* partial, int nblocks, cudaStream_t s);
