@@ -328,13 +328,13 @@ IP_FN u64 mulhi(u64 a, u64 b) {
 }
 IP_FN u32 mulhi32(u32 a, u32 b) { return (u32)(wide(a, b) >> 32); }
 
-// x^a for x in range and positive, 2^-20 <= a < 4 (in [2^-500, 2^500] as a result), within
-// 0.54 units in the last place: log2 and exp2 by tables of 64 entries and polynomials (the
-// scheme of Tang, ACM TOMS 15 (1989) and 16 (1990)) in fixed point, the products of the high
-// terms in 32 bits. The coefficients are Taylor's.
+// x^a for 2^-120 <= x < 2^120, 2^-9 <= a < 4 (in [2^-480, 2^480] as a result), within 0.54
+// units in the last place (0.532 the largest of 3 million samples per binade of a): log2 and
+// exp2 by tables of 64 entries and polynomials (the scheme of Tang, ACM TOMS 15 (1989) and 16
+// (1990)) in fixed point, the products of the high terms in 32 bits. The coefficients are Taylor's.
 IP_FN double pow_core(double x, double a) {
-    // a in Q61
-    const u32 ea = hi(a) >> 20;  // 1003 .. 1024
+    // a in Q61, exactly: its significand's lowest bit is Q62's tenth
+    const u32 ea = hi(a) >> 20;  // 1014 .. 1024
     const u64 am = ((u64)shl2(lo(a), mant_hi(a), 10) << 32) | (lo(a) << 10);  // Q62 of [1, 2)
     const u64 A = am >> (1024u - ea);                                           // Q61: a = am 2^(ea-1023-62)
     // log2(x) = e + F, F in Q62
@@ -384,10 +384,12 @@ IP_FN double pow_core(double x, double a) {
     return round_pack(Eh >> 11, ql, (El << 21) | (ql & 1u), (u32)(k + 1022) << 20);
 }
 IP_RARE double pow_rare(double x, double a) { return ::exp(::log(x) * a); }
-// x^a; what the fixed-point form does not take goes through exp and log
+// x^a; what the fixed-point form does not take goes through exp and log. A smaller exponent (a gas
+// with gamma < 1.004) would lose its last bits in Q61 (up to 0.80 units, exp and log 0.50 to 0.71);
+// from 2^-9 on exp and log are the less exact (0.85 units, 30 at a = 1/4).
 IP_FN double pow(double x, double a) {
-    // 2^-120 <= x < 2^120, 2^-20 <= a < 4
-    if (__builtin_expect(hi(x) - 0x38700000u < 0x0f000000u && hi(a) - 0x3eb00000u < 0x01600000u, 1)) return pow_core(x, a);
+    // 2^-120 <= x < 2^120, 2^-9 <= a < 4
+    if (__builtin_expect(hi(x) - 0x38700000u < 0x0f000000u && hi(a) - 0x3f600000u < 0x00b00000u, 1)) return pow_core(x, a);
     return pow_rare(x, a);
 }
 
