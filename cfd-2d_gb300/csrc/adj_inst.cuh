@@ -137,9 +137,10 @@ __device__ __forceinline__ void adj_flux_lane(const DevCase& c, const AdjCase& a
 // boundary edges (stored last) one thread each in the others
 template <int RECON> constexpr bool kAdjLanes = RECON != RECON_NONE;
 
-template <typename T, int FLUX, int RECON, int SIDE>
+// A: the type the edge is computed in (adj_native)
+template <typename T, int FLUX, int RECON, int SIDE, typename A>
 __device__ __forceinline__ void adj_flux_edge(const DevCase& c, const AdjCase& a, int e);
-template <typename T, int FLUX, int RECON>
+template <typename T, int FLUX, int RECON, typename A = Arith<T>>
 // FP32 faces: at most 128 registers (two 256-thread blocks' worth per SM), measured
 // faster than the compiler's unconstrained choice. With FP64 faces interior and boundary edges
 // (stored last) run their own instantiations.
@@ -154,16 +155,15 @@ k_adj_flux(const DevCase c, const AdjCase a, int n_lane) {
         }
         const int e = t + (kAdjLanes<RECON> ? c.n_int - n_lane * (int)blockDim.x : 0);
         if (e >= c.ne) return;
-        if (!kAdjLanes<RECON> && e < c.n_int) adj_flux_edge<T, FLUX, RECON, EDGE_INNER>(c, a, e);
-        else adj_flux_edge<T, FLUX, RECON, EDGE_BOUNDARY>(c, a, e);
+        if (!kAdjLanes<RECON> && e < c.n_int) adj_flux_edge<T, FLUX, RECON, EDGE_INNER, A>(c, a, e);
+        else adj_flux_edge<T, FLUX, RECON, EDGE_BOUNDARY, A>(c, a, e);
     } else {
         const int e = blockIdx.x * blockDim.x + threadIdx.x;
-        if (e < c.ne) adj_flux_edge<T, FLUX, RECON, EDGE_ANY>(c, a, e);
+        if (e < c.ne) adj_flux_edge<T, FLUX, RECON, EDGE_ANY, A>(c, a, e);
     }
 }
-template <typename T, int FLUX, int RECON, int SIDE>
+template <typename T, int FLUX, int RECON, int SIDE, typename A>
 __device__ __forceinline__ void adj_flux_edge(const DevCase& c, const AdjCase& a, int e) {
-    typedef Arith<T> A;
     const int ne = c.ne;
     const T* W = W_of<T>(c);
     const T* G = G_of<T>(c);
@@ -266,9 +266,9 @@ __global__ void __launch_bounds__(128) k_flux_rec(const DevCase c, const FluxRec
 // k_adj_flux (HLLC) reading the forward's record of each Gauss point instead of
 // recomputing the reconstruction, the ghost state, the sound speeds and minmod's
 // branches: the same reverse operations on the same values, so the same bits.
-template <typename T, int RECON, int SIDE>
+template <typename T, int RECON, int SIDE, typename A>
 __device__ __forceinline__ void adj_flux_rec_edge(const DevCase& c, const AdjCase& a, const FluxRec& r, int e);
-template <typename T, int RECON>
+template <typename T, int RECON, typename A = Arith<T>>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : 128, sizeof(T) == 4 ? 2 : 4)
 k_adj_flux_rec(const DevCase c, const AdjCase a, const FluxRec r, int n_lane) {
     if constexpr (sizeof(T) == 8) {
@@ -280,16 +280,15 @@ k_adj_flux_rec(const DevCase c, const AdjCase a, const FluxRec r, int n_lane) {
         }
         const int e = t + (kAdjLanes<RECON> ? c.n_int - n_lane * (int)blockDim.x : 0);
         if (e >= c.ne) return;
-        if (!kAdjLanes<RECON> && e < c.n_int) adj_flux_rec_edge<T, RECON, EDGE_INNER>(c, a, r, e);
-        else adj_flux_rec_edge<T, RECON, EDGE_BOUNDARY>(c, a, r, e);
+        if (!kAdjLanes<RECON> && e < c.n_int) adj_flux_rec_edge<T, RECON, EDGE_INNER, A>(c, a, r, e);
+        else adj_flux_rec_edge<T, RECON, EDGE_BOUNDARY, A>(c, a, r, e);
     } else {
         const int e = blockIdx.x * blockDim.x + threadIdx.x;
-        if (e < c.ne) adj_flux_rec_edge<T, RECON, EDGE_ANY>(c, a, r, e);
+        if (e < c.ne) adj_flux_rec_edge<T, RECON, EDGE_ANY, A>(c, a, r, e);
     }
 }
-template <typename T, int RECON, int SIDE>
+template <typename T, int RECON, int SIDE, typename A>
 __device__ __forceinline__ void adj_flux_rec_edge(const DevCase& c, const AdjCase& a, const FluxRec& r, int e) {
-    typedef Arith<T> A;
     const int ne = c.ne;
     const T* DL = DL_of<T>(c);
     const A nx(NX_of<T>(c)[e]), ny(NY_of<T>(c)[e]), l(L_of<T>(c)[e]);
@@ -507,11 +506,19 @@ inline int adj_flux_grid(const DevCase& c, int recon, int& n_lane) {
     n_lane = sizeof(KT) == 8 && recon != RECON_NONE ? adj_nblk(2l * c.n_int, 128) : 0;
     return n_lane ? n_lane + adj_nblk(c.ne - c.n_int, 128) : adj_nblk(c.ne, 128);
 }
+// First order, FP64 faces, one thread per edge: on the FP64 unit (A = double) while the mesh has at
+// most a warp for each of an SM's four schedulers, where an operation's latency counts and the
+// unit waits for nobody; products on the integer pipes (A = xd, the same bits) from there on. A
+// gradient (6 steps, SSP-RK3, 152 SMs: the line is at 19,456 edges), xd against double, us: 1,240
+// edges HLLC 1,355 / 1,280, LAX 1,540 / 1,401; 19,360 edges 1,272 / 1,197, 1,396 / 1,278; 27,840
+// edges 1,311 / 1,297, 1,450 / 1,440; 43,440 edges 1,533 / 1,580, 1,682 / 1,816.
+inline bool adj_native(const DevCase& c) { return sizeof(KT) == 8 && c.ne <= 4 * 32 * c.sms; }
 template <int FLUX>
 void adj_flux_by_recon(const DevCase& c, const AdjCase& a, int recon, cudaStream_t s) {
     int n_lane;
     const int g = adj_flux_grid(c, recon, n_lane);
-    if (recon == RECON_NONE) k_adj_flux<KT, FLUX, RECON_NONE><<<g, 128, 0, s>>>(c, a, n_lane);
+    if (recon == RECON_NONE && adj_native(c)) k_adj_flux<KT, FLUX, RECON_NONE, KT><<<g, 128, 0, s>>>(c, a, n_lane);
+    else if (recon == RECON_NONE) k_adj_flux<KT, FLUX, RECON_NONE><<<g, 128, 0, s>>>(c, a, n_lane);
     else if (recon == RECON_LINEAR) k_adj_flux<KT, FLUX, RECON_LINEAR><<<g, 128, 0, s>>>(c, a, n_lane);
     else k_adj_flux<KT, FLUX, RECON_MINMOD><<<g, 128, 0, s>>>(c, a, n_lane);
 }
@@ -531,7 +538,8 @@ void KFN(flux_rec)(const DevCase& c, int recon, const FluxRec& r, cudaStream_t s
 void KFN(adj_flux_rec)(const DevCase& c, const AdjCase& a, int recon, const FluxRec& r, cudaStream_t s) {
     int n_lane;
     const int g = adj_flux_grid(c, recon, n_lane);
-    if (recon == RECON_NONE) k_adj_flux_rec<KT, RECON_NONE><<<g, 128, 0, s>>>(c, a, r, n_lane);
+    if (recon == RECON_NONE && adj_native(c)) k_adj_flux_rec<KT, RECON_NONE, KT><<<g, 128, 0, s>>>(c, a, r, n_lane);
+    else if (recon == RECON_NONE) k_adj_flux_rec<KT, RECON_NONE><<<g, 128, 0, s>>>(c, a, r, n_lane);
     else if (recon == RECON_LINEAR) k_adj_flux_rec<KT, RECON_LINEAR><<<g, 128, 0, s>>>(c, a, r, n_lane);
     else k_adj_flux_rec<KT, RECON_MINMOD><<<g, 128, 0, s>>>(c, a, r, n_lane);
 }

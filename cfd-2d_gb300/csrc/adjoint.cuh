@@ -85,7 +85,7 @@ __device__ __forceinline__ void vjp_cons2prim(const T* U, T gm1, const Prim<T>& 
 // (E = p/(r gm1) + (u^2 + v^2)/2): no read of the FP64 state.
 template <typename T>
 __device__ __forceinline__ void vjp_cons2prim_q(const Prim<T>& q, T gm1, const Prim<T>& pb, T* Ub) {
-        const T ro = q.r, iro = hllc_recip(ro), u = q.u, v = q.v;
+    const T ro = q.r, iro = hllc_recip(ro), u = q.u, v = q.v;
     const T e = hllc_quot(q.p, ro * gm1);
     const T E = madd(e, T(0.5), t_fma(u, u, v * v));
     T rb = madd(pb.r, pb.p * e, gm1);
@@ -198,18 +198,15 @@ __device__ __forceinline__ void vjp_lax(const Prim<T>& L, const Prim<T>& R, T nx
 }
 
 // Ss = num / den as the forward forms it (hllc_quot), and 1/den for the derivatives
-__device__ __forceinline__ xd star_speed(xd num, xd den, xd& iden) {
+template <typename T>
+__device__ __forceinline__ T star_speed(T num, T den, T& iden) {
     iden = hllc_recip(den);
     return hllc_quot(num, den);
-}
-__device__ __forceinline__ float star_speed(float num, float den, float& iden) {
-    iden = 1.0f / den;
-    return num / den;
 }
 
 // HLLC in the single-division star-flux form (flux_hllc in kernels.cuh), with the forward's
 // sound speeds cL, cR given
-template <typename T>
+template <typename T, std::enable_if_t<sizeof(T) == 4, int> = 0>
 __device__ __forceinline__ void vjp_hllc_c(const Prim<T>& L, const Prim<T>& R, T cL, T cR, T nx, T ny, T GAM, T IG1,
                                            const T* fb, Prim<T>& Lb, Prim<T>& Rb) {
     const T unL = dot2(L.u, nx, L.v, ny), unR = dot2(R.u, nx, R.v, ny);
@@ -312,13 +309,13 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<T>& L, const Prim<T>& R, T
 // S_K U_K - F_K from m_K = rho_K d_K, d_K = S_K - un_K, and only the used side's energy),
 // recomputing the forward's values and branches with its own expressions. A sum's first product
 // is written as one (Lb and Rb are empty on entry): on the integer pipes, where a multiply-add
-// onto the empty sum would be an FP64 product.
-__device__ __forceinline__ void vjp_hllc_c(const Prim<xd>& L, const Prim<xd>& R, xd cL, xd cR, xd nx, xd ny, xd GAM,
-                                           xd IG1, const xd* fb, Prim<xd>& Lb, Prim<xd>& Rb) {
-    typedef xd T;
+// onto the empty sum would be an FP64 product. T: xd or double (the same bits).
+template <typename T, std::enable_if_t<sizeof(T) == 8, int> = 0>
+__device__ __forceinline__ void vjp_hllc_c(const Prim<T>& L, const Prim<T>& R, T cL, T cR, T nx, T ny, T GAM, T IG1,
+                                           const T* fb, Prim<T>& Lb, Prim<T>& Rb) {
     const T unL = dot2(L.u, nx, L.v, ny), unR = dot2(R.u, nx, R.v, ny);
     const T sl1 = unL - cL, sl2 = unR - cR, sr1 = unL + cL, sr2 = unR + cR;
-    const bool l1 = ip::less(sl1.v, sl2.v), r1 = ip::less(sr2.v, sr1.v);
+    const bool l1 = less(sl1, sl2), r1 = less(sr2, sr1);
     const T SL = l1 ? sl1 : sl2, SR = r1 ? sr1 : sr2;
     T unLb = acc0<T>(), unRb = acc0<T>(), SLb = acc0<T>(), SRb = acc0<T>(), cLb = acc0<T>(), cRb = acc0<T>();
     // E = p IG1 + .5 r (u^2 + v^2): the adjoint Eb of one side's energy into its state
@@ -408,11 +405,11 @@ __device__ __forceinline__ void vjp_hllc_c(const Prim<xd>& L, const Prim<xd>& R,
     Lb.u = madd(Lb.u, unLb, nx); Lb.v = madd(Lb.v, unLb, ny);
     Rb.u = madd(Rb.u, unRb, nx); Rb.v = madd(Rb.v, unRb, ny);
     // c = sqrt(GAM p / r) = sqrt(a): dc = (GAM dp - a dr) / (2 c r), a = c^2
-    if (!ip::zero(cLb.v)) {
+    if (!is_zero(cLb)) {
         const T ab = hllc_quot(half(cLb), cL * L.r);
         Lb.p = madd(Lb.p, ab, GAM); Lb.r = madd(Lb.r, -ab, cL * cL);
     }
-    if (!ip::zero(cRb.v)) {
+    if (!is_zero(cRb)) {
         const T ab = hllc_quot(half(cRb), cR * R.r);
         Rb.p = madd(Rb.p, ab, GAM); Rb.r = madd(Rb.r, -ab, cR * cR);
     }

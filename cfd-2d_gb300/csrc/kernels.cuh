@@ -59,7 +59,12 @@ template <typename T> __device__ __forceinline__ T t_min(T a, T b) { return a < 
 __device__ __forceinline__ xd t_max(xd a, xd b) { return ip::less(b.v, a.v) ? a : b; }
 __device__ __forceinline__ xd t_min(xd a, xd b) { return ip::less(a.v, b.v) ? a : b; }
 __device__ __forceinline__ bool not_negative(xd x) { return ip::not_negative(x.v); }  // x >= 0
+__device__ __forceinline__ bool not_negative(double x) { return ip::not_negative(x); }
 __device__ __forceinline__ bool not_negative(float x) { return x >= 0.0f; }
+__device__ __forceinline__ bool less(xd a, xd b) { return ip::less(a.v, b.v); }
+__device__ __forceinline__ bool less(double a, double b) { return ip::less(a, b); }
+__device__ __forceinline__ bool is_zero(xd x) { return ip::zero(x.v); }
+__device__ __forceinline__ bool is_zero(double x) { return ip::zero(x); }
 
 template <typename T> __device__ __forceinline__ const T* W_of(const DevCase& c);
 template <> __device__ __forceinline__ const double* W_of<double>(const DevCase& c) { return c.W64; }
@@ -195,6 +200,7 @@ __device__ __forceinline__ xd neg_if(xd x, bool s) { return xd(neg_if(x.v, s)); 
 __device__ __forceinline__ float neg_if(float x, bool s) { return __int_as_float(__float_as_int(x) ^ (s ? (int)0x80000000 : 0)); }
 // a / b given y = RN(1/b): the correctly rounded quotient in FP64, a * y in the FP32 faces.
 __device__ __forceinline__ xd div_by(xd a, xd b, xd) { return a / b; }
+__device__ __forceinline__ double div_by(double a, double b, double) { return ip::quot(a, b); }
 __device__ __forceinline__ float div_by(float a, float, float y) { return a * y; }
 // Quotients by a shared divisor: recip_of the divisor once, div_y per dividend (FP32 divides).
 struct NoRecip {};
@@ -507,10 +513,13 @@ template <typename T> __device__ __forceinline__ T energy(T r, T u, T v, T p, T 
 // integer pipes with FP64 faces. (Newton sequences of FP64 multiply-adds from binary32 seeds,
 // 4 to 6 instructions each, held the FP64 unit longer: a flux evaluation had 16 of them.)
 __device__ __forceinline__ xd hllc_quot(xd a, xd b) { return a / b; }
+__device__ __forceinline__ double hllc_quot(double a, double b) { return ip::quot(a, b); }
 __device__ __forceinline__ float hllc_quot(float a, float b) { return a / b; }
 __device__ __forceinline__ xd hllc_recip(xd b) { return xd(ip::rcp(b.v)); }
+__device__ __forceinline__ double hllc_recip(double b) { return ip::rcp(b); }
 __device__ __forceinline__ float hllc_recip(float b) { return 1.0f / b; }
 __device__ __forceinline__ xd hllc_sound(xd a, xd r) { return t_sqrt(a / r); }
+__device__ __forceinline__ double hllc_sound(double a, double r) { return ip::sqrt(ip::quot(a, r)); }
 __device__ __forceinline__ float hllc_sound(float a, float r) { return t_sqrt(a / r); }
 
 // HLLC (Toro, Riemann Solvers and Numerical Methods for Fluid Dynamics, sec. 10.4-10.6),

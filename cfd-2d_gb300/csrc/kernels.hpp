@@ -86,6 +86,7 @@ enum { KIND_GRAD = 0, KIND_FLUX = 1, KIND_UPDATE = 2, N_TUNED_KINDS = 3 };
 struct DevCase {
     int nc, ne, n_int;
     LaunchShape shape[N_TUNED_KINDS];
+    int sms;               // multiprocessors of the GPU
     // geometry
     const int* face;       // 3*nc
     // the same faces seen from the cell, for the gradient gather (one level of

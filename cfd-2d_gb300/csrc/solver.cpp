@@ -76,6 +76,7 @@ Solver::Solver(const TaskConfig& t, Topo&& topo, const std::vector<int>& cell_re
     try {
         DevCase& c = dc_;
         c.nc = nc; c.ne = ne; c.n_int = lay_.n_int;
+        CUDA_CHECK(cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev_));
         c.face = upload(lay_.face);
         c.ec1 = upload(lay_.ec1);
         c.ec2 = upload(lay_.ec2);
