@@ -222,7 +222,6 @@ Solver::Solver(const TaskConfig& t, Topo&& topo, const std::vector<int>& cell_re
         dtmin_ = dalloc<unsigned long long>(1);
         partial_ = dalloc<double>(4 * kConservationBlocks);
         CUDA_CHECK(cudaMallocHost(&status_host_, sizeof(unsigned)));
-        CUDA_CHECK(cudaEventCreateWithFlags(&copied_, cudaEventDisableTiming));
         CUDA_CHECK(cudaMemsetAsync(c.flags, 0, sizeof(unsigned) * nc, stream_));
         CUDA_CHECK(cudaMemsetAsync(c.n_lim, 0, sizeof(int), stream_));
         CUDA_CHECK(cudaMemsetAsync(c.err, 0, sizeof(unsigned), stream_));
@@ -250,7 +249,6 @@ Solver::Solver(const TaskConfig& t, Topo&& topo, const std::vector<int>& cell_re
         if (gexec_many_) cudaGraphExecDestroy(gexec_many_);
         if (graph_) cudaGraphDestroy(graph_);
         if (status_host_) cudaFreeHost(status_host_);
-        if (copied_) cudaEventDestroy(copied_);
         if (stream_) cudaStreamDestroy(stream_);
         stream_ = nullptr;
         throw;
@@ -286,7 +284,6 @@ Solver::~Solver() {
     if (graph_) cudaGraphDestroy(graph_);
     if (stream_) cudaStreamSynchronize(stream_);
     if (status_host_) cudaFreeHost(status_host_);
-    if (copied_) cudaEventDestroy(copied_);
     for (void* p : allocs_) cudaFree(p);
     if (stream_) cudaStreamDestroy(stream_);
 }
@@ -567,13 +564,12 @@ void Solver::set_state(const double* ro, const double* ru, const double* rv, con
                                        stream_));
         launch_gather_state(dc_, stage_, dc_.A, stream_);
     }
-    CUDA_CHECK(cudaEventRecord(copied_, stream_));
     launch_prims(dc_, task_.precision, stream_);
     if (reset_tau) {
         tau_ = task_.tau;
         compute_tau();
     }
-    CUDA_CHECK(cudaEventSynchronize(copied_));  // the primitives follow on the stream
+    CUDA_CHECK(cudaStreamSynchronize(stream_));
 }
 
 void Solver::get_ctau(double* out) {

@@ -195,7 +195,6 @@ private:
     static constexpr int kGraphSteps = 8;
     void launch_steps(int n);               // n steps' kernels
     unsigned* status_host_ = nullptr;       // pinned: the device error word
-    cudaEvent_t copied_ = nullptr;          // the caller's arrays have been read
     std::vector<Instance> inst_;
     void compute_tau_batch();
     void rebuild_graph();
