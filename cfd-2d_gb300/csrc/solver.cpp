@@ -387,10 +387,6 @@ double Solver::timed_steps(int n) {
     CUDA_CHECK(cudaEventCreate(&b));
     CUDA_CHECK(cudaStreamSynchronize(stream_));
     CUDA_CHECK(cudaEventRecord(a, stream_));
-    for (int k = 0; k < n; k++) {
-        if (!task_.steady) t_ += tau_;
-        steps_++;
-    }
     launch_steps(n);
     CUDA_CHECK(cudaEventRecord(b, stream_));
     CUDA_CHECK(cudaEventSynchronize(b));
@@ -445,9 +441,19 @@ void Solver::build_graph() {
     CUDA_CHECK(e);
 }
 
-void Solver::launch_steps(int n) {
-    for (; n >= kGraphSteps; n -= kGraphSteps) CUDA_CHECK(cudaGraphLaunch(gexec_many_, stream_));
-    for (; n > 0; n--) CUDA_CHECK(cudaGraphLaunch(gexec_, stream_));
+void Solver::launch_steps(int n, bool instances) {
+    while (n > 0) {
+        const int k = n >= kGraphSteps ? kGraphSteps : 1;
+        CUDA_CHECK(cudaGraphLaunch(k > 1 ? gexec_many_ : gexec_, stream_));
+        for (int j = 0; j < k; j++) {
+            steps_++;
+            if (task_.steady) continue;
+            t_ += tau_;  // src/methods/fvm_tvd.cpp:312-316
+            if (instances)
+                for (auto& in : inst_) in.t += in.tau;
+        }
+        n -= k;
+    }
 }
 
 int Solver::read_status() {
@@ -462,13 +468,7 @@ int Solver::read_status() {
 
 int Solver::step(int n) {
     use_device();
-    for (int k = 0; k < n; k++) {
-        if (!task_.steady) t_ += tau_;  // src/methods/fvm_tvd.cpp:312-316
-        if (!task_.steady)
-            for (auto& in : inst_) in.t += in.tau;
-        steps_++;
-    }
-    launch_steps(n);
+    launch_steps(n, true);
     return read_status();
 }
 

@@ -193,7 +193,9 @@ private:
     // steps of one graph launch: between graphs the GPU waits 2-3 us longer than between a
     // graph's kernels, a tenth of a step on a small mesh
     static constexpr int kGraphSteps = 8;
-    void launch_steps(int n);               // n steps' kernels
+    // n steps' kernels; the time and the step count (instances: and the instances' times) move
+    // with each launch, so that after one that failed they are those of what was launched
+    void launch_steps(int n, bool instances = false);
     unsigned* status_host_ = nullptr;       // pinned: the device error word
     std::vector<Instance> inst_;
     void compute_tau_batch();

@@ -179,10 +179,6 @@ double Solver::forward(int nsteps, int k, int* status) {
             last_recorded_ = true;
             continue;
         }
-        for (int j = 0; j < n; j++) {
-            if (!task_.steady) t_ += tau_;
-            steps_++;
-        }
         launch_steps(n);
     }
     fw_steps_ = nsteps;

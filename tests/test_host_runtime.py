@@ -161,3 +161,13 @@ def test_set_state_returns_with_its_work_done(seen, call):
     assert "kernel" in log
     last = len(log) - 1 - log[::-1].index("kernel")
     assert "wait-stream" in log[last:], log
+
+
+def test_steps_and_time_are_those_launched_when_a_launch_fails(seen):
+    per_step = seen["step7"]["kernels"] // 7
+    before = seen["step16"][1]
+    for r in seen["fail"]:
+        assert not r["ok"]
+        assert (r["steps"] - before["steps"]) * per_step == r["kernels"]
+        assert r["time"] == 0.125 * r["steps"]
+        before = r
