@@ -385,6 +385,7 @@ double Solver::timed_steps(int n) {
     cudaEvent_t a, b;
     CUDA_CHECK(cudaEventCreate(&a));
     CUDA_CHECK(cudaEventCreate(&b));
+    if (n >= kGraphSteps && !gexec_many_ && !many_failed_) build_many();
     CUDA_CHECK(cudaStreamSynchronize(stream_));
     CUDA_CHECK(cudaEventRecord(a, stream_));
     launch_steps(n);
@@ -419,31 +420,46 @@ void Solver::profile_steps(int n, double ms[4], int launches[4]) {
     for (auto& e : ev) cudaEventDestroy(e);
 }
 
+cudaGraph_t Solver::capture_steps(int n) {
+    cudaGraph_t g = nullptr;
+    CUDA_CHECK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+    try {
+        for (int k = 0; k < n; k++) enqueue_step();
+    } catch (...) {
+        cudaStreamEndCapture(stream_, &g);
+        if (g) cudaGraphDestroy(g);
+        throw;
+    }
+    CUDA_CHECK(cudaStreamEndCapture(stream_, &g));
+    return g;
+}
+
 void Solver::build_graph() {
-    auto capture = [&](int steps) {
-        cudaGraph_t g = nullptr;
-        CUDA_CHECK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-        try {
-            for (int k = 0; k < steps; k++) enqueue_step();
-        } catch (...) {
-            cudaStreamEndCapture(stream_, &g);
-            if (g) cudaGraphDestroy(g);
-            throw;
-        }
-        CUDA_CHECK(cudaStreamEndCapture(stream_, &g));
-        return g;
-    };
-    graph_ = capture(1);
+    graph_ = capture_steps(1);
     CUDA_CHECK(cudaGraphInstantiate(&gexec_, graph_, 0));
-    cudaGraph_t many = capture(kGraphSteps);
-    const cudaError_t e = cudaGraphInstantiate(&gexec_many_, many, 0);
-    cudaGraphDestroy(many);
-    CUDA_CHECK(e);
+}
+
+// The graph of kGraphSteps steps. A handle that cannot have it goes on with single steps.
+void Solver::build_many() {
+    many_wanted_ = false;
+    cudaGraph_t g = nullptr;
+    try {
+        g = capture_steps(kGraphSteps);
+        CUDA_CHECK(cudaGraphInstantiate(&gexec_many_, g, 0));
+        CUDA_CHECK(cudaGraphUpload(gexec_many_, stream_));
+    } catch (const Error&) {
+        cudaGetLastError();
+        if (gexec_many_) cudaGraphExecDestroy(gexec_many_);
+        gexec_many_ = nullptr;
+        many_failed_ = true;
+    }
+    if (g) cudaGraphDestroy(g);
 }
 
 void Solver::launch_steps(int n, bool instances) {
+    if (n >= kGraphSteps && !gexec_many_ && !many_failed_) many_wanted_ = true;
     while (n > 0) {
-        const int k = n >= kGraphSteps ? kGraphSteps : 1;
+        const int k = n >= kGraphSteps && gexec_many_ ? kGraphSteps : 1;
         CUDA_CHECK(cudaGraphLaunch(k > 1 ? gexec_many_ : gexec_, stream_));
         for (int j = 0; j < k; j++) {
             steps_++;
@@ -458,6 +474,7 @@ void Solver::launch_steps(int n, bool instances) {
 
 int Solver::read_status() {
     CUDA_CHECK(cudaMemcpyAsync(status_host_, dc_.err, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_));
+    if (many_wanted_) build_many();  // while the GPU runs the steps that wanted it
     CUDA_CHECK(cudaStreamSynchronize(stream_));
     const unsigned e = *status_host_;
     if (e) CUDA_CHECK(cudaMemsetAsync(dc_.err, 0, sizeof(unsigned), stream_));

@@ -189,7 +189,14 @@ private:
     cudaStream_t stream_ = nullptr;
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t gexec_ = nullptr;
-    cudaGraphExec_t gexec_many_ = nullptr;  // kGraphSteps steps
+    // kGraphSteps steps. Made by the first call that takes so many at once, while the GPU runs that
+    // call's single steps (that call 614 us against 613 with the graph made beforehand, mixed 300
+    // against 285; a later one 574, 252; 162 triangles, eight steps). Made with the handle it cost
+    // every handle 170 us (FP64, 450 -> 620) or 130 us (mixed).
+    cudaGraphExec_t gexec_many_ = nullptr;
+    bool many_wanted_ = false, many_failed_ = false;
+    cudaGraph_t capture_steps(int n);
+    void build_many();
     // steps of one graph launch: between graphs the GPU waits 2-3 us longer than between a
     // graph's kernels, a tenth of a step on a small mesh
     static constexpr int kGraphSteps = 8;

@@ -143,6 +143,7 @@ void Solver::rebuild_graph() {
     if (graph_) cudaGraphDestroy(graph_);
     gexec_ = gexec_many_ = nullptr;
     graph_ = nullptr;
+    many_wanted_ = many_failed_ = false;
     build_graph();
 }
 

@@ -171,3 +171,24 @@ def test_steps_and_time_are_those_launched_when_a_launch_fails(seen):
         assert (r["steps"] - before["steps"]) * per_step == r["kernels"]
         assert r["time"] == 0.125 * r["steps"]
         before = r
+
+
+def test_graph_of_many_steps_is_made_by_the_first_call_that_takes_them(seen):
+    per_step = seen["step7"]["kernels"] // 7
+    one, many = ["make%d" % per_step], ["make%d" % (8 * per_step)]
+
+    def makes(log):
+        return [c for c in log if c.startswith("make")]
+
+    assert makes(seen["create"]) == one
+    assert makes(seen["step7"]["log"]) == []
+    first, second = (r["log"] for r in seen["step16"])
+    assert makes(first) == many and makes(second) == []
+    # made behind the launches, before the wait for them
+    assert [c for c in first if c != "kernel"] == ["graph%d" % per_step] * 16 + many + ["wait-stream"]
+    assert [c for c in second if c != "kernel"] == ["graph%d" % (8 * per_step)] * 2 + ["wait-stream"]
+
+
+def test_steps_go_on_where_the_graph_of_many_cannot_be_made(seen):
+    for k, r in enumerate(seen["no_graph"]):
+        assert r["ok"] and r["steps"] == 16 * (k + 1) and r["kernels"] == 16 * (seen["step7"]["kernels"] // 7)
