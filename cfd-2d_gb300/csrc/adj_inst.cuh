@@ -137,6 +137,15 @@ __device__ __forceinline__ void adj_flux_lane(const DevCase& c, const AdjCase& a
 // boundary edges (stored last) one thread each in the others
 template <int RECON> constexpr bool kAdjLanes = RECON != RECON_NONE;
 
+// SIDE: EDGE_ANY (interior or boundary, decided at run time), EDGE_INNER or EDGE_BOUNDARY (known at
+// compile time: the interior instantiation carries no boundary code, which a warp would
+// otherwise issue, predicated off, for every interior edge).
+enum { EDGE_ANY = 0, EDGE_INNER = 1, EDGE_BOUNDARY = 2 };
+template <int SIDE>
+__device__ __forceinline__ bool edge_inner(const DevCase& c, int e) {
+    return SIDE == EDGE_INNER ? true : (SIDE == EDGE_BOUNDARY ? false : e < c.n_int);
+}
+
 // A: the type the edge is computed in (adj_native)
 template <typename T, int FLUX, int RECON, int SIDE, typename A>
 __device__ __forceinline__ void adj_flux_edge(const DevCase& c, const AdjCase& a, int e);

@@ -4,8 +4,8 @@
 // own, as in the reference's x86/ARM build) and by kern_mixed.cu.
 //
 // Bit-reproducibility without atomics: every interior edge flux is computed
-// once (k_flux, one thread per edge) and each cell gathers its three edge
-// fluxes in ascending original edge number with the reference's signs
+// once (k_flux; FP64 with a reconstruction by two lanes per edge, else by one
+// thread) and each cell gathers its three edge fluxes in ascending original edge number with the reference's signs
 // (c1: -=, c2: +=, src/methods/fvm_tvd.cpp:353-363). That is the order in which
 // the reference's edge loop accumulates into each cell, so the FP64 sums are
 // the reference's sums.
@@ -936,37 +936,25 @@ __device__ __forceinline__ EdgeGeo<T> load_geo(const DevCase& c, int e) {
         g.nx = ldcs(NX_of<T>(c) + e);
         g.ny = ldcs(NY_of<T>(c) + e);
         g.l = ldcs(L_of<T>(c) + e);
-        if (RECON != RECON_NONE) {
-            const T* __restrict__ DL = DL_of<T>(c);
-#pragma unroll
-            for (int k = 0; k < 8; k++) g.dl[k] = ldcs(DL + (size_t)k * c.ne + e);
-        }
     }
     return g;
 }
 
 // With REC (HLLC only) the evaluation also leaves what the adjoint's recorded path reads
 // (FluxRec): per Gauss point the two face states and sound speeds, and minmod's branches.
-// SIDE: EDGE_ANY (interior or boundary, decided at run time), EDGE_INNER or EDGE_BOUNDARY
-// (known at compile time: the interior instantiation carries no boundary code, which a
-// warp would otherwise issue, predicated off, for every interior edge; the adjoint's flux
-// kernels use them).
-enum { EDGE_ANY = 0, EDGE_INNER = 1, EDGE_BOUNDARY = 2 };
-template <int SIDE>
-__device__ __forceinline__ bool edge_inner(const DevCase& c, int e) {
-    return SIDE == EDGE_INNER ? true : (SIDE == EDGE_BOUNDARY ? false : e < c.n_int);
-}
-template <typename T, int FLUX, int RECON, bool REC = false, int SIDE = EDGE_ANY>
+// FP32 faces, or no reconstruction (FP64 with one: flux_lane).
+template <typename T, int FLUX, int RECON, bool REC = false>
 __device__ __forceinline__ void flux_core(const DevCase& c, int e, int c1, const Prim<T>& qL_, const T* gL,
                                           const Prim<T>& qR_, const T* gR, T* out, const EdgeGeo<T>& geo,
                                           const FluxRec& rec = FluxRec{}) {
     typedef Arith<T> A;
     const Prim<A> qL = prim_as<A>(qL_), qR = prim_as<A>(qR_);
     static_assert(!REC || FLUX == FLUX_HLLC, "flux records are kept for HLLC");
+    static_assert(sizeof(T) == 4 || RECON == RECON_NONE, "FP64 with a reconstruction: flux_lane");
     // qR: the second cell's primitives on interior edges (e < n_int), qL on boundary edges
     const A nx(geo.nx), ny(geo.ny), l(geo.l);
     const A GAM = gam_of<A>(c), IG1 = ig1_of<A>(c);
-    const bool inner = edge_inner<SIDE>(c, e);
+    const bool inner = e < c.n_int;
     Prim<A> gc = qL;
     DevBnd b{};
     A Tc = A(0), M = A(0);
@@ -977,21 +965,15 @@ __device__ __forceinline__ void flux_core(const DevCase& c, int e, int c1, const
         M = mt.M;
         if (RECON == RECON_MINMOD) gc = ghost_state(b, qL, Tc, nx, ny, M);
     }
-    // minmod's neighbour-minus-centre differences of both sides: formed once per edge in
-    // FP64 (the FP64 pipe is the bound there); per Gauss point in FP32 (fewer live registers)
+    // minmod's neighbour-minus-centre differences of both sides, per Gauss point (fewer live registers)
     Prim<A> dL = qL, dR = qL;
-    if (RECON == RECON_MINMOD && sizeof(T) == 8) {
-        const Prim<A>& nb = inner ? qR : gc;
-        dL.r = nb.r - qL.r; dL.u = nb.u - qL.u; dL.v = nb.v - qL.v; dL.p = nb.p - qL.p;
-        dR.r = neg_if(dL.r, true); dR.u = neg_if(dL.u, true); dR.v = neg_if(dL.v, true); dR.p = neg_if(dL.p, true);
-    }
     A fs[4] = {A(0.0), A(0.0), A(0.0), A(0.0)};
     bool hit = false;
     unsigned codes = 0;
 #pragma unroll
     for (int gp = 0; gp < 2; gp++) {
         Prim<A> pL = qL, pR;
-        if (RECON == RECON_MINMOD && sizeof(T) == 4) {
+        if (RECON == RECON_MINMOD) {
             const Prim<A>& nb = inner ? qR : gc;
             dL.r = nb.r - qL.r; dL.u = nb.u - qL.u; dL.v = nb.v - qL.v; dL.p = nb.p - qL.p;
             dR.r = qL.r - qR.r; dR.u = qL.u - qR.u; dR.v = qL.v - qR.v; dR.p = qL.p - qR.p;
@@ -1036,12 +1018,12 @@ __device__ __forceinline__ void flux_core(const DevCase& c, int e, int c1, const
 }
 
 // The flux of edge e (what F holds for it) from the stage's W and G (with REC: and its record).
-template <typename T, int FLUX, int RECON, bool REC = false, int SIDE = EDGE_ANY>
+template <typename T, int FLUX, int RECON, bool REC = false>
 __device__ __forceinline__ void flux_edge(const DevCase& c, int e, T* out, const FluxRec& rec = FluxRec{}) {
     const T* __restrict__ W = W_of<T>(c);
     const T* __restrict__ G = G_of<T>(c);
     const int c1 = ldcs(c.ec1 + e);
-    const bool inner = edge_inner<SIDE>(c, e);
+    const bool inner = e < c.n_int;
     const Prim<T> qL = load_prim(W, c1);
     T gL[8], gR[8];
     if (RECON != RECON_NONE) ld8(G, c1, gL);
@@ -1051,7 +1033,7 @@ __device__ __forceinline__ void flux_edge(const DevCase& c, int e, T* out, const
         qR = load_prim(W, c2);
         if (RECON != RECON_NONE) ld8(G, c2, gR);
     }
-    flux_core<T, FLUX, RECON, REC, SIDE>(c, e, c1, qL, gL, qR, gR, out, load_geo<T, RECON>(c, e), rec);
+    flux_core<T, FLUX, RECON, REC>(c, e, c1, qL, gL, qR, gR, out, load_geo<T, RECON>(c, e), rec);
 }
 
 template <typename T, int FLUX, int RECON>
