@@ -192,15 +192,14 @@ Solver::Solver(const TaskConfig& t, Topo&& topo, const std::vector<int>& cell_re
         c.newton_cap = task_.newton_cap;
         c.flux_pipe = mixed && task_.flux_pipe != 0 ? 1 : 0;
         if (c.flux_pipe) launch_flux_prepare_mixed();
-        // FP64 face kernels are long (the flux up to 100 KB of code): warps of one block run
-        // through it together and share the instruction cache, so large blocks are faster once
-        // they fill the chip three times (flux, 152 SMs x 3 blocks of 256 lanes: 7% at 130k
-        // triangles, 1.8% at 2.1M); on a smaller mesh (1.7 fillings: 1.5% slower) their last,
-        // partly filled round costs more than that
-        if (!mixed && task_.recon != RECON_NONE) {
-            if (2ll * ne >= 3 * 152 * 3 * 256) c.shape[KIND_FLUX].block = 256;
-            if (nc >= 152 * 4 * 256) c.shape[KIND_GRAD].block = 128;
-        }
+        // The FP64 flux kernel is long (up to 100 KB of code): warps of one block run through it
+        // together and share the instruction cache, so 256-thread blocks are the faster ones where
+        // the mesh fills the chip several times. From 9 such blocks per SM on; SSP-RK3 steps with 64
+        // against 256 threads, us: 130,050 triangles GODUNOV 503 / 469, ROE 304 / 305, HLLC 190 / 192,
+        // LAX 227 / 229; 259,200 942 / 880, 561 / 553, 352 / 347, 411 / 410; 2,097,152 7,362 / 6,740,
+        // 4,201 / 4,062, 2,419 / 2,378, 2,997 / 2,980. Below, the last round's filling decides: 64,800
+        // triangles 273 / 271, 172 / 179, 124 / 123, 133 / 137; 24,200 140 / 146, 95 / 95, 75 / 75, 81 / 80.
+        if (!mixed && task_.recon != RECON_NONE && 2ll * ne >= 9ll * 256 * c.sms) c.shape[KIND_FLUX].block = 256;
         c.A = dalloc<double>(4 * (size_t)nc);
         c.B = dalloc<double>(4 * (size_t)nc);
         c.cfl = dalloc<double>(nc);
