@@ -182,6 +182,13 @@ __global__ void k_selftest(int which, long long n, unsigned long long seed, unsi
             // x^(1/7), x in [0.5, 1.5): CUDA's pow is within 2 units in the last place, so is the difference
             const double x = 0.5 + (double)(r1 >> 12) * 0x1p-52, p7 = ::pow(x, 1.0 / 7.0);
             local += llabs(__double_as_longlong(ip::pow(x, 1.0 / 7.0)) - __double_as_longlong(p7)) > 2;
+            // comparisons, and x^a over all exponents and bases of the fixed-point form: 0.54 units here, 2
+            // in CUDA's pow, up to five units of the smaller binade where the two results lie in two
+            local += (ip::less(a2, c) != (a2 < c)) + (ip::less(a2, b2) != (a2 < b2)) + (ip::positive(b2) != (b2 > 0.0)) +
+                     (ip::not_negative(b2) != (b2 >= 0.0));
+            const double xw = __longlong_as_double((long long)((903ull + r3 % 240) << 52 | (r1 & 0xfffffffffffffull)));
+            const double aw = __longlong_as_double((long long)((1014ull + (r3 >> 16) % 11) << 52 | (r2 & 0xfffffffffffffull)));
+            local += llabs(__double_as_longlong(ip::pow(xw, aw)) - __double_as_longlong(::pow(xw, aw))) > 5;
         } else if (which == 1) {  // widening of random normal floats
             const float f = __uint_as_float((unsigned)(((r1 % 254) + 1) << 23) | (unsigned)(r2 & 0x807fffffu));
             local += __double_as_longlong(widen(f)) != __double_as_longlong((double)f);

@@ -186,7 +186,8 @@ int cfd2d_profile_steps(cfd2d_t* h, int nsteps, double kernel_ms[4], int kernel_
 /* Built-in check of the device arithmetic helpers on n seeded random operands,
  * against the hardware operation on the current device: which = 0 the FP64
  * operations formed on the integer pipes (product, quotient, reciprocal, root: must equal the
- * hardware's bit for bit; x^(1/7) within 2 units in the last place of pow's), 1 FP32->FP64
+ * hardware's bit for bit; comparisons; x^(1/7) within 2 units in the last place of pow's, x^a
+ * over all exponents within 5), 1 FP32->FP64
  * widening on the integer pipe (must equal the conversion), 2 FP64->FP32
  * narrowing on the integer pipe (within 1 ulp), 3 FP64 minmod with its
  * integer-pipe sign test (must equal a*b > 0 ? (|a| < |b| ? a : b) : 0 bit for
