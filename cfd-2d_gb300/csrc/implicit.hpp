@@ -37,7 +37,7 @@ enum ImpBndKind { IBND_INLET = 1, IBND_OUTLET = 2, IBND_WALL = 3 };
 enum : int { SOLVE_OK = 0, SOLVE_MAX_ITER = 0x2, SOLVE_CONVERG = 0x4 };
 
 constexpr int kGmresMaxKdim = 64;   // Krylov dimension bound of the device control block
-constexpr int kRedBlocks = 456;     // most blocks of a reduction kernel (3 per SM)
+constexpr int kRedBlocks = 456;     // most blocks of a reduction kernel (3 for each of GB300's 152 SMs)
 
 constexpr int kNotDone = 1 << 30;   // GmresCtl::done_col while the Arnoldi loop runs
 

@@ -1,20 +1,23 @@
 // IEEE binary64 arithmetic on the integer pipes.
 //
 // GB300's FP64 unit takes two lanes per clock and SM: a warp's FP64 instruction holds it for
-// 16 clocks, in which the SM can issue 64 instructions to its other pipes. The FP64 kernels
-// keep that unit 83-88% busy and the integer pipes under 5%, so an operation formed from about
-// thirty integer instructions is cheaper than the FP64 instruction itself, and the two run side
-// by side. Every function here returns the correctly rounded (to nearest, ties to even) result,
-// the very bits of the FP64 instruction or of the IEEE quotient and square root, so a kernel may
-// form any of its operations on either side.
+// 16 clocks, in which the SM can issue 64 instructions to its other pipes. Kernels that form
+// everything on that unit held it 83-88% and the integer pipes under 5%; an operation formed
+// from about thirty integer instructions then costs less than the FP64 instruction, and the two
+// run side by side (the flux kernel now: 72% and 53%). Every function here returns the correctly
+// rounded (to nearest, ties to even) result, the very bits of the FP64 instruction or of the
+// IEEE quotient and square root, so a kernel may form any of its operations on either side
+// (x^a: within 0.54 units in the last place).
 //
 // Measured on one SM with all warps resident (clocks per warp operation): product or sum 20
 // native (17 as a multiply-add of three registers; an operand from the constant bank or an
 // immediate costs the 20), product 10.9 here, 8.3 per product with two native to three here;
-// reciprocal 24 (90 native), quotient 34 (144), square root 34 (170). A sum formed here takes
-// 22.6 and lost in every kernel it was tried in (two steps at 2.1M triangles 6.48 -> 7.17 ms),
-// so sums stay native. Kernels: k_flux at 2.1M triangles 1.42 -> 0.62 ms, with a lane per Gauss
-// point; the same arithmetic in one thread per edge gained nothing (200-255 registers).
+// reciprocal 24 (90 native), quotient 34 (144), square root 34 (170). An integer sum took 22.6
+// and lost in every kernel it was tried in (two steps at 2.1M triangles 6.48 -> 7.17 ms); it was
+// not kept, sums are native. Kernels: k_flux at 2.1M triangles 1.42 -> 0.62 ms, with a lane per
+// Gauss point; the same arithmetic in one thread per edge gained nothing there (200-255
+// registers). With a warp or less per scheduler an operation's latency counts, and the native
+// product is the shorter one (adj_native in adj_inst.cuh).
 //
 // The common path takes operands with 2^-510 <= |x| < 2^510, whose products and quotients
 // stay normal; zeros, and anything else, leave it by a branch.
@@ -148,9 +151,13 @@ IP_FN void muln(double* r, const double* a, const double* b) {
 
 // ---- reciprocal, quotient, square root
 
-// 1/m for the significand m of b (1 <= m < 2), Q63, within 4 units: a binary32 seed and two
-// Newton steps in fixed point, the first with a 64-bit significand and a 32-bit reciprocal
-// (error 2^-22 -> 2^-43), the second with both in 64 bits (-> 2^-62).
+// 1/m for the significand m of b (1 <= m < 2), Q63, at most 1 unit too small and 2 too large
+// (measured over 1.8e8 operands with seeds two units off: -1.002 to 1.996): a binary32 seed and
+// two Newton steps in fixed point, the first with a 64-bit significand and a 32-bit reciprocal
+// (error 2^-22 -> 2^-43), the second with both in 64 bits, where the error left (2^-86) is far
+// below a unit. What counts is the rounding of that second step: the remainder's product without
+// its lowest part Bl yl (below 2^-62) makes y up to 2 units too large, the last shift, rounding
+// down, up to 1 too small; the remainder's own shift (2^-72) and yh for y (2^-74) add 2^-9 units.
 // The last bit of a quotient is decided by the guard bits below it unless these lie within the
 // approximation's error of one half; then the exact remainder decides (a quotient of two
 // 53-bit significands is never a tie).
@@ -180,7 +187,7 @@ IP_RARE u32 round_by_remainder(u64 nl, u32 qh, u32 ql, u32 mbh, u32 mbl) {
 // 1/b, b in range, y = recip_of(b)
 IP_FN double rcp_core(double b, const Recip& y) {
     const u32 ql = shr2(y.yl, y.yh, 10), qh = y.yh >> 10;
-    u32 z = y.yl << 22;  // ten guard bits; y is at most 1 unit too small, 2 too large
+    u32 z = y.yl << 22;  // ten guard bits, y's error as recip_of says
     if (__builtin_expect(z - (0x80000000u - (2u << 22)) <= (5u << 22), 0))
         z = round_by_remainder(0ull, qh, ql, mant_hi(b), lo(b));
     return round_pack(qh, ql, z, ((2044u << 20) - (hi(b) & 0x7ff00000u)) + (hi(b) & 0x80000000u));
@@ -193,7 +200,7 @@ IP_FN double quot_core(double a, double b, const Recip& y) {
     const u32 Th = (u32)(T >> 32), Tl = (u32)T;
     const u32 s = Th >> 30, sh = 9 + s;
     const u32 ql = shr2(Tl, Th, sh), qh = Th >> sh;
-    u32 z = shr2(0u, Tl, sh);  // nine or ten guard bits; T is within 5 units
+    u32 z = shr2(0u, Tl, sh);  // nine or ten guard bits; T within 5 units: y's 2, three products rounded down
     if (__builtin_expect(z - (0x80000000u - (5u << 23)) <= (10u << 23), 0))
         z = round_by_remainder((((u64)mant_hi(a) << 32) | lo(a)) << (53 - s), qh, ql, mant_hi(b), lo(b));
     const u32 E = (hi(a) & 0x7ff00000u) - (hi(b) & 0x7ff00000u) + ((1021u + s) << 20);
