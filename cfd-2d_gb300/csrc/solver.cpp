@@ -456,18 +456,26 @@ void Solver::build_many() {
 }
 
 void Solver::launch_steps(int n, bool instances) {
-    if (n >= kGraphSteps && !gexec_many_ && !many_failed_) many_wanted_ = true;
-    while (n > 0) {
-        const int k = n >= kGraphSteps && gexec_many_ ? kGraphSteps : 1;
-        CUDA_CHECK(cudaGraphLaunch(k > 1 ? gexec_many_ : gexec_, stream_));
-        for (int j = 0; j < k; j++) {
+    auto launch = [&](cudaGraphExec_t g, int k) {
+        CUDA_CHECK(cudaGraphLaunch(g, stream_));
+        n -= k;
+        for (; k > 0; k--) {
             steps_++;
             if (task_.steady) continue;
             t_ += tau_;  // src/methods/fvm_tvd.cpp:312-316
             if (instances)
                 for (auto& in : inst_) in.t += in.tau;
         }
-        n -= k;
+    };
+    if (n >= kGraphSteps && !gexec_many_ && !many_failed_) {
+        // the GPU's work while the graph of many is made: at once where more steps can use it
+        for (int k = 0; k < kGraphSteps; k++) launch(gexec_, 1);
+        if (n >= kGraphSteps) build_many();
+        else many_wanted_ = true;
+    }
+    while (n > 0) {
+        const bool many = n >= kGraphSteps && gexec_many_;
+        launch(many ? gexec_many_ : gexec_, many ? kGraphSteps : 1);
     }
 }
 

@@ -189,10 +189,11 @@ private:
     cudaStream_t stream_ = nullptr;
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t gexec_ = nullptr;
-    // kGraphSteps steps. Made by the first call that takes so many at once, while the GPU runs that
-    // call's single steps (that call 614 us against 613 with the graph made beforehand, mixed 300
-    // against 285; a later one 574, 252; 162 triangles, eight steps). Made with the handle it cost
-    // every handle 170 us (FP64, 450 -> 620) or 130 us (mixed).
+    // kGraphSteps steps. Made by the first call that takes so many at once, while the GPU runs eight
+    // single steps of it (set_state and ten steps, us, this call / a later one / the first with the
+    // graph made beforehand / no such graph: 162 triangles FP64 773 / 742 / 767 / 857, 20,000 first
+    // order 221 / 187 / 194 / 258, 11,250 mixed 415 / 381 / 404 / 422). Made with the handle it cost
+    // every handle 170 us (162 triangles, FP64, 450 -> 620) or 130 us (mixed).
     cudaGraphExec_t gexec_many_ = nullptr;
     bool many_wanted_ = false, many_failed_ = false;
     cudaGraph_t capture_steps(int n);

@@ -123,6 +123,13 @@ with tempfile.TemporaryDirectory() as d:
         r["log"] = log()
         return r
     out["step7"] = step(7)
+    other = capi.Solver(path, mesh=m)
+    log()
+    h, mine = other, h
+    out["step9"] = [step(9), step(9)]
+    h.close()
+    log()
+    h = mine
     out["step16"] = [step(16), step(16)]
     out["fail"] = []
     for k in (0, 1, 2, 3):
@@ -182,11 +189,11 @@ def test_graph_of_many_steps_is_made_by_the_first_call_that_takes_them(seen):
 
     assert makes(seen["create"]) == one
     assert makes(seen["step7"]["log"]) == []
-    first, second = (r["log"] for r in seen["step16"])
-    assert makes(first) == many and makes(second) == []
-    # made behind the launches, before the wait for them
-    assert [c for c in first if c != "kernel"] == ["graph%d" % per_step] * 16 + many + ["wait-stream"]
-    assert [c for c in second if c != "kernel"] == ["graph%d" % (8 * per_step)] * 2 + ["wait-stream"]
+    alone, eight = ["graph%d" % per_step], ["graph%d" % (8 * per_step)]
+    for calls, expect in (("step16", (alone * 8 + many + eight, eight * 2)),  # behind eight steps, for the others
+                          ("step9", (alone * 9 + many, eight + alone))):      # behind all of them, for the next call
+        for r, e in zip(seen[calls], expect):
+            assert [c for c in r["log"] if c != "kernel"] == e + ["wait-stream"]
 
 
 def test_steps_go_on_where_the_graph_of_many_cannot_be_made(seen):
